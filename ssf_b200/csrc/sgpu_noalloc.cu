@@ -13,10 +13,10 @@
 // event creation).
 //
 // Limits and sharing:
-//  - at most SGPU_NOALLOC_MAX_N equations (131072): the array holds five
-//    FP64 vectors of that length plus reduction slots, about 5 MiB;
+//  - at most SGPU_NOALLOC_MAX_N equations (131072): the array holds four
+//    FP64 vectors of that length plus reduction slots, about 4 MiB;
 //  - every call uses the same array, which keeps the last call's contents;
-//    the entry point clears what must start at zero (reduction tickets,
+//    the entry point clears what must start at zero (the grid barrier, the
 //    iteration state) on every call;
 //  - calls whose work overlaps on the GPU (two host threads, or two streams
 //    of one process, at the same time on the same device) race on the
@@ -39,8 +39,9 @@
 // leaves x untouched.  The caller's col/val arrays must hold rowptr[n]
 // entries: the checks keep every read inside [0, rowptr[n]).
 //
-// The iteration is the reference's symcomprow::cg_prec with the diagonal
-// preconditioner (GEFEL/scr.cpp:1093-1205): stop on (r.r)/(f.f) < res, and
+// The iteration (k_pcg_resident, one cooperative launch of a CTA per SM with
+// a thread or more per row, hence the largest size) is the reference's
+// symcomprow::cg_prec with the diagonal preconditioner (GEFEL/scr.cpp:1093-1205): stop on (r.r)/(f.f) < res, and
 // *ani = i, *ares = (r.h)/(f.f) written only on convergence.
 #include <cuda_runtime.h>
 
@@ -49,50 +50,44 @@
 #include <string>
 
 #include "sgpu_internal.cuh"
+#include "sgpu_persist.cuh"
+
+using namespace sgpu;
 
 namespace {
 
 constexpr int kTPB = 256;
 constexpr int kMaxN = SGPU_NOALLOC_MAX_N;
-constexpr int kBlocks = 148 * 4;      // grid of every kernel here
-constexpr int kChunk = 16;            // iterations launched between state reads
-
-struct NaState {
-  double nory, nom, denom, alpha, beta, rr, ares, res, zero;
-  long long it, ni, ani;
-  int done, status, ani_set, pad;
-};
+constexpr int kBlocks = 148 * 4;  // grid of the input check
+// iterations of one launch, between two reads of the state: under 50 ms at
+// the largest size, and few enough waits that they cost nothing
+constexpr long long kChunk = 2048;
 
 // byte layout of the scratch array
 constexpr size_t kVecBytes = sizeof(double) * (size_t)kMaxN;
 constexpr size_t kOffDiag = 0;
 constexpr size_t kOffR = kOffDiag + kVecBytes;
-constexpr size_t kOffH = kOffR + kVecBytes;
-constexpr size_t kOffD = kOffH + kVecBytes;
-constexpr size_t kOffP = kOffD + kVecBytes;
-constexpr size_t kOffPart = kOffP + kVecBytes;                    // 2 * kBlocks doubles
-constexpr size_t kOffState = kOffPart + 2 * kBlocks * sizeof(double);
-constexpr size_t kOffTicket = kOffState + 256;                    // 4 unsigned
-constexpr size_t kScratchBytes = kOffTicket + 256;
+constexpr size_t kOffDh = kOffR + kVecBytes;  // pairs {direction, preconditioned residual}
+constexpr size_t kOffSync = kOffDh + 2 * kVecBytes;
+constexpr size_t kOffState = kOffSync + sizeof(GridSync);
+constexpr size_t kScratchBytes = kOffState + ((sizeof(PcgState) + 255) & ~(size_t)255);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 struct Scratch {
-  double *diag, *r, *h, *d, *p, *part;
-  NaState *st;
-  unsigned *ticket;
+  double *diag, *r;
+  double2 *dh;
+  GridSync *gs;
+  PcgState *st;
 };
 
 Scratch carve(unsigned char *base) {
   Scratch s;
   s.diag = reinterpret_cast<double *>(base + kOffDiag);
   s.r = reinterpret_cast<double *>(base + kOffR);
-  s.h = reinterpret_cast<double *>(base + kOffH);
-  s.d = reinterpret_cast<double *>(base + kOffD);
-  s.p = reinterpret_cast<double *>(base + kOffP);
-  s.part = reinterpret_cast<double *>(base + kOffPart);
-  s.st = reinterpret_cast<NaState *>(base + kOffState);
-  s.ticket = reinterpret_cast<unsigned *>(base + kOffTicket);
+  s.dh = reinterpret_cast<double2 *>(base + kOffDh);
+  s.gs = reinterpret_cast<GridSync *>(base + kOffSync);
+  s.st = reinterpret_cast<PcgState *>(base + kOffState);
   return s;
 }
 
@@ -117,58 +112,16 @@ int scratch_address(unsigned char **out) {
   return SGPU_OK;
 }
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// block sums of NV values; the last block to arrive adds the partials in
-// block order and returns true in its thread 0
-template <int NV>
-__device__ bool grid_sum(double (&v)[NV], double *part, unsigned *ticket, double (&tot)[NV]) {
-  __shared__ double sh[NV][kTPB / 32];
-  __shared__ bool last;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NV; q++) v[q] = warp_sum(v[q]);
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < NV; q++) sh[q][w] = v[q];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; q++) {
-      double t = 0.0;
-      for (int k = 0; k < kTPB / 32; k++) t += sh[q][k];
-      part[q * gridDim.x + blockIdx.x] = t;
-    }
-    __threadfence();
-    last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (!last || threadIdx.x != 0) return false;
-  __threadfence();
-#pragma unroll
-  for (int q = 0; q < NV; q++) {
-    double t = 0.0;
-    for (int b = 0; b < (int)gridDim.x; b++) t += __ldcg(part + q * gridDim.x + b);
-    tot[q] = t;
-  }
-  *ticket = 0u;
-  return true;
-}
-
-// clears the state and the reduction tickets (one thread: nothing else of the
-// call runs before it)
+// clears the state (one thread: nothing else of the call runs before it)
 __global__ void k_na_clear(Scratch s, long long ni, double res, double zero) {
-  NaState z = {};
+  PcgState z = {};
   z.ni = ni;
   z.res = res;
   z.zero = zero;
+  z.crit = SGPU_CRIT_SCR_PREC;
+  z.prec = 1;
   z.ani = -1;
   *s.st = z;
-  for (int k = 0; k < 4; k++) s.ticket[k] = 0u;
 }
 
 // checks every row and extracts the diagonal; a malformed row stops the call
@@ -199,123 +152,6 @@ __global__ void k_na_setup(int n, const int *__restrict__ rowptr, const int *__r
   }
 }
 
-// y = A v, 16 lanes per row; with DOT, d.p -> alpha (and the breakdown test)
-template <bool DOT>
-__global__ void k_na_spmv(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
-                          const double *__restrict__ val, const double *__restrict__ v, double *__restrict__ y,
-                          Scratch s) {
-  if (s.st->done) return;
-  const int lane = threadIdx.x & 31, g = lane >> 4, sub = lane & 15;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-  double acc = 0.0;
-  for (int base = warp * 2; base < n; base += nw * 2) {
-    const int i = base + g;
-    int b = 0, e = 0;
-    if (i < n) { b = rowptr[i]; e = rowptr[i + 1]; }
-    double t = 0.0;
-    for (int k = b + sub; k < e; k += 16) t += val[k] * v[col[k]];
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o, 16);
-    if (sub == 0 && i < n) {
-      y[i] = t;
-      acc += v[i] * t;
-    }
-  }
-  if (DOT) {
-    double a[1] = {acc}, tot[1];
-    if (grid_sum<1>(a, s.part, s.ticket + 0, tot)) {
-      NaState *st = s.st;
-      st->denom = tot[0];
-      if (fabs(tot[0]) < st->zero) {  // scr.cpp:1146-1151
-        st->ani = st->it;
-        st->ares = st->nom;
-        st->ani_set = 1;
-        if (st->status == 0) st->status = SGPU_BREAKDOWN;  // a zero right-hand side keeps its status
-        st->done = 1;
-      } else {
-        st->alpha = st->nom / tot[0];
-      }
-    }
-  }
-}
-
-// r = f - p (p = A x0 when iv, else x = 0 and r = f), h = r/diag, d = h;
-// f.f and r.h
-__global__ void k_na_start(int n, const double *__restrict__ f, double *__restrict__ x, int iv, Scratch s) {
-  if (s.st->done) return;  // malformed input: x stays as the caller left it
-  double v[2] = {0.0, 0.0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double ri;
-    if (iv) {
-      ri = f[i] - s.p[i];
-    } else {
-      ri = f[i];
-      x[i] = 0.0;
-    }
-    const double hi = ri / s.diag[i];
-    s.r[i] = ri;
-    s.h[i] = hi;
-    s.d[i] = hi;
-    v[0] += f[i] * f[i];
-    v[1] += ri * hi;
-  }
-  double t[2];
-  if (grid_sum<2>(v, s.part, s.ticket + 1, t)) {
-    NaState *st = s.st;
-    st->nory = t[0];
-    st->nom = t[1];
-    if (t[0] < st->zero) {  // scr.cpp:1117-1120: reported, the iteration goes on
-      st->status = SGPU_ZERO_RHS;
-      st->ares = t[0];
-      st->ani = 0;
-      st->ani_set = 1;
-    }
-    if (st->ni <= 0) st->done = 1;
-  }
-}
-
-// x += alpha d; r -= alpha p; h = r/diag; stop test on (r.r)/(f.f)
-__global__ void k_na_update(int n, double *__restrict__ x, Scratch s) {
-  if (s.st->done) return;
-  const double alpha = s.st->alpha;
-  double v[2] = {0.0, 0.0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    x[i] += alpha * s.d[i];
-    const double ri = s.r[i] - alpha * s.p[i];
-    const double hi = ri / s.diag[i];
-    s.r[i] = ri;
-    s.h[i] = hi;
-    v[0] += ri * ri;
-    v[1] += ri * hi;
-  }
-  double t[2];
-  if (grid_sum<2>(v, s.part, s.ticket + 2, t)) {
-    NaState *st = s.st;
-    st->rr = t[0];
-    st->beta = t[1] / st->nom;
-    st->nom = t[1];
-    const long long it = st->it;
-    st->it = it + 1;
-    if (fabs(t[0] / st->nory) < st->res) {  // scr.cpp:1188
-      st->ani = it;
-      st->ares = t[1] / st->nory;
-      st->ani_set = 1;
-      st->done = 1;
-    } else if (it + 1 >= st->ni) {
-      st->done = 1;
-      if (st->status == 0) st->status = SGPU_NOT_CONVERGED;
-    }
-  }
-}
-
-// d = beta d + h
-__global__ void k_na_dir(int n, Scratch s) {
-  if (s.st->done) return;
-  const double beta = s.st->beta;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    s.d[i] = beta * s.d[i] + s.h[i];
-}
-
 }  // namespace
 
 extern "C" SGPU_API int sgpu_csr_pcg_noalloc_d(int32_t n, const int32_t *rowptr_d, const int32_t *col_d,
@@ -340,25 +176,37 @@ extern "C" SGPU_API int sgpu_csr_pcg_noalloc_d(int32_t n, const int32_t *rowptr_
   int rc = scratch_address(&base);
   if (rc != SGPU_OK) return rc;
   const Scratch s = carve(base);
+  const int grid = resident_grid();
+  if (!resident_rows_fit(n, grid))  // fewer than 128 SMs
+    return sgpu::fail(SGPU_CUDA_ERROR, "the device has too few SMs for the no-allocation solver's resident grid");
   k_na_clear<<<1, 1, 0, st>>>(s, (long long)ni, res, zero);
   k_na_setup<<<kBlocks, kTPB, 0, st>>>(n, rowptr_d, col_d, val_d, s);
-  if (iv) k_na_spmv<false><<<kBlocks, kTPB, 0, st>>>(n, rowptr_d, col_d, val_d, x_d, s.p, s);
-  k_na_start<<<kBlocks, kTPB, 0, st>>>(n, f_d, x_d, iv != 0, s);
-  sgpu::count_launches(iv ? 4 : 3);
-  NaState h = {};
-  for (;;) {
-    for (int k = 0; k < kChunk; k++) {
-      k_na_spmv<true><<<kBlocks, kTPB, 0, st>>>(n, rowptr_d, col_d, val_d, s.d, s.p, s);
-      k_na_update<<<kBlocks, kTPB, 0, st>>>(n, x_d, s);
-      k_na_dir<<<kBlocks, kTPB, 0, st>>>(n, s);
-    }
-    sgpu::count_launches(3 * kChunk);
-    cudaError_t e = cudaGetLastError();
+  sgpu::count_launches(2);
+  ResidentArgs a = {};
+  a.n = n;
+  a.rowptr = rowptr_d;
+  a.col = col_d;
+  a.val = val_d;
+  a.diag = s.diag;
+  a.f = f_d;
+  a.x = x_d;
+  a.r = s.r;
+  a.dh = s.dh;
+  a.st = s.st;
+  a.gs = s.gs;
+  a.iv = iv != 0;
+  a.most = kChunk;
+  PcgState h = {};
+  for (a.start = 1;; a.start = 0) {
+    cudaError_t e = cudaMemsetAsync(s.gs, 0, sizeof(GridSync), st);
+    if (e == cudaSuccess) e = launch_resident(a, 0, grid, st);
+    sgpu::count_launches(1);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, s.st, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return sgpu::fail(SGPU_CUDA_ERROR, std::string("no-allocation PCG: ") + cudaGetErrorString(e));
     if (h.done) break;
   }
+  if (h.status == SGPU_CUDA_ERROR) return sgpu::fail(SGPU_CUDA_ERROR, "no-allocation PCG: the grid's barrier ran out");
   if (iterations) *iterations = h.it;
   if (h.ani_set) {
     if (ani) *ani = h.ani;

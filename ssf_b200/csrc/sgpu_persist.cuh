@@ -1,0 +1,450 @@
+// Jacobi-PCG as one resident grid.
+//
+// A small system's iteration is bound by latency, not by bytes: as three
+// launches with a serial sum of the block partials, an iteration of a
+// 101,404-equation plate (1.8M entries, 22 MB) took 77 us on B200, of which
+// reading its matrix needs 3.  Here the whole iteration runs inside one
+// cooperative launch of one CTA per SM and costs one gather and two grid
+// barriers: 8.1 us on that plate (162.8 -> 16.9 ms for its 2094 iterations),
+// 6.4 to 7 us on systems of 1500 to 24,000 equations.
+#pragma once
+
+#include <algorithm>
+
+#include "sgpu_internal.cuh"
+
+namespace sgpu {
+
+// ---------------------------------------------------------------------------
+// grid barrier that also sums
+// ---------------------------------------------------------------------------
+// Every CTA stores its partial sums, adds to an arrival counter (release) and
+// one thread polls the counter (acquire); the first warp then reads all
+// partials.  Sums of even and odd barriers have their own slots: a CTA writes
+// those of barrier e + 2 only after every CTA has arrived at e + 1, so after
+// it has read those of e.  All CTAs add the same values in the same order, so
+// every thread of the grid gets the same bits and the control flow that
+// follows is uniform.  Measured on 148 CTAs of 1024 threads: 2.3 us, of which
+// the CTA's own reduction 0.7; polling 148 flagged partials directly (no
+// counter) took 4.1 us, with 148 x 148 polls in flight.
+//
+// The launch is cooperative, so all CTAs are resident; the poll still has a
+// limit, after which the CTA gives up (the others then run out too) and the
+// caller reports SGPU_CUDA_ERROR.
+constexpr int kPollLimit = 1 << 22;  // about 3 s of polls
+constexpr int kMaxGrid = 256;        // CTAs the slots hold
+
+struct GridSync {  // in global memory, zeroed before each launch
+  unsigned arrived;
+  unsigned pad[31];
+  double part[2][2][kMaxGrid];  // parity, sum, CTA
+};
+
+__device__ __forceinline__ double persist_warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+struct GridSumShared {
+  double part[2][32];  // per warp
+  double tot[2];
+};
+
+// v: the thread's partial sums in, the grid's sums out (every thread); e: the
+// number of this barrier in the launch, from 1.  Orders every global write
+// before it (of all CTAs) before every read after it.  False: gave up.
+template <int NV>
+__device__ __forceinline__ bool grid_barrier_sum(double (&v)[NV], GridSync *gs, unsigned e, GridSumShared &sh) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int G = gridDim.x;
+#pragma unroll
+  for (int q = 0; q < NV; q++) {
+    v[q] = persist_warp_sum(v[q]);
+    if (lane == 0) sh.part[q][w] = v[q];
+  }
+  __syncthreads();
+  bool ok = true;
+  if (w == 0) {
+    double t[NV];
+#pragma unroll
+    for (int q = 0; q < NV; q++) t[q] = persist_warp_sum(lane < nw ? sh.part[q][lane] : 0.0);
+    if (lane == 0) {
+#pragma unroll
+      for (int q = 0; q < NV; q++) __stcg(&gs->part[e & 1][q][blockIdx.x], t[q]);
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gs->arrived) : "memory");
+      unsigned c;
+      int tries = 0;
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&gs->arrived) : "memory");
+        ok = ++tries < kPollLimit;
+      } while (c < e * (unsigned)G && ok);
+    }
+    __syncwarp();
+    double s[NV];
+#pragma unroll
+    for (int q = 0; q < NV; q++) s[q] = 0.0;
+#pragma unroll
+    for (int u = 0; u < kMaxGrid / 32; u++) {
+      const int k = lane + 32 * u;
+      if (k < G) {
+#pragma unroll
+        for (int q = 0; q < NV; q++) s[q] += __ldcg(&gs->part[e & 1][q][k]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+      s[q] = persist_warp_sum(s[q]);
+      if (lane == 0) sh.tot[q] = s[q];
+    }
+  }
+  ok = __syncthreads_and(ok);
+#pragma unroll
+  for (int q = 0; q < NV; q++) v[q] = sh.tot[q];
+  return ok;
+}
+
+// ---------------------------------------------------------------------------
+// scalars of the iteration
+// ---------------------------------------------------------------------------
+// The state of the solve, one copy per CTA in shared memory.  Every thread
+// evaluates the same tests on the same sums (so no broadcast is needed) and
+// thread 0 alone records the outcome; a thread keeps only r.h and beta in
+// registers.  What thread 0 writes here is read by the others after the next
+// grid barrier at the earliest.
+struct CgShared {
+  PcgState s;
+  __device__ __forceinline__ void load(const PcgState *st) {
+    if (threadIdx.x == 0) s = *st;
+  }
+  // f.f and r.h of the start (scr.cpp:1117-1120: a zero right-hand side is
+  // reported and the iteration goes on to the zero denominator;
+  // cr.cpp:1160-1164 returns at once); true: stop
+  __device__ __forceinline__ bool begin(double ff, double rh) {
+    const bool zero_rhs = ff < s.zero;
+    const bool stop = (zero_rhs && s.crit == SGPU_CRIT_CR_PREC) || s.ni <= 0;
+    if (threadIdx.x == 0) {
+      s.nory = ff;
+      s.nom = rh;
+      s.beta = 0.0;
+      s.it = 0;
+      if (zero_rhs) {
+        s.status = SGPU_ZERO_RHS;
+        s.ares = ff;
+        s.ani = 0;
+        s.ani_set = 1;
+      }
+      if (stop) s.done = 1;
+    }
+    return stop;
+  }
+  // denom = d.p: the breakdown test (scr.cpp:1146-1151, cr.cpp:1177-1181)
+  // and alpha; true: stop
+  __device__ __forceinline__ bool direction(double dp, double nom, double &alpha) {
+    const bool stop = fabs(dp) < s.zero;
+    alpha = nom / dp;
+    if (threadIdx.x == 0) {
+      s.denom = dp;
+      if (stop) {
+        s.ani = s.it;
+        s.ares = nom;
+        s.ani_set = 1;
+        if (s.status == 0) s.status = SGPU_BREAKDOWN;
+        s.done = 1;
+      } else {
+        s.alpha = alpha;
+      }
+    }
+    return stop;
+  }
+  // r.r and r.h after the update: beta and the routine's stopping test at
+  // iteration it (counted from 0); true: stop (or pause, for SGPU_CRIT_TRUE:
+  // the host confirms on the true residual)
+  __device__ __forceinline__ bool updated(double rr, double rh, long long it, double &nom, double &beta) {
+    beta = rh / nom;
+    const int crit = s.crit;
+    bool conv;
+    if (crit == SGPU_CRIT_SCR_PREC) conv = fabs(rr / s.nory) < s.res;    // scr.cpp:1188
+    else if (crit == SGPU_CRIT_CR_PREC) conv = sqrt(rh / s.nory) < s.res;  // cr.cpp:1217
+    else conv = rr < s.tol2 * s.nory;
+    const bool last = it + 1 >= s.ni;
+    if (threadIdx.x == 0) {
+      s.rr = rr;
+      s.rho_prev = nom;
+      s.beta = beta;
+      s.nom = rh;
+      s.it = it + 1;
+      if (conv) {
+        s.ani = it;
+        s.ares = crit == SGPU_CRIT_CR_PREC ? rh : rh / s.nory;
+        s.ani_set = 1;
+        if (crit == SGPU_CRIT_TRUE) s.pause = 1;
+        else s.done = 1;
+      } else if (last) {
+        s.done = 1;
+        if (s.status == 0) s.status = SGPU_NOT_CONVERGED;
+        if (crit == SGPU_CRIT_CR_PREC) {
+          s.ani = s.ni;
+          s.ares = rh;
+          s.ani_set = 1;
+        }
+      }
+    }
+    nom = rh;
+    return conv || last;
+  }
+};
+
+// ---------------------------------------------------------------------------
+// the resident iteration
+// ---------------------------------------------------------------------------
+// T lanes own one row for the whole solve: its x, r, h, d and diagonal entry
+// stay in their registers and its matrix entries in shared memory (lane s of
+// a row has entries s, s + T, ...; a warp's entries are stored slot by slot,
+// so a warp reads one contiguous segment per slot).  T is the largest power
+// of two that still gives every row of the CTA its lanes, so a small system
+// spreads its rows over many lanes and a large one has a thread per row.
+//
+// Per iteration:
+//   gather  y = A d with d = beta d_old + h formed at the gather from the
+//           16-byte pairs dh[c] = {d_old, h}: one load per entry instead of
+//           a second barrier between the direction update and the product
+//   barrier d.y -> alpha
+//   update  x, r, h in registers; dh[i] = {d, h} for the next gather
+//   barrier r.r, r.h -> beta, stopping test
+//
+// Warps whose entries do not fit the CTA's shared memory read them from the
+// CSR arrays each iteration, eight lanes to a row (105,840 equations with 8M
+// entries, where a quarter fits: 28.5 us an iteration).
+//
+// The kernel starts the solve itself (start != 0: r = f - A x0) and runs at
+// most `most` iterations; x and r then go back to memory, so that the next
+// launch goes on.  x_in for the start is read when iv != 0.
+constexpr int kResidentTPB = 1024;
+
+struct ResidentArgs {
+  int n;
+  const int *rowptr, *col;
+  const double *val, *diag, *f;
+  double *x, *r;
+  double2 *dh;
+  PcgState *st;
+  GridSync *gs;
+  int rows_per_cta;  // <= kResidentTPB / T
+  int cap;           // matrix entries the dynamic shared memory holds
+  int start, iv;
+  long long most;
+};
+
+// what one gather of the iteration reads
+struct GatherDir {
+  const double2 *dh;
+  double beta;
+  __device__ __forceinline__ double operator()(int c) const {
+    const double2 g = dh[c];
+    return fma(beta, g.x, g.y);
+  }
+};
+struct GatherPlain {
+  const double *x;
+  __device__ __forceinline__ double operator()(int c) const { return x[c]; }
+};
+
+// y of the lane's row (valid in all T lanes of the row)
+template <int T, class X>
+__device__ __forceinline__ double resident_product(const ResidentArgs &a, bool resident, int slots, const double *sv,
+                                                   const int *sc, int i, bool active, const X &x) {
+  const int lane = threadIdx.x & 31;
+  double y = 0.0;
+  if (resident) {
+#pragma unroll 6
+    for (int s = 0; s < slots; s++) y = fma(sv[32 * s], x(sc[32 * s]), y);
+#pragma unroll
+    for (int o = T / 2; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    return y;
+  }
+  // 8 lanes per row (T, where more lanes own a row), 32 / 8 rows of the warp at a time
+  constexpr int L = T < 8 ? 8 : T, RPW = 32 / L, ROWS = 32 / T;
+  const int sub = lane % L, g = lane / L;
+  const int i0 = __shfl_sync(0xffffffffu, i, 0);
+  const unsigned act = __ballot_sync(0xffffffffu, active);
+#pragma unroll 1
+  for (int q = 0; q < ROWS; q += RPW) {
+    const int lr = q + g;  // row of the warp, owned by lanes T lr ...
+    const int row = i0 + lr;
+    double s = 0.0;
+    if ((act >> (T * lr)) & 1u) {
+      const int b = a.rowptr[row], e = a.rowptr[row + 1];
+#pragma unroll 4
+      for (int k = b + sub; k < e; k += L) s = fma(a.val[k], x(a.col[k]), s);
+    }
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    // the owners of rows q .. q + RPW - 1 take their sums
+    const int mine = lane / T;
+    const double t = __shfl_sync(0xffffffffu, s, ((mine - q) & (RPW - 1)) * L);
+    if (mine >= q && mine < q + RPW) y = t;
+  }
+  return y;
+}
+
+template <int T>
+__global__ void __launch_bounds__(kResidentTPB, 1) k_pcg_resident(const ResidentArgs a) {
+  extern __shared__ double dyn[];
+  __shared__ GridSumShared sums;
+  __shared__ CgShared cg;
+  __shared__ int woff[kResidentTPB / 32 + 1];
+  double *sval = dyn;
+  int *scol = reinterpret_cast<int *>(dyn + a.cap);
+  if (a.st->done | a.st->pause) return;  // the same in every CTA: this grid writes it after its last barrier
+  cg.load(a.st);
+  const int prec = a.st->prec;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lrow = threadIdx.x / T, sub = threadIdx.x % T;
+  const int i = blockIdx.x * a.rows_per_cta + lrow;
+  const bool active = lrow < a.rows_per_cta && i < a.n;
+  const bool owner = active && sub == 0;
+
+  // the rows' entries into shared memory
+  int b = 0, len = 0;
+  if (active) {
+    b = a.rowptr[i];
+    len = a.rowptr[i + 1] - b;
+  }
+  const int slots = len > sub ? (len - sub + T - 1) / T : 0;
+  int ws = slots;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ws = max(ws, __shfl_xor_sync(0xffffffffu, ws, o));
+  if (lane == 0) woff[w + 1] = 32 * min(ws, a.cap / 32 + 1);
+  if (threadIdx.x == 0) woff[0] = 0;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int k = 0; k < kResidentTPB / 32; k++) woff[k + 1] = min(woff[k] + woff[k + 1], a.cap + 32);
+  __syncthreads();
+  const bool resident = woff[w + 1] <= a.cap;
+  const double *sv = sval + woff[w] + lane;
+  const int *sc = scol + woff[w] + lane;
+  if (resident) {
+    double *wv = sval + woff[w] + lane;
+    int *wc = scol + woff[w] + lane;
+#pragma unroll 4
+    for (int s = 0; s < slots; s++) {
+      wv[32 * s] = a.val[b + sub + T * s];
+      wc[32 * s] = a.col[b + sub + T * s];
+    }
+  }
+
+  unsigned epoch = 0;
+  double xi = 0.0, ri = 0.0, hi = 0.0, di = 0.0, dg = 1.0, nom, beta;
+  long long it = a.start ? 0 : a.st->it;
+  bool ok = true, stop = false;
+  if (active && prec) dg = a.diag[i];
+  if (a.start) {
+    if (a.iv && active) xi = a.x[i];
+    double y = 0.0;
+    if (a.iv) y = resident_product<T>(a, resident, slots, sv, sc, i, active, GatherPlain{a.x});
+    double v[2] = {0.0, 0.0};
+    if (active) {
+      const double fi = a.f[i];
+      ri = fi - y;
+      hi = prec ? ri / dg : ri;
+      if (owner) {
+        a.dh[i] = make_double2(0.0, hi);
+        v[0] = fi * fi;
+        v[1] = ri * hi;
+      }
+    }
+    ok = grid_barrier_sum<2>(v, a.gs, ++epoch, sums);
+    stop = cg.begin(v[0], v[1]);
+    nom = v[1];
+    beta = 0.0;
+  } else {
+    nom = a.st->nom;
+    beta = a.st->beta;
+    if (active) {
+      xi = a.x[i];
+      ri = a.r[i];
+      const double2 g = a.dh[i];
+      di = g.x;
+      hi = g.y;
+    }
+  }
+
+  for (long long k = 0; ok && !stop && k < a.most; k++, it++) {
+    // y = A d, d.y
+    const double y = resident_product<T>(a, resident, slots, sv, sc, i, active, GatherDir{a.dh, beta});
+    di = fma(beta, di, hi);
+    double v1[1] = {owner ? di * y : 0.0}, alpha;
+    ok = grid_barrier_sum<1>(v1, a.gs, ++epoch, sums);
+    if (!ok || cg.direction(v1[0], nom, alpha)) break;
+    double v[2] = {0.0, 0.0};
+    if (active) {
+      xi = fma(alpha, di, xi);
+      ri = fma(-alpha, y, ri);
+      hi = prec ? ri / dg : ri;
+      if (owner) {
+        a.dh[i] = make_double2(di, hi);
+        v[0] = ri * ri;
+        v[1] = ri * hi;
+      }
+    }
+    ok = grid_barrier_sum<2>(v, a.gs, ++epoch, sums);
+    if (!ok) break;
+    stop = cg.updated(v[0], v[1], it, nom, beta);
+  }
+  if (owner) {
+    a.x[i] = xi;
+    a.r[i] = ri;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (!ok) {
+      cg.s.status = SGPU_CUDA_ERROR;
+      cg.s.done = 1;
+    }
+    *a.st = cg.s;
+  }
+}
+
+// CTAs of a resident grid on the current device (one per SM), and the entries
+// its shared memory holds
+inline int resident_grid() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 0;
+  return sms < kMaxGrid ? sms : kMaxGrid;
+}
+constexpr int kResidentSmem = 220 * 1024;  // beside about 1.2 KB of static shared memory
+constexpr int kResidentCap = kResidentSmem / 12;
+
+template <int T>
+inline cudaError_t launch_resident_t(const ResidentArgs &a, int grid, cudaStream_t s) {
+  const size_t smem = (size_t)a.cap * 12;
+  cudaError_t e = cudaFuncSetAttribute(k_pcg_resident<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmem);
+  if (e != cudaSuccess) return e;
+  ResidentArgs args = a;
+  void *p[] = {&args};
+  return cudaLaunchCooperativeKernel((const void *)k_pcg_resident<T>, dim3(grid), dim3(kResidentTPB), p, smem, s);
+}
+
+// Whether n rows have a thread each in the resident grid.
+inline bool resident_rows_fit(int64_t n, int grid) { return grid > 0 && n <= (int64_t)grid * kResidentTPB; }
+
+// nnz: entries of the matrix where the host knows them (twice a CTA's share
+// is asked for, the rest of the SM's memory stays L1), else 0
+inline cudaError_t launch_resident(ResidentArgs a, int64_t nnz, int grid, cudaStream_t s) {
+  int64_t cap = kResidentCap;
+  if (nnz > 0) cap = std::min<int64_t>(cap, 2 * (nnz / grid) + 2048);
+  a.cap = (int)cap & ~31;
+  a.rows_per_cta = (a.n + grid - 1) / grid;
+  grid = (a.n + a.rows_per_cta - 1) / a.rows_per_cta;  // no CTA without rows
+  const int r = a.rows_per_cta;
+  if (r > 512) return launch_resident_t<1>(a, grid, s);
+  if (r > 256) return launch_resident_t<2>(a, grid, s);
+  if (r > 128) return launch_resident_t<4>(a, grid, s);
+  if (r > 64) return launch_resident_t<8>(a, grid, s);
+  if (r > 32) return launch_resident_t<16>(a, grid, s);
+  return launch_resident_t<32>(a, grid, s);
+}
+
+}  // namespace sgpu

@@ -1,0 +1,97 @@
+"""The resident Jacobi-PCG grid at the sizes where its layout changes.
+
+Rows are spread over 32, 16, ... 1 lanes as the system grows (148 CTAs of
+1024 threads: the split changes at multiples of 148 x 32 rows), and warps
+whose entries do not fit the SM's memory read them from the caller's arrays.
+The matrices are diagonally dominant with condition below 4, so a residual of
+1e-10 bounds the relative solution error by 4e-10; 1e-9 is asserted.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from ssf_b200 import _lib as L
+
+pytestmark = pytest.mark.gpu
+
+
+def banded(n, offsets, seed, uneven=False):
+    """CSR of a symmetric matrix with entries in (-1, 0) / (2 * len(offsets)) at the given offsets and a diagonal of
+    2: eigenvalues in [1, 3].  uneven: the offsets beyond the first only in every third row and column."""
+    rng = np.random.default_rng(seed)
+    rows, cols, vals = [np.arange(n)], [np.arange(n)], [np.full(n, 2.0)]
+    for q, o in enumerate(offsets):
+        i = np.arange(n - o)
+        if uneven and q:
+            i = i[(i % 3 == 0)]
+        v = -rng.random(i.size) / (2.0 * len(offsets))
+        rows += [i, i + o]
+        cols += [i + o, i]
+        vals += [v, v]
+    r, c, v = np.concatenate(rows), np.concatenate(cols), np.concatenate(vals)
+    order = np.lexsort((c, r))
+    r, c, v = r[order], c[order], v[order]
+    rowptr = np.zeros(n + 1, dtype=np.int32)
+    rowptr[1:] = np.cumsum(np.bincount(r, minlength=n))
+    return rowptr, c.astype(np.int32), v
+
+
+def product(rowptr, col, val, x):
+    return np.add.reduceat(val * x[col], rowptr[:-1])
+
+
+def solve(rowptr, col, val, f, x, ni=20000, iv=0):
+    import torch
+    d = [torch.from_numpy(v).cuda() for v in (rowptr, col, val, f, x)]
+    ani, ares, its = C.c_int64(-1), C.c_double(-1.0), C.c_int64(0)
+    st = L.lib().sgpu_csr_pcg_noalloc_d(f.size, *[v.data_ptr() for v in d], ni, 1e-20, 1e-30, iv, None, C.byref(ani),
+                                        C.byref(ares), C.byref(its))
+    return st, d[4].cpu().numpy(), ani.value, its.value
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 148, 149, 4736, 4737, 9473, 18945, 37889, 75776, 75777, L.NOALLOC_MAX_N])
+@pytest.mark.parametrize("uneven", [False, True])
+def test_row_splits(gpu_lib, n, uneven):
+    offsets = [o for o in (1, 7, 300) if o < n]
+    rowptr, col, val = banded(n, offsets, n, uneven)
+    x = np.random.default_rng(n + 1).standard_normal(n)
+    f = product(rowptr, col, val, x)
+    st, got, ani, its = solve(rowptr, col, val, f, np.full(n, 7.0))
+    assert st == L.OK and its == ani + 1
+    assert np.linalg.norm(got - x) <= 1e-9 * np.linalg.norm(x)
+
+
+@pytest.mark.parametrize("n,width", [(L.NOALLOC_MAX_N, 24), (60000, 60), (20000, 90)])
+def test_rows_beyond_shared_memory(gpu_lib, n, width):
+    rowptr, col, val = banded(n, list(range(1, width + 1)), n)
+    x = np.random.default_rng(5).standard_normal(n)
+    f = product(rowptr, col, val, x)
+    x0 = np.random.default_rng(6).standard_normal(n)
+    for iv, start in ((0, np.zeros(n)), (1, x0)):
+        st, got, _, _ = solve(rowptr, col, val, f, start, iv=iv)
+        assert st == L.OK
+        # the start residual of x0 is below 10 |f|: the same bound times 10
+        assert np.linalg.norm(got - x) <= 1e-9 * np.linalg.norm(x)
+
+
+def test_more_iterations_than_one_launch(gpu_lib, oracle):
+    """A 1D Laplacian takes about as many iterations as it has equations: more than the 2048 of one launch."""
+    n = 2600
+    rowptr, col, val = banded(n, [1], 0)
+    val = np.where(val == 2.0, 2.0, -1.0)
+    f = np.random.default_rng(1).standard_normal(n)
+    st, x, ani, its = solve(rowptr, col, val, f, np.zeros(n))
+    assert st == L.OK and its > 2048
+    # the recurrence residual met 1e-10; the true one adds the iteration's rounding, a few times
+    # eps ||K|| ||x|| / ||f||
+    r = f - product(rowptr, col, val, x)
+    assert np.linalg.norm(r) <= 1e-10 * np.linalg.norm(f) + 64 * 2.3e-16 * 4.0 * np.linalg.norm(x)
+
+
+def test_iteration_limit_and_zero_right_hand_side(gpu_lib):
+    rowptr, col, val = banded(500, [1], 3)
+    st, _, ani, its = solve(rowptr, col, val, np.ones(500), np.zeros(500), ni=2)
+    assert st == L.NOT_CONVERGED and ani == -1 and its == 2
+    st, x, ani, _ = solve(rowptr, col, val, np.zeros(500), np.zeros(500))
+    assert st == L.ZERO_RHS and ani == 0 and not x.any()
