@@ -2565,7 +2565,7 @@ SGPU_API int sgpu_assemble_copy(sgpu_matrix src, int32_t kind, const double *ema
   ad.node_rows = sa.node_rows;
 #undef DUP
   if (st != SGPU_OK) return bail(st);
-  if (c.val.alloc(c.nnz) != SGPU_OK || c.diag.alloc(c.n) != SGPU_OK) return bail(SGPU_CUDA_ERROR);
+  if (c.val.alloc(c.nnz + 2) != SGPU_OK || c.diag.alloc(c.n) != SGPU_OK) return bail(SGPU_CUDA_ERROR);
   m->bsr.valid = false;
   m->bsr.nb = -1;  // examined on first use
   if (emat && cudaMemcpyAsync(ad.emat.p, emat, ad.ne * (ad.general ? 36 : 2) * sizeof(double),

@@ -277,6 +277,7 @@ int sgpu_matrix_set_spmv(sgpu_matrix m, int32_t precision, int32_t format, int32
   p.format = format;
   p.variant = variant;
   p.tuned = true;
+  p.pinned = true;
   return SGPU_OK;
 }
 

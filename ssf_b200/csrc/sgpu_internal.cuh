@@ -89,6 +89,7 @@ struct Csr {
   DevBuf<double> dscale;     // 1 / sqrt(a_ii)
   bool have32 = false;
   bool diag_positive = false;
+  int longest = 0;           // entries of the longest row; 0 not yet known
 };
 
 // 3x3 block rows (BSR3): node-blocked form of a CSR whose equations come in
@@ -103,6 +104,7 @@ struct Bsr3 {
   DevBuf<int64_t> csr2bsr;  // CSR entry -> position in bval (for value updates)
   bool valid = false;
   bool have32 = false;
+  int longest = 0;  // blocks of the longest block row; 0 not yet known
   // most blocks in one tile of 32 block rows (the FP32 level-0 products that
   // stream tiles through shared memory); 0 not yet known
   int tile_cap = 0;
@@ -128,6 +130,7 @@ struct SpmvPlan {
   int format = 0;   // 0 CSR, 2 sliced ELL (FP64), 3 BSR3
   int variant = 0;  // kernel variant id
   bool tuned = false;
+  bool pinned = false;  // set by the caller (or the environment): the FP64 solve iterates with it too
 };
 
 // ---------------------------------------------------------------------------
@@ -161,6 +164,8 @@ struct Work {
   DevBuf<double> partials;              // block partial sums
   DevBuf<unsigned> counters;            // last-block tickets
   DevBuf<unsigned char> scal;           // PcgState (see sgpu_pcg.cu)
+  DevBuf<double> pair;                  // {direction, preconditioned residual} per equation (resident solve)
+  DevBuf<unsigned char> gsync;          // GridSync (sgpu_persist.cuh)
 };
 
 }  // namespace sgpu
@@ -182,6 +187,7 @@ struct sgpu_matrix_s {
   sgpu::Bsr3 bsr;
   sgpu::Sell sell;
   sgpu::SpmvPlan plan64, plan32;
+  sgpu::SpmvPlan used64;  // what the last FP64 solve iterated with (reported)
   sgpu::Work w;
   cudaStream_t stream = nullptr;      // stream all work of the handle runs on
   cudaStream_t own_stream = nullptr;  // the handle's own (created) stream

@@ -175,6 +175,7 @@ __global__ void k_bsr3_check(int nb, const int *__restrict__ rowptr, const int *
                              int *__restrict__ blen, unsigned *err) {
   int lane = threadIdx.x & 31;
   for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb; b += (gridDim.x * blockDim.x) >> 5) {
+    if (*(volatile unsigned *)err) return;  // not node-blocked: nothing here is used
     int r0 = rowptr[3 * b], r1 = rowptr[3 * b + 1], r2 = rowptr[3 * b + 2], r3 = rowptr[3 * b + 3];
     int len = r1 - r0;
     bool ok = (r2 - r1 == len) && (r3 - r2 == len) && (len % 3 == 0);
@@ -289,8 +290,8 @@ int matrix_build_from_device_src(sgpu_matrix m) {
   const int nnz32 = (int)nnz;
   SGPU_CUDA(cudaMemcpy(c.rowptr.p + n, &nnz32, sizeof(int), cudaMemcpyHostToDevice));
   c.nnz = nnz;
-  SGPU_TRY(c.col.alloc(nnz));
-  SGPU_TRY(c.val.alloc(nnz));
+  SGPU_TRY(c.col.alloc(nnz + 4));
+  SGPU_TRY(c.val.alloc(nnz + 2));
   SGPU_TRY(c.diag.alloc(n));
   SGPU_TRY(m->map_lo.alloc(negm));
   SGPU_TRY(m->map_up.alloc(negm));
@@ -540,7 +541,7 @@ int ensure_bsr3(sgpu_matrix m) {
   // 16 bytes of slack after the columns and the FP32 values: bulk copies of
   // whole tiles round their end up to a 16-byte boundary
   SGPU_TRY(b.bcol.alloc((size_t)nblk + 4));
-  SGPU_TRY(b.bval.alloc((size_t)nblk * 9));
+  SGPU_TRY(b.bval.alloc((size_t)nblk * 9 + 2));
   SGPU_TRY(b.csr2bsr.alloc(c.nnz));
   k_bsr3_fill<<<blocks_for((int64_t)nb * 32), TPB, 0, s>>>(nb, c.rowptr.p, c.col.p, b.browptr.p, b.bcol.p,
                                                            b.csr2bsr.p);

@@ -4,14 +4,17 @@
 //   p = A d; denom = d.p; alpha = nom/denom; x += alpha d; r -= alpha p;
 //   rr = r.r; h = r/diag; nom' = r.h; beta = nom'/nom; stop on rr/(f.f) < res;
 //   d = beta d + h.
-// Here one iteration is three kernels:
+// The whole iteration runs inside one cooperative launch (sgpu_persist.cuh):
+// with the matrix in shared memory where it fits the SMs, else streamed
+// through it.  Rows too long or too many for its stages, and a product pinned
+// by the caller, take the general form, three kernels per iteration:
 //   K_A  spmv + d.p  (last block: alpha, breakdown test)
 //   K_B  x,r update, h = r/diag, r.r and r.h (last block: beta, stop test)
 //   K_C  d = beta d + h
 // Reductions are deterministic: every block writes one partial, the last block
 // to arrive (atomic ticket, no waiting) sums the partials in block order.
-// G iterations are captured in one CUDA graph; every kernel returns at once
-// when the device-side state says the iteration has stopped, so a graph
+// There G iterations are captured in one CUDA graph; every kernel returns at
+// once when the device-side state says the iteration has stopped, so a graph
 // launched past convergence costs only empty launches.
 //
 // The mixed form iterates CG in FP32 on the Jacobi-scaled matrix
@@ -35,6 +38,7 @@
 #include <type_traits>
 
 #include "sgpu_internal.cuh"
+#include "sgpu_persist.cuh"
 
 namespace sgpu {
 
@@ -509,6 +513,21 @@ __global__ void __launch_bounds__(TPB) k_resid_norm(int n, const double *__restr
   }
 }
 
+// the resident solve's pairs after the host confirmed: h replaced
+__global__ void k_pair_h(int n, const double *__restrict__ h, double2 *__restrict__ dh) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dh[i].y = h[i];
+}
+
+// the longest row (units of ptr)
+__global__ void k_longest(int units, const int *__restrict__ ptr, int *out) {
+  int most = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < units; i += gridDim.x * blockDim.x)
+    most = max(most, ptr[i + 1] - ptr[i]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(out, most);
+}
+
 __global__ void k_fill(int n, double *__restrict__ a, double v) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a[i] = v;
 }
@@ -918,7 +937,7 @@ int spmv_autotune(sgpu_matrix m, int precision) {
     int f = -1, v = 0;
     if (sscanf(pin, "%d:%d", &f, &v) >= 1) {
       for (const Cand &c : cands)
-        if (c.format == f && c.variant == v) { p.format = f; p.variant = v; }
+        if (c.format == f && c.variant == v) { p.format = f; p.variant = v; p.pinned = true; }
     }
   } else {
     std::lock_guard<std::mutex> lk(g_plan_mu);
@@ -994,10 +1013,26 @@ int capture_fp32_chunk(sgpu_matrix m, int iters, cudaGraphExec_t *exec, int64_t 
   return SGPU_OK;
 }
 
+// The kernel of a solve's few plain products: the tuned one, else (no tuning
+// run for a handful of launches) the usual winner of its format.
+SpmvPlan plain_plan(sgpu_matrix m) {
+  if (m->plan64.tuned) return m->plan64;
+  SpmvPlan p;
+  if (m->bsr.nb >= 0 && m->bsr.valid) {
+    p.format = 3;
+    p.variant = 132;
+  } else {
+    const double mean = (double)m->csr.nnz / (double)m->n;
+    p.variant = mean > 40 ? 16 : (mean > 12 ? 8 : 4);
+  }
+  return p;
+}
+
 // true residual of the current w.x against w.f, into st->true_rel
 int true_residual(sgpu_matrix m, const double *x) {
   cudaStream_t s = m->stream;
-  SGPU_TRY(launch_spmv64<EpiNone>(m, m->plan64.format, m->plan64.variant, x, m->w.p.p, s, 0));
+  const SpmvPlan pl = plain_plan(m);
+  SGPU_TRY(launch_spmv64<EpiNone>(m, pl.format, pl.variant, x, m->w.p.p, s, 0));
   k_resid_norm<<<grid_for_vectors(), TPB, 0, s>>>((int)m->n, m->w.f.p, m->w.p.p, state_of(m), m->w.partials.p,
                                                   m->w.counters.p + 3);
   count_launches(1);
@@ -1005,13 +1040,70 @@ int true_residual(sgpu_matrix m, const double *x) {
 }
 
 constexpr int kChunk = 32;
+// iterations of one cooperative launch, between two reads of the state: below
+// a second at 1M equations
+constexpr long long kPersistChunk = 4096;
+
+// How an FP64 solve iterates.
+enum class Form { kResident, kTiles, kGraph };
+
+int longest_row(sgpu_matrix m, int units, const int *ptr, int *cached) {
+  if (*cached > 0) return SGPU_OK;
+  int *out = reinterpret_cast<int *>(m->w.counters.p + 8);
+  SGPU_CUDA(cudaMemsetAsync(out, 0, sizeof(int), m->stream));
+  k_longest<<<std::min((units + TPB - 1) / TPB, 4 * kNumSMs), TPB, 0, m->stream>>>(units, ptr, out);
+  count_launches(1);
+  SGPU_CUDA(cudaMemcpyAsync(cached, out, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+  SGPU_CUDA(cudaStreamSynchronize(m->stream));
+  return SGPU_OK;
+}
+
+// Resident where every row has a thread and the entries (12 bytes each) fit
+// the SMs' shared memory with 15 % to spare for uneven rows: 27,000 equations
+// in 1.96M entries took 8.6 us an iteration resident against 10.1 streamed,
+// 101,404 in 1.8M 8.1 against 10.7; 105,840 in 8M (a quarter fits) 28.5
+// against 19.  Streamed otherwise, in 3x3 blocks where the matrix has them.
+int choose_form(sgpu_matrix m, int sms, Form *form, TileMat *tm, int *longest, int *lanes) {
+  *form = Form::kGraph;
+  if (m->plan64.pinned || getenv("SGPU_SPMV64")) return SGPU_OK;
+  const Csr &c = m->csr;
+  if (resident_rows_fit(m->n, sms) && 12.0 * (double)c.nnz <= 0.85 * (double)sms * kResidentSmem) {
+    *form = Form::kResident;
+    m->used64.format = 0;
+    m->used64.variant = 0;
+    return SGPU_OK;
+  }
+  SGPU_TRY(ensure_bsr3(m));
+  Bsr3 &b = m->bsr;
+  *tm = b.valid ? TileMat{b.nb, b.browptr.p, b.bcol.p, b.bval.p, 0, 0, 0}
+                : TileMat{c.n, c.rowptr.p, c.col.p, c.val.p, 0, 0, 0};
+  SGPU_TRY(longest_row(m, tm->units, tm->ptr, b.valid ? &b.longest : &m->csr.longest));
+  *longest = b.valid ? b.longest : c.longest;
+  *lanes = b.valid ? tile_lanes<3>(*tm, *longest, sms) : tile_lanes<1>(*tm, *longest, sms);
+  if (*lanes > 0) {
+    *form = Form::kTiles;
+    m->used64.format = b.valid ? 3 : 0;
+    m->used64.variant = *lanes;
+  }
+  return SGPU_OK;
+}
 
 int solve_fp64(sgpu_matrix m, int64_t ni, double res, double zero, int64_t iv, int crit, int prec,
                PcgState *hs) {
   cudaStream_t s = m->stream;
   Work &w = m->w;
   const int n = (int)m->n;
-  if (!m->plan64.tuned) SGPU_TRY(spmv_autotune(m, 64));
+  const int vg = grid_for_vectors(), sms = resident_grid();
+  Form form;
+  TileMat tm{};
+  int longest = 0, lanes = 0;
+  SGPU_TRY(choose_form(m, sms, &form, &tm, &longest, &lanes));
+  SGPU_TRY(w.gsync.alloc(sizeof(GridSync)));
+  if (form == Form::kResident) SGPU_TRY(w.pair.alloc(2 * (size_t)n));
+  if (form == Form::kGraph) {
+    if (!m->plan64.tuned) SGPU_TRY(spmv_autotune(m, 64));
+    m->used64 = m->plan64;
+  }
   PcgState init{};
   init.ni = ni;
   init.res = res;
@@ -1020,29 +1112,49 @@ int solve_fp64(sgpu_matrix m, int64_t ni, double res, double zero, int64_t iv, i
   init.crit = crit;
   init.prec = prec;
   SGPU_TRY(write_state(m, &init));
-  // p = A x0 (x0 = 0 when iv == 0, as the reference zeroes x and multiplies)
   if (iv == 0) SGPU_CUDA(cudaMemsetAsync(w.x.p, 0, (size_t)n * sizeof(double), s));
-  SGPU_TRY(launch_spmv64<EpiNone>(m, m->plan64.format, m->plan64.variant, w.x.p, w.p.p, s, 0));
-  k_pcg64_init<<<grid_for_vectors(), TPB, 0, s>>>(n, w.f.p, w.p.p, m->csr.diag.p, w.r.p, w.h.p, w.d.p,
-                                                  state_of(m), w.partials.p, w.counters.p + 2);
-  count_launches(1);
+  const SpmvPlan pl = plain_plan(m);
+  if (form != Form::kResident) {  // the resident grid starts its solve itself
+    // p = A x0: zero for x0 = 0 (iv == 0, where the reference zeroes x and multiplies)
+    if (iv == 0) SGPU_CUDA(cudaMemsetAsync(w.p.p, 0, (size_t)n * sizeof(double), s));
+    else SGPU_TRY(launch_spmv64<EpiNone>(m, pl.format, pl.variant, w.x.p, w.p.p, s, 0));
+    k_pcg64_init<<<vg, TPB, 0, s>>>(n, w.f.p, w.p.p, m->csr.diag.p, w.r.p, w.h.p, w.d.p, state_of(m), w.partials.p,
+                                    w.counters.p + 2);
+    count_launches(1);
+  }
+  GridSync *gs = reinterpret_cast<GridSync *>(w.gsync.p);
+  ResidentArgs ra = {n,     m->csr.rowptr.p, m->csr.col.p, m->csr.val.p, m->csr.diag.p, w.f.p, w.x.p, w.r.p,
+                     reinterpret_cast<double2 *>(w.pair.p), state_of(m), gs, 0, 0, 1, (int)(iv != 0), kPersistChunk};
+  const TileArgs ta = {n, m->csr.diag.p, w.x.p, w.r.p, w.h.p, w.d.p, w.p.p, state_of(m), gs, kPersistChunk};
   cudaGraphExec_t exec = nullptr;
   int64_t nodes = 0;
-  SGPU_TRY(capture_fp64_chunk(m, kChunk, &exec, &nodes));
+  if (form == Form::kGraph) SGPU_TRY(capture_fp64_chunk(m, kChunk, &exec, &nodes));
   int rc = SGPU_OK;
   std::vector<double> confirms;
   for (;;) {
-    cudaError_t e = cudaGraphLaunch(exec, s);
-    if (e != cudaSuccess) { rc = fail(SGPU_CUDA_ERROR, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e)); break; }
-    count_launches(nodes);
+    cudaError_t e = cudaSuccess;
+    if (form == Form::kGraph) {
+      e = cudaGraphLaunch(exec, s);
+      count_launches(nodes);
+    } else {
+      e = cudaMemsetAsync(gs, 0, sizeof(GridSync), s);
+      if (e == cudaSuccess && form == Form::kResident) e = launch_resident(ra, m->csr.nnz, sms, s);
+      else if (e == cudaSuccess)
+        e = m->used64.format == 3 ? launch_tiles<3>(ta, tm, longest, lanes, sms, s)
+                                  : launch_tiles<1>(ta, tm, longest, lanes, sms, s);
+      ra.start = 0;
+      count_launches(1);
+    }
+    if (e != cudaSuccess) { rc = fail(SGPU_CUDA_ERROR, std::string("PCG launch: ") + cudaGetErrorString(e)); break; }
     rc = read_state(m, hs);
     if (rc != SGPU_OK) break;
+    if (hs->status == SGPU_CUDA_ERROR) { rc = fail(SGPU_CUDA_ERROR, "PCG: a wait inside the grid ran out"); break; }
     if (hs->done) break;
     if (hs->pause) {  // SGPU_CRIT_TRUE: confirm on the true residual
-      rc = launch_spmv64<EpiNone>(m, m->plan64.format, m->plan64.variant, w.x.p, w.p.p, s, 0);
+      rc = launch_spmv64<EpiNone>(m, pl.format, pl.variant, w.x.p, w.p.p, s, 0);
       if (rc != SGPU_OK) break;
-      k_pcg64_confirm<<<grid_for_vectors(), TPB, 0, s>>>(n, w.f.p, w.p.p, m->csr.diag.p, w.r.p, w.h.p,
-                                                         state_of(m), w.partials.p, w.counters.p + 2);
+      k_pcg64_confirm<<<vg, TPB, 0, s>>>(n, w.f.p, w.p.p, m->csr.diag.p, w.r.p, w.h.p, state_of(m), w.partials.p,
+                                         w.counters.p + 2);
       count_launches(1);
       rc = read_state(m, hs);
       if (rc != SGPU_OK || hs->done) break;
@@ -1062,11 +1174,12 @@ int solve_fp64(sgpu_matrix m, int64_t ni, double res, double zero, int64_t iv, i
         *hs = t;
         break;
       }
-      k_pcg64_dir<<<grid_for_vectors(), TPB, 0, s>>>(n, w.d.p, w.h.p, state_of(m));
+      if (form == Form::kResident) k_pair_h<<<vg, TPB, 0, s>>>(n, w.h.p, ra.dh);
+      else k_pcg64_dir<<<vg, TPB, 0, s>>>(n, w.d.p, w.h.p, state_of(m));
       count_launches(1);
     }
   }
-  cudaGraphExecDestroy(exec);
+  if (exec) cudaGraphExecDestroy(exec);
   return rc;
 }
 
@@ -1233,7 +1346,7 @@ int pcg_run(sgpu_matrix m, int64_t ni, double res, double zero, int64_t iv, int 
     else info->crit_value = sqrt(hs.rr / (hs.nory > 0 ? hs.nory : 1.0));
     info->true_relres = fin.true_rel;
     info->solve_ms = solve_ms;
-    const SpmvPlan &pl = mode == SGPU_MIXED ? m->plan32 : m->plan64;
+    const SpmvPlan &pl = mode == SGPU_MIXED ? m->plan32 : m->used64;
     info->spmv_format = pl.format;
     info->spmv_variant = pl.variant;
     info->spmv_bytes = spmv_bytes(m, pl.format, mode == SGPU_MIXED ? 32 : 64);

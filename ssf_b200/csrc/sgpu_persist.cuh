@@ -49,7 +49,19 @@ __device__ __forceinline__ double persist_warp_sum(double v) {
 struct GridSumShared {
   double part[2][32];  // per warp
   double tot[2];
+  int ok;  // written by thread 0 in each barrier
 };
+
+// thread 0: arrives and waits until every CTA has; false: gave up
+__device__ __forceinline__ bool grid_arrive_wait(GridSync *gs, unsigned target) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gs->arrived) : "memory");
+  unsigned c;
+  for (int tries = 0; tries < kPollLimit; tries++) {
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&gs->arrived) : "memory");
+    if (c >= target) return true;
+  }
+  return false;
+}
 
 // v: the thread's partial sums in, the grid's sums out (every thread); e: the
 // number of this barrier in the launch, from 1.  Orders every global write
@@ -64,7 +76,6 @@ __device__ __forceinline__ bool grid_barrier_sum(double (&v)[NV], GridSync *gs, 
     if (lane == 0) sh.part[q][w] = v[q];
   }
   __syncthreads();
-  bool ok = true;
   if (w == 0) {
     double t[NV];
 #pragma unroll
@@ -72,13 +83,7 @@ __device__ __forceinline__ bool grid_barrier_sum(double (&v)[NV], GridSync *gs, 
     if (lane == 0) {
 #pragma unroll
       for (int q = 0; q < NV; q++) __stcg(&gs->part[e & 1][q][blockIdx.x], t[q]);
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gs->arrived) : "memory");
-      unsigned c;
-      int tries = 0;
-      do {
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&gs->arrived) : "memory");
-        ok = ++tries < kPollLimit;
-      } while (c < e * (unsigned)G && ok);
+      sh.ok = grid_arrive_wait(gs, e * (unsigned)G);
     }
     __syncwarp();
     double s[NV];
@@ -98,10 +103,18 @@ __device__ __forceinline__ bool grid_barrier_sum(double (&v)[NV], GridSync *gs, 
       if (lane == 0) sh.tot[q] = s[q];
     }
   }
-  ok = __syncthreads_and(ok);
+  __syncthreads();
 #pragma unroll
   for (int q = 0; q < NV; q++) v[q] = sh.tot[q];
-  return ok;
+  return sh.ok != 0;
+}
+
+// The barrier alone (same counter, same numbering).
+__device__ __forceinline__ bool grid_barrier(GridSync *gs, unsigned e, GridSumShared &sh) {
+  __syncthreads();
+  if (threadIdx.x == 0) sh.ok = grid_arrive_wait(gs, e * gridDim.x);
+  __syncthreads();
+  return sh.ok != 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -445,6 +458,349 @@ inline cudaError_t launch_resident(ResidentArgs a, int64_t nnz, int grid, cudaSt
   if (r > 64) return launch_resident_t<8>(a, grid, s);
   if (r > 32) return launch_resident_t<16>(a, grid, s);
   return launch_resident_t<32>(a, grid, s);
+}
+
+
+// ---------------------------------------------------------------------------
+// the streaming iteration: matrices that do not fit the SMs
+// ---------------------------------------------------------------------------
+// One cooperative launch of a CTA per SM; a CTA owns a contiguous range of
+// rows.  Per iteration:
+//   product  p = A d over the CTA's rows, d.p
+//   barrier  alpha
+//   update   x, r, h over the CTA's rows; r.r, r.h
+//   barrier  beta, stopping test
+//   d = beta d + h
+//   barrier
+//
+// The matrix arrives by bulk copies (cp.async.bulk on an mbarrier) into
+// stages that belong to one warp each: a warp multiplies a tile, then its
+// lane 0 starts the copy of the tile `depth` ahead into the same stage.  The
+// order never ends: behind the last tile of an iteration comes the first of
+// the next, so the copies run on through the barriers and the vector phases,
+// and HBM works while the three-launch form had ramps, tails and gaps.  The
+// gathers of d stay plain loads (d changes between barriers); evict-first
+// copies leave L2 to the vectors.
+//
+// Measured per iteration (B200), against three launches per iteration in a
+// graph: 1,008,600 equations in 3x3 blocks (683 MB) 149.7 -> 129.4 us, of
+// which the bytes take 104.5 and the barriers and vectors about 12; 132,300
+// equations (84 MB, in L2) 33.1 -> 21.8 us; 481,200 equations of CSR (104
+// MB) 39.4 -> 27.8 us; 2,130,048 of CSR (640 MB) 196 -> 178 us.  Variants that
+// lost: plain loads instead of bulk copies (152 us on the first), 12 or 24
+// warps there (133 to 139), evict-last copies (157).  A second stage per warp
+// (LPR 16) lost to wider tiles (139): a tile's gathers, not its copy, are
+// what a warp waits for.
+__device__ __forceinline__ unsigned ring_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool ring_test(unsigned long long *bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(ring_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// bounded wait (a try_wait suspends for up to about a microsecond)
+__device__ __forceinline__ bool ring_wait(unsigned long long *bar, unsigned parity) {
+  for (int tries = 0; tries < kPollLimit; tries++)
+    if (ring_test(bar, parity)) return true;
+  return false;
+}
+
+// A matrix as units of rows: block rows of 3 (BSR3, values component-major
+// per block row) or single rows (CSR).  The arrays are readable for 16 bytes
+// past their last entry.
+struct TileMat {
+  int units;
+  const int *ptr;  // units + 1
+  const int *col;
+  const double *val;
+  int per;    // units of a CTA
+  int ent;    // entries a stage holds: the most any tile has
+  int depth;  // stages of a warp
+};
+
+// ROWS 1: CSR, ROWS 3: BSR3; LPR lanes per unit, tiles of 32 / LPR units.
+template <int ROWS, int LPR>
+struct TileKind {
+  static constexpr int kRows = ROWS;
+  static constexpr int kLpr = LPR;
+  static constexpr int kUnits = 32 / kLpr;
+  static constexpr int kVals = ROWS * ROWS;
+  __host__ __device__ static constexpr int val_bytes(int ent) { return (8 * (kVals * ent + 2) + 15) & ~15; }
+  __host__ __device__ static constexpr int stage_bytes(int ent) { return val_bytes(ent) + ((4 * (ent + 6) + 15) & ~15); }
+};
+
+struct TileArgs {
+  int n;
+  const double *diag;
+  double *x, *r, *h, *d, *p;
+  PcgState *st;
+  GridSync *gs;
+  long long most;
+};
+
+template <int ROWS, int LPR, int TPBX>
+__global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const TileMat m) {
+  using K = TileKind<ROWS, LPR>;
+  constexpr int kTileWarps = TPBX / 32;
+  extern __shared__ __align__(128) unsigned char ring[];
+  __shared__ GridSumShared sums;
+  __shared__ CgShared cg;
+  __shared__ int bad;
+  if (a.st->done | a.st->pause) return;  // the same in every CTA: this grid writes it after its last barrier
+  const int D = m.depth, vb = K::val_bytes(m.ent), sb = K::stage_bytes(m.ent);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned char *stages = ring + (size_t)w * D * sb;
+  unsigned long long *full = reinterpret_cast<unsigned long long *>(ring + (size_t)kTileWarps * D * sb) + w * D;
+  int *sp = reinterpret_cast<int *>(ring + (size_t)kTileWarps * D * (sb + 8));
+  const int u0 = blockIdx.x * m.per, nu = min(m.per, m.units - u0);  // >= 1: no CTA without units
+  const int ntiles = (nu + K::kUnits - 1) / K::kUnits;
+  const int mine = ntiles > w ? (ntiles - w + kTileWarps - 1) / kTileWarps : 0;  // the warp's tiles
+  cg.load(a.st);
+  for (int q = threadIdx.x; q <= nu; q += TPBX) sp[q] = m.ptr[u0 + q];
+  if (lane == 0)
+    for (int q = 0; q < D; q++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ring_u32(full + q)) : "memory");
+  if (threadIdx.x == 0) bad = 0;
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  const int prec = a.st->prec;
+  double nom = a.st->nom, beta = a.st->beta;
+  long long it = a.st->it;
+  __syncthreads();
+
+  unsigned long long policy;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  // lane 0: copies the warp's tile number j into stage q
+  auto issue = [&](int j, int q) {
+    const int t = w + kTileWarps * j;
+    const int e0 = sp[t * K::kUnits], e1 = sp[min((t + 1) * K::kUnits, nu)];
+    const long long v0 = ((long long)K::kVals * e0) & ~1ll, v1 = ((long long)K::kVals * e1 + 1) & ~1ll;
+    const int c0 = e0 & ~3, c1 = (e1 + 3) & ~3;
+    const unsigned nv = (unsigned)(8 * (v1 - v0)), nc = (unsigned)(4 * (c1 - c0));
+    unsigned char *dst = stages + (size_t)q * sb;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(ring_u32(full + q)), "r"(nv + nc)
+                 : "memory");
+    if (nv)
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+          ::"r"(ring_u32(dst)), "l"(m.val + v0), "r"(nv), "r"(ring_u32(full + q)), "l"(policy)
+          : "memory");
+    if (nc)
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+          ::"r"(ring_u32(dst + vb)), "l"(m.col + c0), "r"(nc), "r"(ring_u32(full + q)), "l"(policy)
+          : "memory");
+  };
+  int next = 0;       // the warp's next tile to copy (0 .. mine - 1, then the next iteration's first)
+  int q = 0;          // stage of the next tile to read
+  unsigned ph = 0;    // its phase
+  if (mine && lane == 0)
+    for (int z = 0; z < D; z++) {
+      issue(next, z);
+      if (++next == mine) next = 0;
+    }
+
+  const int r0 = u0 * K::kRows, r1 = (u0 + nu) * K::kRows;
+  unsigned epoch = 0;
+  bool ok = true;
+  for (long long k = 0; k < a.most; k++, it++) {
+    double acc = 0.0;
+    for (int j = 0; j < mine; j++) {
+      const int t = w + kTileWarps * j;
+      if (!ring_wait(full + q, ph)) {
+        bad = 1;
+        break;
+      }
+      const unsigned char *stage = stages + (size_t)q * sb;
+      const int t0 = t * K::kUnits, e0 = sp[t0];
+      const double *vals = reinterpret_cast<const double *>(stage) + ((K::kVals * e0) & 1);
+      const int *cols = reinterpret_cast<const int *>(stage + vb) + (e0 & 3);
+      const int sub = lane % LPR, u = t0 + lane / LPR;
+      if constexpr (ROWS == 1) {
+        double y = 0.0, y2 = 0.0;
+        if (u < nu) {
+          const int b = sp[u] - e0, len = sp[u + 1] - e0 - b;
+          const double *v = vals + b;
+          const int *c = cols + b;
+          constexpr int U = LPR == 2 ? 7 : 4;
+          for (int e = sub; e < len; e += LPR * U) {
+            double xx[U];
+#pragma unroll
+            for (int z = 0; z < U; z++) xx[z] = a.d[c[min(e + LPR * z, len - 1)]];
+#pragma unroll
+            for (int z = 0; z < U; z++) {
+              if (e + LPR * z < len) {
+                if (z & 1) y2 = fma(v[e + LPR * z], xx[z], y2);
+                else y = fma(v[e + LPR * z], xx[z], y);
+              }
+            }
+          }
+          y += y2;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int o = LPR / 2; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o, LPR);
+        if (sub == 0 && u < nu) {
+          a.p[u0 + u] = y;
+          acc += a.d[u0 + u] * y;
+        }
+      } else {
+        double y0 = 0.0, y1 = 0.0, y2 = 0.0;
+        if (u < nu) {
+          const int s = sp[u] - e0, nbr = sp[u + 1] - e0 - s;
+          const double *v = vals + 9 * s;
+          const int *c = cols + s;
+          constexpr int U = LPR == 8 ? 4 : (LPR == 16 ? 2 : 1);
+          for (int e = sub; e < nbr; e += LPR * U) {
+            double x0[U], x1[U], x2[U];
+#pragma unroll
+            for (int z = 0; z < U; z++) {
+              const double *xp = a.d + 3 * c[min(e + LPR * z, nbr - 1)];
+              x0[z] = xp[0];
+              x1[z] = xp[1];
+              x2[z] = xp[2];
+            }
+#pragma unroll
+            for (int z = 0; z < U; z++) {
+              const int jj = e + LPR * z;
+              if (jj < nbr) {
+                y0 += v[jj] * x0[z] + v[nbr + jj] * x1[z] + v[2 * nbr + jj] * x2[z];
+                y1 += v[3 * nbr + jj] * x0[z] + v[4 * nbr + jj] * x1[z] + v[5 * nbr + jj] * x2[z];
+                y2 += v[6 * nbr + jj] * x0[z] + v[7 * nbr + jj] * x1[z] + v[8 * nbr + jj] * x2[z];
+              }
+            }
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int o = LPR / 2; o > 0; o >>= 1) {
+          y0 += __shfl_xor_sync(0xffffffffu, y0, o, LPR);
+          y1 += __shfl_xor_sync(0xffffffffu, y1, o, LPR);
+          y2 += __shfl_xor_sync(0xffffffffu, y2, o, LPR);
+        }
+        if (sub < 3 && u < nu) {
+          const double yv = sub == 0 ? y0 : (sub == 1 ? y1 : y2);
+          const int i = 3 * (u0 + u) + sub;
+          a.p[i] = yv;
+          acc += a.d[i] * yv;
+        }
+      }
+      __syncwarp();  // the stage is read: the warp's next copy may overwrite it
+      if (lane == 0) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        issue(next, q);
+        if (++next == mine) next = 0;
+      }
+      if (++q == D) {
+        q = 0;
+        ph ^= 1;
+      }
+    }
+    double dp[1] = {acc}, alpha;
+    ok = grid_barrier_sum<1>(dp, a.gs, ++epoch, sums) && !bad;
+    if (!ok || cg.direction(dp[0], nom, alpha)) break;
+    double v[2] = {0.0, 0.0};
+#pragma unroll 4
+    for (int i = r0 + threadIdx.x; i < r1; i += TPBX) {
+      a.x[i] = fma(alpha, a.d[i], a.x[i]);
+      const double ri = fma(-alpha, a.p[i], a.r[i]);
+      const double hi = prec ? ri / __ldg(a.diag + i) : ri;
+      a.r[i] = ri;
+      a.h[i] = hi;
+      v[0] += ri * ri;
+      v[1] += ri * hi;
+    }
+    ok = grid_barrier_sum<2>(v, a.gs, ++epoch, sums);
+    if (!ok || cg.updated(v[0], v[1], it, nom, beta)) break;
+#pragma unroll 4
+    for (int i = r0 + threadIdx.x; i < r1; i += TPBX) a.d[i] = fma(beta, a.d[i], a.h[i]);
+    ok = grid_barrier(a.gs, ++epoch, sums);
+    if (!ok) break;
+  }
+  // the copies that nobody reads
+  if (mine && lane == 0)
+    for (int z = 0; z < D; z++) {
+      ring_wait(full + q, ph);
+      if (++q == D) {
+        q = 0;
+        ph ^= 1;
+      }
+    }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (!ok) {
+      cg.s.status = SGPU_CUDA_ERROR;
+      cg.s.done = 1;
+    }
+    *a.st = cg.s;
+  }
+}
+
+// The rule of the launch: the fewest lanes per unit whose stages (one per
+// warp at least) fit.  Fewer lanes mean wider tiles, fewer shuffles and more
+// gathers in flight per lane; the longest unit decides whether they fit
+// (8 lanes up to 43 blocks a row, 32 up to 166 of BSR3; 2 lanes up to 43
+// entries a row, 32 up to 700 of CSR).  BSR3 runs 16 warps of up to 128
+// registers, CSR, whose lanes hold less, 24.
+constexpr int kTileRing = 200 * 1024;    // stages
+constexpr int kTileSmem = 225 * 1024;    // with the unit pointers
+template <int ROWS>
+constexpr int kTileTPB = ROWS == 3 ? 512 : 768;
+
+template <int ROWS, int LPR>
+inline bool tiles_fit(const TileMat &m, int longest, int sms) {
+  using K = TileKind<ROWS, LPR>;
+  const int ent = (longest * K::kUnits + 3) & ~3, per = (m.units + sms - 1) / sms;
+  const int64_t stage = (int64_t)kTileTPB<ROWS> / 32 * (K::stage_bytes(ent) + 8);
+  return longest > 0 && longest < 4096 && stage <= kTileRing && stage + 4ll * (per + 1) <= kTileSmem;
+}
+
+template <int ROWS, int LPR>
+inline cudaError_t launch_tiles_as(const TileArgs &a, TileMat m, int longest, int sms, cudaStream_t s) {
+  using K = TileKind<ROWS, LPR>;
+  constexpr int TPBX = kTileTPB<ROWS>, W = TPBX / 32;
+  m.ent = (longest * K::kUnits + 3) & ~3;
+  m.per = (m.units + sms - 1) / sms;
+  const int grid = (m.units + m.per - 1) / m.per;  // no CTA without units
+  const int sb = K::stage_bytes(m.ent) + 8, ntiles = (m.per + K::kUnits - 1) / K::kUnits;
+  const int room = std::min(kTileRing, kTileSmem - 4 * (m.per + 1));
+  m.depth = std::min(room / (W * sb), (ntiles + W - 1) / W + 1);
+  const size_t smem = (size_t)W * m.depth * sb + 4ull * (m.per + 1);
+  auto k = k_pcg_tiles<ROWS, LPR, TPBX>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem);
+  if (e != cudaSuccess) return e;
+  TileArgs args = a;
+  void *p[] = {&args, &m};
+  return cudaLaunchCooperativeKernel((const void *)k, dim3(grid), dim3(TPBX), p, smem, s);
+}
+
+// lanes per unit (0: the rows are too long or too many for the tiles)
+template <int ROWS>
+inline int tile_lanes(const TileMat &m, int longest, int sms) {
+  if (sms <= 0) return 0;
+  if constexpr (ROWS == 3) {
+    if (tiles_fit<3, 8>(m, longest, sms)) return 8;
+    if (tiles_fit<3, 16>(m, longest, sms)) return 16;
+    if (tiles_fit<3, 32>(m, longest, sms)) return 32;
+  } else {
+    if (tiles_fit<1, 2>(m, longest, sms)) return 2;
+    if (tiles_fit<1, 8>(m, longest, sms)) return 8;
+    if (tiles_fit<1, 32>(m, longest, sms)) return 32;
+  }
+  return 0;
+}
+template <int ROWS>
+inline cudaError_t launch_tiles(const TileArgs &a, const TileMat &m, int longest, int lanes, int sms, cudaStream_t s) {
+  if constexpr (ROWS == 3) {
+    if (lanes == 8) return launch_tiles_as<3, 8>(a, m, longest, sms, s);
+    if (lanes == 16) return launch_tiles_as<3, 16>(a, m, longest, sms, s);
+    return launch_tiles_as<3, 32>(a, m, longest, sms, s);
+  } else {
+    if (lanes == 2) return launch_tiles_as<1, 2>(a, m, longest, sms, s);
+    if (lanes == 8) return launch_tiles_as<1, 8>(a, m, longest, sms, s);
+    return launch_tiles_as<1, 32>(a, m, longest, sms, s);
+  }
 }
 
 }  // namespace sgpu

@@ -213,8 +213,8 @@ SGPU_API int sgpu_matrix_combine(sgpu_matrix K, sgpu_matrix C, double a, double 
   const int64_t n = K->n, nnz = K->csr.nnz, negm = K->src_negm;
   int st;
   if ((st = m->src_adr.alloc(n + 1)) || (st = m->src_ci.alloc(negm)) || (st = m->map_lo.alloc(negm)) ||
-      (st = m->map_up.alloc(negm)) || (st = m->csr.rowptr.alloc(n + 1)) || (st = m->csr.col.alloc(nnz)) ||
-      (st = m->csr.val.alloc(nnz)) || (st = m->csr.diag.alloc(n)))
+      (st = m->map_up.alloc(negm)) || (st = m->csr.rowptr.alloc(n + 1)) || (st = m->csr.col.alloc(nnz + 4)) ||
+      (st = m->csr.val.alloc(nnz + 2)) || (st = m->csr.diag.alloc(n)))
     return bail(st);
   m->csr.n = (int)n;
   m->csr.nnz = nnz;
