@@ -11,10 +11,11 @@
 // conductivity_matrix / capacity_matrix (TRFEL/SRC/globmatt.cpp:19/92).
 //
 // Here:
-//  1. pattern: every element emits its (row, col <= row) equation pairs as
-//     64-bit keys; one radix sort + unique gives the SCR pattern
-//     (symcomprow::initiate, GEFEL/scr.cpp:556), from which the full CSR is
-//     built (sgpu_matrix.cu);
+//  1. pattern: each node's sorted neighbours give its rows of the full CSR;
+//     for code numbers not in node order every element emits its (row, col <=
+//     row) equation pairs as 64-bit keys, and one radix sort + unique gives
+//     the SCR pattern (symcomprow::initiate, GEFEL/scr.cpp:556), from which
+//     the full CSR is built (sgpu_matrix.cu);
 //  2. colouring: greedy first-fit on the host over node masks -- elements of
 //     one colour share no node, so their element matrices can be added into
 //     the CSR without atomics, and the sum order is fixed (deterministic);
@@ -116,15 +117,43 @@ __global__ void k_inc_fill(int64_t m, int nne, const int64_t *__restrict__ elems
   }
 }
 
-// one warp per node i: the sorted distinct nodes j <= i that share an element
-// with i (bitonic sort of the candidates in shared memory).  FILL = false
-// counts them into ucnt[i]; FILL = true writes them at nptr[i].  A node with
-// more than kAdjCap candidates sets err bit 16 (the caller falls back).
-template <bool FILL>
-__global__ void __launch_bounds__(TPB) k_node_adj(int64_t nn, int nne, const int64_t *__restrict__ elems,
+// Code numbers as gencodnum gives them (consecutive in node, component
+// order): code[q] = the 0-based equation, -1 for none.  free_before is the
+// exclusive scan of "cn > 0", so a positive code number must be one more than
+// it; err bit 32 otherwise, bit 64 where a node has some components free and
+// some not.
+__global__ void k_code_flags(int64_t m, const int64_t *__restrict__ cn, int *__restrict__ flag) {
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < m; q += (int64_t)gridDim.x * blockDim.x)
+    flag[q] = cn[q] > 0;
+}
+__global__ void k_codes(int64_t m, int ndofn, const int64_t *__restrict__ cn, const int *__restrict__ free_before,
+                        int *__restrict__ code, unsigned *err) {
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < m; q += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = cn[q];
+    int v = -1;
+    if (c > 0) {
+      v = free_before[q];
+      if (c != (int64_t)v + 1) atomicOr(err, 32u);
+    }
+    code[q] = v;
+    if (q % ndofn && (c > 0) != (cn[q - 1] > 0)) atomicOr(err, 64u);
+  }
+}
+
+// one warp per node i: the sorted distinct nodes that share an element with
+// i (i among them), at nadj[nne * iptr[i]] -- the candidates' own number, so
+// one pass needs no count before it.  cnt[i]: how many; len[i]: entries of
+// i's rows (components times free components of the list).  Up to 64
+// candidates are sorted in registers, two per lane; more (quadratic elements)
+// bitonically in shared memory.  A node with more than kAdjCap candidates
+// sets err bit 16 (the caller falls back), one with equations but no element
+// bit 2.
+// On the 1.01M-equation cantilever (344,000 nodes of 64 candidates) the list
+// of the lower neighbours took two passes of 0.37 ms in shared memory.
+__global__ void __launch_bounds__(TPB) k_node_adj(int64_t nn, int nne, int ndofn, const int64_t *__restrict__ elems,
                                                   const int *__restrict__ iptr, const int *__restrict__ inc,
-                                                  int *__restrict__ ucnt, const int64_t *__restrict__ nptr,
-                                                  int *__restrict__ nadj, unsigned *err) {
+                                                  const int *__restrict__ code, int *__restrict__ cnt,
+                                                  int *__restrict__ len, int *__restrict__ nadj, unsigned *err) {
   __shared__ int buf[WPB][kAdjCap];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   int *sb = buf[wib];
@@ -132,98 +161,127 @@ __global__ void __launch_bounds__(TPB) k_node_adj(int64_t nn, int nne, const int
     const int b = iptr[i], e = iptr[i + 1];
     const int ncand = (e - b) * nne;
     if (ncand > kAdjCap) {
-      if (lane == 0) atomicOr(err, 16u);
+      if (lane == 0) {
+        atomicOr(err, 16u);
+        cnt[i] = 0;
+        len[i] = 0;
+      }
       continue;
     }
-    int P = 32;
-    while (P < ncand) P <<= 1;
-    for (int q = lane; q < P; q += 32) {
-      int v = INT_MAX;
-      if (q < ncand) {
-        const int64_t j = elems[(int64_t)inc[b + q / nne] * nne + q % nne];
-        if (j <= i) v = (int)j;
+    int *out = nadj + (int64_t)nne * b;
+    int total = 0, nfree = 0;
+    if (ncand <= 64) {
+      int v[2];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int q = 2 * lane + h;
+        v[h] = q < ncand ? (int)elems[(int64_t)inc[b + q / nne] * nne + q % nne] : INT_MAX;
       }
-      sb[q] = v;
-    }
-    __syncwarp();
-    for (int k = 2; k <= P; k <<= 1)
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        for (int q = lane; q < P; q += 32) {
-          const int x = q ^ j;
-          if (x > q) {
-            const int a = sb[q], c = sb[x];
-            if ((a > c) == ((q & k) == 0)) {
-              sb[q] = c;
-              sb[x] = a;
-            }
+      // element 2 lane + h: a partner at distance 1 is the lane's other value
+#pragma unroll
+      for (int k = 2; k <= 64; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 1; j >>= 1) {
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int q = 2 * lane + h;
+            const int other = __shfl_xor_sync(0xffffffffu, v[h], j >> 1);
+            const bool up = (q & k) == 0, low = (q & j) == 0;
+            v[h] = (up == low) ? min(v[h], other) : max(v[h], other);
           }
         }
-        __syncwarp();
+        const bool up = ((2 * lane) & k) == 0;
+        const int lo = min(v[0], v[1]), hi = max(v[0], v[1]);
+        v[0] = up ? lo : hi;
+        v[1] = up ? hi : lo;
       }
-    int total = 0;
-    for (int q0 = 0; q0 < P; q0 += 32) {
-      const int q = q0 + lane;
-      const bool keep = q < P && sb[q] != INT_MAX && (q == 0 || sb[q] != sb[q - 1]);
-      const unsigned bal = __ballot_sync(0xffffffffu, keep);
-      if (FILL && keep) nadj[nptr[i] + total + __popc(bal & ((1u << lane) - 1u))] = sb[q];
-      total += __popc(bal);
-    }
-    if (!FILL && lane == 0) ucnt[i] = total;
-    __syncwarp();
-  }
-}
-
-// SCR row lengths from the node adjacency, for code numbers that grow with
-// (node, component): row (i, c) holds the free components of every lower
-// neighbour j < i and the free components d <= c of i itself
-__global__ void k_scr_rowlen(int64_t nn, int ndofn, const int64_t *__restrict__ cn, const int64_t *__restrict__ nptr,
-                             const int *__restrict__ nadj, int64_t *__restrict__ rowlen, int64_t n, unsigned *err) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nn; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t base = 0;
-    bool self = false;
-    for (int64_t q = nptr[i]; q < nptr[i + 1]; q++) {
-      const int j = nadj[q];
-      if (j == i) {
-        self = true;
-        continue;
-      }
-      for (int d = 0; d < ndofn; d++) base += cn[(int64_t)j * ndofn + d] > 0;
-    }
-    int own = 0;
-    for (int c = 0; c < ndofn; c++) {
-      const int64_t r = cn[i * ndofn + c];
-      if (r <= 0) continue;
-      own++;
-      if (r > n) {
-        atomicOr(err, 1u);
-        continue;
-      }
-      if (!self) atomicOr(err, 2u);  // an equation no element touches
-      rowlen[r - 1] = base + own;
-    }
-  }
-}
-
-__global__ void k_scr_fill(int64_t nn, int ndofn, const int64_t *__restrict__ cn, const int64_t *__restrict__ nptr,
-                           const int *__restrict__ nadj, const int64_t *__restrict__ adr, int64_t *__restrict__ ci,
-                           int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nn; i += (int64_t)gridDim.x * blockDim.x) {
-    for (int c = 0; c < ndofn; c++) {
-      const int64_t r = cn[i * ndofn + c];
-      if (r <= 0 || r > n) continue;
-      int64_t w = adr[r - 1];
-      for (int64_t q = nptr[i]; q < nptr[i + 1]; q++) {
-        const int j = nadj[q];
-        if (j == i) continue;
-        for (int d = 0; d < ndofn; d++) {
-          const int64_t cc = cn[(int64_t)j * ndofn + d];
-          if (cc > 0) ci[w++] = cc - 1;
+      const int before = __shfl_up_sync(0xffffffffu, v[1], 1);
+      const bool keep0 = v[0] != INT_MAX && (lane == 0 || v[0] != before), keep1 = v[1] != INT_MAX && v[1] != v[0];
+      const unsigned b0 = __ballot_sync(0xffffffffu, keep0), b1 = __ballot_sync(0xffffffffu, keep1);
+      const unsigned below = (1u << lane) - 1u;
+      const int at = __popc(b0 & below) + __popc(b1 & below);
+      if (keep0) out[at] = v[0];
+      if (keep1) out[at + keep0] = v[1];
+      total = __popc(b0) + __popc(b1);
+      for (int c = 0; c < ndofn; c++)
+        nfree += (keep0 && code[(int64_t)v[0] * ndofn + c] >= 0) + (keep1 && code[(int64_t)v[1] * ndofn + c] >= 0);
+    } else {
+      int P = 128;
+      while (P < ncand) P <<= 1;
+      for (int q = lane; q < P; q += 32)
+        sb[q] = q < ncand ? (int)elems[(int64_t)inc[b + q / nne] * nne + q % nne] : INT_MAX;
+      __syncwarp();
+      for (int k = 2; k <= P; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+          for (int q = lane; q < P; q += 32) {
+            const int x = q ^ j;
+            if (x > q) {
+              const int a = sb[q], c = sb[x];
+              if ((a > c) == ((q & k) == 0)) {
+                sb[q] = c;
+                sb[x] = a;
+              }
+            }
+          }
+          __syncwarp();
         }
+      for (int q0 = 0; q0 < P; q0 += 32) {
+        const int q = q0 + lane;
+        const int v = sb[q];
+        const bool keep = v != INT_MAX && (q == 0 || v != sb[q - 1]);
+        const unsigned bal = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          out[total + __popc(bal & ((1u << lane) - 1u))] = v;
+          for (int c = 0; c < ndofn; c++) nfree += code[(int64_t)v * ndofn + c] >= 0;
+        }
+        total += __popc(bal);
       }
-      for (int d = 0; d <= c; d++) {
-        const int64_t cc = cn[i * ndofn + d];
-        if (cc > 0) ci[w++] = cc - 1;
-      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nfree += __shfl_xor_sync(0xffffffffu, nfree, o);
+    if (lane == 0) {
+      int own = 0;
+      for (int c = 0; c < ndofn; c++) own += code[i * ndofn + c] >= 0;
+      cnt[i] = total;
+      len[i] = own * nfree;
+      if (own && !total) atomicOr(err, 2u);  // an equation no element touches
+    }
+  }
+}
+
+// one warp per node: the rows of its equations, all with the same columns --
+// the free components of its neighbours.  row0: exclusive scan of len.
+__global__ void __launch_bounds__(TPB) k_csr_fill(int64_t nn, int nne, int ndofn, const int *__restrict__ iptr,
+                                                  const int *__restrict__ code, const int *__restrict__ cnt,
+                                                  const int *__restrict__ len, const int *__restrict__ row0,
+                                                  const int *__restrict__ nadj, int *__restrict__ rowptr,
+                                                  int *__restrict__ col, int n) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < nn;
+       i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    if (i == nn - 1 && lane == 0) rowptr[n] = row0[nn];
+    const int L = len[i];
+    if (L == 0) continue;
+    int own = 0, first = -1;
+    for (int c = 0; c < ndofn; c++) {
+      const int r = code[i * ndofn + c];
+      if (r >= 0 && first < 0) first = r;
+      own += r >= 0;
+    }
+    const int w = L / own, base = row0[i];
+    if (lane < own) rowptr[first + lane] = base + lane * w;
+    const int *list = nadj + (int64_t)nne * iptr[i];
+    const int m = cnt[i] * ndofn;  // candidate columns: (neighbour, component)
+    int done = 0;
+    for (int q0 = 0; q0 < m; q0 += 32) {
+      const int q = q0 + lane;
+      const int cc = q < m ? code[(int64_t)list[q / ndofn] * ndofn + q % ndofn] : -1;
+      const unsigned bal = __ballot_sync(0xffffffffu, cc >= 0);
+      const int at = done + __popc(bal & ((1u << lane) - 1u));
+      if (cc >= 0)
+        for (int c = 0; c < own; c++) col[base + c * w + at] = cc;
+      done += __popc(bal);
     }
   }
 }
@@ -2022,49 +2080,71 @@ int build_incidence(const int64_t *elems_d, int64_t nn, int64_t ne, int nne, Dev
   return SGPU_OK;
 }
 
-// The SCR pattern from the node adjacency when the code numbers grow with
-// (node, component) (gencodnum's numbering): from the node -> element
-// incidence (build_incidence), per-node sorted lower neighbours, row
-// lengths, scan, fill.  Returns
-// SGPU_OK, or 1 when a node has too many candidate neighbours (the caller
-// uses the element-pair sort instead).  Writes m->src_adr / src_ci / src_negm.
-int pattern_adjacency(sgpu_matrix m, const int64_t *elems_d, const int64_t *cn_d, int64_t nn, int nne, int ndofn,
-                      int64_t n, const int *iptr_d, const int *inc_d, unsigned *err_d, cudaStream_t s) {
-  AsyncBuf<int> ucnt(s), nadj(s);
-  AsyncBuf<int64_t> nptr(s), rowlen(s);
-  SGPU_TRY(ucnt.alloc(nn + 1));
-  SGPU_CUDA(cudaMemsetAsync(ucnt.p, 0, (nn + 1) * sizeof(int), s));
-  const int gadj = (int)std::min<int64_t>((nn + WPB - 1) / WPB, (int64_t)kNumSMs * 32);
-  k_node_adj<false><<<gadj, TPB, 0, s>>>(nn, nne, elems_d, iptr_d, inc_d, ucnt.p, nullptr, nullptr, err_d);
+// Code numbers on the device (k_codes): their 0-based equations in code_d,
+// the number of positive ones and the error bits set so far.
+int examine_codes(const int64_t *cn_d, int64_t ncode, int ndofn, int *code_d, unsigned *err_d, int *nfree,
+                  unsigned *flags, cudaStream_t s) {
+  AsyncBuf<int> flag(s), before(s);
+  SGPU_TRY(flag.alloc(ncode + 1));
+  SGPU_TRY(before.alloc(ncode + 1));
+  SGPU_CUDA(cudaMemsetAsync(flag.p + ncode, 0, sizeof(int), s));
+  k_code_flags<<<blocks_for(ncode), TPB, 0, s>>>(ncode, cn_d, flag.p);
   count_launches(1);
+  SGPU_TRY(scan_into(flag.p, before.p, ncode, s));
+  k_codes<<<blocks_for(ncode), TPB, 0, s>>>(ncode, ndofn, cn_d, before.p, code_d, err_d);
+  count_launches(1);
+  SGPU_CUDA(cudaMemcpyAsync(nfree, before.p + ncode, sizeof(int), cudaMemcpyDeviceToHost, s));
+  return read_err(err_d, s, flags);
+}
+
+// The full CSR pattern from the node adjacency when the code numbers are
+// gencodnum's (code_d from k_codes): per-node sorted neighbours, row lengths,
+// scan, fill.  Returns SGPU_OK, or 1 when a node has too many candidate
+// neighbours (the caller uses the element-pair sort instead).  The rows are
+// symmetric and complete, so the SCR form (and the maps from it, built when
+// values arrive in its order) follow from them; node_blocked says that every
+// node is free or fixed as a whole.
+int pattern_adjacency(sgpu_matrix m, const int64_t *elems_d, const int *code_d, int64_t nn, int64_t ne, int nne,
+                      int ndofn, int64_t n, const int *iptr_d, const int *inc_d, unsigned *err_d, bool node_blocked,
+                      cudaStream_t s) {
+  AsyncBuf<int> cnt(s), len(s), nadj(s), row0(s);
+  SGPU_TRY(cnt.alloc(nn));
+  SGPU_TRY(len.alloc(nn + 1));
+  SGPU_TRY(row0.alloc(nn + 1));
+  SGPU_TRY(nadj.alloc((size_t)ne * nne * nne));
+  SGPU_CUDA(cudaMemsetAsync(len.p + nn, 0, sizeof(int), s));
+  const int gadj = (int)std::min<int64_t>((nn + WPB - 1) / WPB, (int64_t)kNumSMs * 32);
+  k_node_adj<<<gadj, TPB, 0, s>>>(nn, nne, ndofn, elems_d, iptr_d, inc_d, code_d, cnt.p, len.p, nadj.p, err_d);
+  count_launches(1);
+  AsyncBuf<int64_t> total(s);  // the row lengths may add up past int32
+  {
+    SGPU_TRY(total.alloc(1));
+    size_t tmp = 0;
+    cub::DeviceReduce::Reduce(nullptr, tmp, len.p, total.p, (int)nn, cuda::std::plus<int64_t>(), (int64_t)0, s);
+    AsyncBuf<unsigned char> t(s);
+    SGPU_TRY(t.alloc(tmp));
+    cub::DeviceReduce::Reduce(t.p, tmp, len.p, total.p, (int)nn, cuda::std::plus<int64_t>(), (int64_t)0, s);
+    count_launches(1);
+  }
+  SGPU_TRY(scan_into(len.p, row0.p, nn, s));
+  int64_t nnz = 0;
+  SGPU_CUDA(cudaMemcpyAsync(&nnz, total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   unsigned e = 0;
   SGPU_TRY(read_err(err_d, s, &e));
   if (e & 16u) {
     SGPU_CUDA(cudaMemsetAsync(err_d, 0, sizeof(unsigned), s));
     return 1;
   }
-  SGPU_TRY(nptr.alloc(nn + 1));
-  SGPU_TRY(scan_into(ucnt.p, nptr.p, nn, s));
-  int64_t nadj_total = 0;
-  SGPU_CUDA(cudaMemcpyAsync(&nadj_total, nptr.p + nn, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  SGPU_CUDA(cudaStreamSynchronize(s));
-  SGPU_TRY(nadj.alloc((size_t)nadj_total));
-  k_node_adj<true><<<gadj, TPB, 0, s>>>(nn, nne, elems_d, iptr_d, inc_d, nullptr, nptr.p, nadj.p, err_d);
-  SGPU_TRY(rowlen.alloc(n + 1));
-  SGPU_CUDA(cudaMemsetAsync(rowlen.p, 0, (n + 1) * sizeof(int64_t), s));
-  k_scr_rowlen<<<blocks_for(nn), TPB, 0, s>>>(nn, ndofn, cn_d, nptr.p, nadj.p, rowlen.p, n, err_d);
-  count_launches(2);
-  SGPU_TRY(m->src_adr.alloc(n + 1));
-  SGPU_TRY(scan_into(rowlen.p, m->src_adr.p, n, s));
-  int64_t negm = 0;
-  SGPU_CUDA(cudaMemcpyAsync(&negm, m->src_adr.p + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  SGPU_TRY(read_err(err_d, s, &e));
-  if (e) return fail(SGPU_BAD_INPUT, "code numbers: element node out of range or unused equation");
-  m->src_negm = negm;
-  SGPU_TRY(m->src_ci.alloc(negm));
-  k_scr_fill<<<blocks_for(nn), TPB, 0, s>>>(nn, ndofn, cn_d, nptr.p, nadj.p, m->src_adr.p, m->src_ci.p, n);
+  if (e & 3u) return fail(SGPU_BAD_INPUT, "code numbers: element node out of range or unused equation");
+  if (nnz >= (1LL << 31) - 1) return fail(SGPU_BAD_INPUT, "matrix too large for int32 device indices");
+  Csr &c = m->csr;
+  SGPU_TRY(matrix_alloc_csr(m, n, nnz));
+  m->src_negm = (nnz + n) / 2;
+  k_csr_fill<<<(int)std::min<int64_t>((nn + WPB - 1) / WPB, (int64_t)kNumSMs * 64), TPB, 0, s>>>(
+      nn, nne, ndofn, iptr_d, code_d, cnt.p, len.p, row0.p, nadj.p, c.rowptr.p, c.col.p, (int)n);
   count_launches(1);
   SGPU_CUDA(cudaGetLastError());
+  m->bsr.known = node_blocked && ndofn == 3;
   return SGPU_OK;
 }
 
@@ -2301,15 +2381,7 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   if (mesh->ne > (1LL << 31) - 1) return fail(SGPU_BAD_INPUT, "too many elements");
   const int64_t nn = mesh->nn, ne = mesh->ne;
   const int ndofe = nne * ndofn;
-  // number of equations = largest code number
-  int64_t n = 0;
-  for (int64_t q = 0; q < nn * ndofn; q++) n = std::max<int64_t>(n, mesh->cn[q]);
-  if (n <= 0) return fail(SGPU_BAD_INPUT, "no free equations");
-  for (int64_t q = 0; q < ne * nne; q++)
-    if (mesh->elems[q] < 0 || mesh->elems[q] >= nn) return fail(SGPU_BAD_INPUT, "element node out of range");
-
   sgpu_matrix m = new sgpu_matrix_s();
-  m->n = n;
   m->src_sym = 1;
   auto bail = [&](int st) {
     if (m->stream) cudaStreamSynchronize(m->stream);
@@ -2369,21 +2441,28 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   cudaMemsetAsync(err.p, 0, sizeof(unsigned), s);
   k_elem_codes<<<blocks_for(ne * ndofe), TPB, 0, s>>>(ne, nne, ndofn, ad.elems.p, cn_d.p, ad.cne.p, err.p, nn);
   count_launches(1);
+  // are the code numbers gencodnum's (consecutive in node, component order)?
+  // Then their count is the number of equations.
+  const int64_t ncode = nn * ndofn;
+  if (ncode > (1LL << 31) - 2) return bail(fail(SGPU_BAD_INPUT, "too many nodes"));
+  DevBuf<int> code;
+  BAIL_ON(code.alloc(ncode));
+  int nfree = 0;
+  unsigned flags = 0;
+  BAIL_ON(examine_codes(cn_d.p, ncode, ndofn, code.p, err.p, &nfree, &flags, s));
+  const bool monotone = !(flags & 32u);
+  int64_t n = nfree;
+  if (!monotone)  // number of equations = largest code number
+    for (int64_t q = 0; q < ncode; q++) n = std::max<int64_t>(n, mesh->cn[q]);
+  if (n <= 0) return bail(fail(SGPU_BAD_INPUT, "no free equations"));
+  if (flags & 1u) return bail(fail(SGPU_BAD_INPUT, "element node out of range"));
+  if (n >= (1LL << 31) - 1) return bail(fail(SGPU_BAD_INPUT, "n out of range for int32 device indices"));
+  m->n = n;
+  cudaMemsetAsync(err.p, 0, sizeof(unsigned), s);
 
-  // pattern: from the node adjacency when the code numbers grow with (node,
-  // component), else (or for a node of very high valence) lower-triangle
-  // element pairs -> sort -> unique -> SCR
-  bool monotone = true;
-  {
-    int64_t last = 0;
-    for (int64_t q = 0; q < nn * ndofn && monotone; q++) {
-      const int64_t c = mesh->cn[q];
-      if (c > 0) {
-        monotone = c == last + 1;  // gencodnum's consecutive numbering
-        last = c;
-      }
-    }
-  }
+  // pattern: from the node adjacency when the code numbers are gencodnum's,
+  // else (or for a node of very high valence) lower-triangle element pairs ->
+  // sort -> unique -> SCR
   int adj_st = 1;
   int inc_st = 1;
   if (monotone) {
@@ -2392,7 +2471,8 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
     ad.node_rows = inc_st == SGPU_OK;
   }
   if (inc_st == SGPU_OK && !std::getenv("SGPU_PATTERN_SORT")) {
-    adj_st = pattern_adjacency(m, ad.elems.p, cn_d.p, nn, nne, ndofn, n, ad.iptr.p, ad.inc.p, err.p, s);
+    adj_st = pattern_adjacency(m, ad.elems.p, code.p, nn, ne, nne, ndofn, n, ad.iptr.p, ad.inc.p, err.p,
+                               !(flags & 64u), s);
     if (adj_st != SGPU_OK && adj_st != 1) BAIL_ON(adj_st);
   }
   if (adj_st != SGPU_OK) {
@@ -2434,8 +2514,8 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
     unsigned e = 0;
     BAIL_ON(read_err(err.p, s, &e));
     if (e) return bail(fail(SGPU_BAD_INPUT, "code numbers: element node out of range or unused equation"));
+    BAIL_ON(matrix_build_from_device_src(m));
   }
-  BAIL_ON(matrix_build_from_device_src(m));
   cudaEventRecord(t1, s);
   cudaEventSynchronize(t1);
   float pattern_ms = 0.f;
@@ -2547,10 +2627,6 @@ SGPU_API int sgpu_assemble_copy(sgpu_matrix src, int32_t kind, const double *ema
         cudaMemcpyAsync((dst).p, (from).p, (from).n * sizeof(*(from).p), cudaMemcpyDeviceToDevice, s) != cudaSuccess) \
       st = fail(SGPU_CUDA_ERROR, "device copy of the pattern failed");                        \
   }
-  DUP(m->src_adr, src->src_adr);
-  DUP(m->src_ci, src->src_ci);
-  DUP(m->map_lo, src->map_lo);
-  DUP(m->map_up, src->map_up);
   DUP(c.rowptr, src->csr.rowptr);
   DUP(c.col, src->csr.col);
   DUP(ad.coords, sa.coords);
@@ -2568,6 +2644,7 @@ SGPU_API int sgpu_assemble_copy(sgpu_matrix src, int32_t kind, const double *ema
   if (c.val.alloc(c.nnz + 2) != SGPU_OK || c.diag.alloc(c.n) != SGPU_OK) return bail(SGPU_CUDA_ERROR);
   m->bsr.valid = false;
   m->bsr.nb = -1;  // examined on first use
+  m->bsr.known = src->bsr.known;
   if (emat && cudaMemcpyAsync(ad.emat.p, emat, ad.ne * (ad.general ? 36 : 2) * sizeof(double),
                               cudaMemcpyHostToDevice, s) != cudaSuccess)
     return bail(fail(SGPU_CUDA_ERROR, "copy of emat failed"));

@@ -101,7 +101,7 @@ struct Bsr3 {
   DevBuf<int> browptr, bcol;
   DevBuf<double> bval;   // nblk * 9, component-major per block row: bval[9*s + comp*nbr + j]
   DevBuf<float> bval32s; // scaled FP32 copy
-  DevBuf<int64_t> csr2bsr;  // CSR entry -> position in bval (for value updates)
+  bool known = false;  // node-blocked by construction: no check of the rows needed
   bool valid = false;
   bool have32 = false;
   int longest = 0;  // blocks of the longest block row; 0 not yet known
@@ -181,8 +181,8 @@ struct sgpu_matrix_s {
   int64_t n = 0;
   int32_t src_sym = 0;     // storage the handle was created from
   int64_t src_negm = 0;
-  sgpu::DevBuf<int64_t> src_adr, src_ci;  // source pattern (device, int64 as given)
-  sgpu::DevBuf<int> map_lo, map_up;       // source entry -> CSR positions
+  sgpu::DevBuf<int64_t> src_adr, src_ci;  // source pattern (device, int64 as given) while the CSR is built from it
+  sgpu::DevBuf<int> map_lo, map_up;       // source entry -> CSR positions (ensure_maps)
   sgpu::Csr csr;
   sgpu::Bsr3 bsr;
   sgpu::Sell sell;
@@ -204,6 +204,8 @@ struct sgpu_matrix_s {
 namespace sgpu {
 // sgpu_matrix.cu
 int matrix_build_from_device_src(sgpu_matrix m);     // src_* + a (device) -> csr
+int matrix_alloc_csr(sgpu_matrix m, int64_t n, int64_t nnz);  // arrays of the full CSR, derived forms reset
+int ensure_maps(sgpu_matrix m);                      // map_lo / map_up from the CSR
 int matrix_set_values_device(sgpu_matrix m, const double *a_d);
 int ensure_fp32(sgpu_matrix m);
 int finish_values(sgpu_matrix m);  // diag, derived formats after val changed

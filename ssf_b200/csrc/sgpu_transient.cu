@@ -210,24 +210,15 @@ SGPU_API int sgpu_matrix_combine(sgpu_matrix K, sgpu_matrix C, double a, double 
   // the two sources must be complete before their arrays are read here
   if (cudaStreamSynchronize(K->stream) != cudaSuccess || cudaStreamSynchronize(C->stream) != cudaSuccess)
     return bail(fail(SGPU_CUDA_ERROR, "synchronising the source matrices failed"));
-  const int64_t n = K->n, nnz = K->csr.nnz, negm = K->src_negm;
-  int st;
-  if ((st = m->src_adr.alloc(n + 1)) || (st = m->src_ci.alloc(negm)) || (st = m->map_lo.alloc(negm)) ||
-      (st = m->map_up.alloc(negm)) || (st = m->csr.rowptr.alloc(n + 1)) || (st = m->csr.col.alloc(nnz + 4)) ||
-      (st = m->csr.val.alloc(nnz + 2)) || (st = m->csr.diag.alloc(n)))
-    return bail(st);
-  m->csr.n = (int)n;
-  m->csr.nnz = nnz;
-  cudaMemcpyAsync(m->src_adr.p, K->src_adr.p, (n + 1) * sizeof(int64_t), cudaMemcpyDeviceToDevice, s);
-  cudaMemcpyAsync(m->src_ci.p, K->src_ci.p, negm * sizeof(int64_t), cudaMemcpyDeviceToDevice, s);
-  cudaMemcpyAsync(m->map_lo.p, K->map_lo.p, negm * sizeof(int), cudaMemcpyDeviceToDevice, s);
-  cudaMemcpyAsync(m->map_up.p, K->map_up.p, negm * sizeof(int), cudaMemcpyDeviceToDevice, s);
+  const int64_t n = K->n, nnz = K->csr.nnz;
+  int st = matrix_alloc_csr(m, n, nnz);
+  if (st != SGPU_OK) return bail(st);
+  m->bsr.known = K->bsr.known;
   cudaMemcpyAsync(m->csr.rowptr.p, K->csr.rowptr.p, (n + 1) * sizeof(int), cudaMemcpyDeviceToDevice, s);
   cudaMemcpyAsync(m->csr.col.p, K->csr.col.p, nnz * sizeof(int), cudaMemcpyDeviceToDevice, s);
   k_combine<<<blocks_for(nnz), TPB, 0, s>>>(nnz, K->csr.val.p, C->csr.val.p, a, b, m->csr.val.p);
   count_launches(1);
   if (cudaGetLastError() != cudaSuccess) return bail(fail(SGPU_CUDA_ERROR, "combine kernel failed"));
-  m->bsr.nb = -1;
   st = finish_values(m);
   if (st != SGPU_OK) return bail(st);
   if (cudaStreamSynchronize(s) != cudaSuccess) return bail(fail(SGPU_CUDA_ERROR, "combine failed"));
