@@ -1,6 +1,8 @@
 // Many independent systems of uneven size: batched Jacobi-PCG over a
-// block-diagonal matrix, as one persistent launch (the default) or as a
-// graph of segmented launches per iteration.
+// block-diagonal matrix, as one launch of clusters (the default), as one
+// persistent launch of CTAs (systems too large for a cluster's shared memory,
+// or coupled by the matrix), or as a graph of segmented launches per
+// iteration.
 //
 // The uneven batch (hundreds of plane-stress plates of different sizes, each
 // its own symcomprow::cg_prec in the reference, GEFEL/scr.cpp:1093) is held
@@ -22,11 +24,13 @@
 #include <vector>
 
 #include "sgpu_internal.cuh"
+#include "sgpu_persist.cuh"
 
 using namespace sgpu;
 
 namespace sgpu {
 int pcg_prepare(sgpu_matrix m, bool mixed);
+int longest_row(sgpu_matrix m, int *longest);
 }
 
 namespace {
@@ -395,6 +399,469 @@ __global__ void __launch_bounds__(PTPB, 2) k_bpersist(int nsys, const int *__res
   }
 }
 
+// ---------------------------------------------------------------------------
+// the cluster form: a system's iteration on the eight SMs of a cluster
+// ---------------------------------------------------------------------------
+// One CTA per system leaves the largest systems to run alone at the end, one
+// SM's bandwidth each, and gathers d through L1.  Here a cluster of eight CTAs
+// takes a system (small systems: one CTA each, eight to a cluster), largest
+// first, as the block scheduler places the clusters.  A CTA owns a contiguous
+// range of the rows: r, p and d stay in its shared memory, and a gather reads
+// its own d there and a neighbour's through distributed shared memory.  The
+// matrix streams through per-warp stages by bulk copies, as in k_pcg_tiles;
+// tiles that fit beside the two streaming stages of a warp are copied once
+// and stay.  The sums are exchanged through distributed shared memory and the
+// hardware's cluster barrier (0.75 us with the CTA's own reduction, against 2.3
+// for a barrier of the whole grid).  Every sum is formed in a fixed order, so
+// a solve repeats bit for bit.
+//
+// Measured on B200: 256 plates of 16 to 128 quadrilaterals a side (2.69M
+// equations, 393 iterations on average) 465 -> 68 ms; of the largest system's
+// iteration (29,440 equations) the product takes about two thirds.  16 warps:
+// 24 leave a warp one stage of the largest systems' matrix.
+constexpr int kClu = 8;
+constexpr int kCluTPB = 512;
+constexpr int kCluWarps = kCluTPB / 32;
+constexpr int kCluSmem = 222 * 1024;
+constexpr int kCluMaxStages = 24;  // of one warp
+constexpr int kCluMine = 8;        // rows of a thread
+// rows up to which a CTA runs a system alone: an iteration of 2048 plate rows
+// costs one SM about 9 us, eight of them 2.3 us each
+constexpr int kCluAlone = 2048;
+
+using CluTile = TileKind<1, 2>;
+
+struct CluArgs {
+  const int *items;         // system of each CTA (-1: none)
+  const long long *sysptr;
+  const int *rowptr, *col;  // col: k_local_cols
+  const double *val, *diag, *f;
+  double *x;
+  SysState *st;
+  int ent;                  // entries a stage holds
+  long long ni;
+  double res, zero;
+};
+
+struct CluShared {
+  double part[2][kCluWarps];
+  double slot[2][3][kClu];  // parity, {sum, sum, gave up}, CTA
+  unsigned long long full[kCluWarps][kCluMaxStages];
+  int bad;
+};
+
+__device__ __forceinline__ unsigned clu_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void clu_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned clu_map(const void *p, unsigned rank) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+// v = the double at a where p is set (volatile: stays between the barriers)
+__device__ __forceinline__ void clu_load_if(double &v, unsigned a, bool p) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.shared::cluster.f64 %0, [%1];\n\t}"
+               : "+d"(v)
+               : "r"(a), "r"((unsigned)p));
+}
+// a column entry of k_local_cols below 0: the neighbour's d it names
+__device__ __forceinline__ unsigned far_address(const double *ds, int at) {
+  return clu_map(ds, ((unsigned)at >> 24) & 7u) + ((unsigned)at & 0xffffffu);
+}
+__device__ __forceinline__ void clu_store(unsigned a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+// sums over the group's CTAs, and a barrier of the group; false: a CTA gave up
+template <int NV>
+__device__ __forceinline__ bool clu_sum(double (&v)[NV], int C, unsigned rank, unsigned &e, CluShared &sh) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < NV; q++) {
+    v[q] = warp_sum(v[q]);
+    if (lane == 0) sh.part[q][w] = v[q];
+  }
+  __syncthreads();
+  e ^= 1u;
+  if (w == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+      const double t = warp_sum(lane < kCluWarps ? sh.part[q][lane] : 0.0);
+      if (C == 1) sh.slot[e][q][0] = t;
+      else if (lane < C) clu_store(clu_map(&sh.slot[e][q][rank], lane), t);
+    }
+    if (C == 1) sh.slot[e][2][0] = sh.bad ? 1.0 : 0.0;
+    else if (lane < C) clu_store(clu_map(&sh.slot[e][2][rank], lane), sh.bad ? 1.0 : 0.0);
+  }
+  if (C > 1) clu_barrier();
+  else __syncthreads();
+  if (C == 1) {
+#pragma unroll
+    for (int q = 0; q < NV; q++) v[q] = sh.slot[e][q][0];
+    return sh.slot[e][2][0] == 0.0;
+  }
+  double gave_up = 0.0;
+#pragma unroll
+  for (int q = 0; q < NV; q++) {
+    double t[kClu];
+#pragma unroll
+    for (int c = 0; c < kClu; c++) t[c] = sh.slot[e][q][c];
+    v[q] = ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+  }
+#pragma unroll
+  for (int c = 0; c < kClu; c++) gave_up = fmax(gave_up, sh.slot[e][2][c]);
+  return gave_up == 0.0;
+}
+
+__global__ void __cluster_dims__(kClu, 1, 1) __launch_bounds__(kCluTPB, 1) k_bcluster(const CluArgs a) {
+  extern __shared__ __align__(128) unsigned char dyn[];
+  __shared__ CluShared sh;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // a cluster holds one system (its eight entries equal) or up to eight
+  const int *it = a.items + (blockIdx.x / kClu) * kClu;
+  const unsigned crank = clu_rank();
+  const bool whole = it[0] == it[1];
+  const int k = it[crank];
+  if (k < 0) return;  // only beside systems of one CTA each
+  const int C = whole ? kClu : 1;
+  const unsigned rank = whole ? crank : 0u;
+  const int r0 = (int)a.sysptr[k], n = (int)(a.sysptr[k + 1] - a.sysptr[k]);
+  const int per = (n + C - 1) / C;
+  const int g0 = r0 + min((int)rank * per, n), nu = min(per, n - min((int)rank * per, n));
+  // shared memory: r, p, d of the CTA's rows, their pointers, the stages
+  double *rs = reinterpret_cast<double *>(dyn), *ps = rs + per, *ds = ps + per;
+  const unsigned char *dsb = reinterpret_cast<const unsigned char *>(ds);
+  int *sp = reinterpret_cast<int *>(ds + per);
+  const size_t used = ((size_t)28 * per + 4 + 127) & ~(size_t)127;
+  const int vb = CluTile::val_bytes(a.ent), sb = CluTile::stage_bytes(a.ent);
+  const int D = min((int)((kCluSmem - used) / ((size_t)kCluWarps * sb)), kCluMaxStages);
+  unsigned char *stages = dyn + used + (size_t)w * D * sb;
+  unsigned long long *full = sh.full[w];
+  const int ntiles = (nu + CluTile::kUnits - 1) / CluTile::kUnits;
+  const int mine = ntiles > w ? (ntiles - w + kCluWarps - 1) / kCluWarps : 0;
+  const int fixed = mine <= D ? mine : max(0, D - 2), S = D - fixed;  // tiles that stay; streaming stages
+  for (int q = threadIdx.x; q <= nu; q += kCluTPB) sp[q] = a.rowptr[g0 + q];
+  if (lane == 0)
+    for (int q = 0; q < D; q++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ring_u32(full + q)) : "memory");
+  if (threadIdx.x == 0) sh.bad = 0;
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  if (C > 1) clu_barrier();  // the neighbours' shared memory is there from here on
+  else __syncthreads();
+  auto issue = [&](int j, int q) {
+    const int t = w + kCluWarps * j;
+    const int e0 = sp[t * CluTile::kUnits], e1 = sp[min((t + 1) * CluTile::kUnits, nu)];
+    const long long v0 = (long long)e0 & ~1ll, v1 = ((long long)e1 + 1) & ~1ll;
+    const int c0 = e0 & ~3, c1 = (e1 + 3) & ~3;
+    const unsigned nv = (unsigned)(8 * (v1 - v0)), nc = (unsigned)(4 * (c1 - c0));
+    unsigned char *dst = stages + (size_t)q * sb;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(ring_u32(full + q)), "r"(nv + nc)
+                 : "memory");
+    if (nv)
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                       ring_u32(dst)),
+                   "l"(a.val + v0), "r"(nv), "r"(ring_u32(full + q))
+                   : "memory");
+    if (nc)
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                       ring_u32(dst + vb)),
+                   "l"(a.col + c0), "r"(nc), "r"(ring_u32(full + q))
+                   : "memory");
+  };
+  int next = fixed;  // the next streamed tile to copy
+  if (lane == 0) {
+    for (int q = 0; q < fixed; q++) issue(q, q);
+    if (fixed < mine)
+      for (int z = 0; z < S; z++) {
+        issue(next, fixed + z);
+        if (++next == mine) next = fixed;
+      }
+  }
+  int q = 0;         // streaming stage of the next tile to read
+  unsigned ph = 0;   // its phase
+
+  // start from x = 0: r = f, h = r/diag, d = h; f.f and r.h
+  double v2[2] = {0.0, 0.0};
+  for (int i = threadIdx.x; i < nu; i += kCluTPB) {
+    const double fi = a.f[g0 + i], hi = fi / a.diag[g0 + i];
+    a.x[g0 + i] = 0.0;
+    rs[i] = fi;
+    ds[i] = hi;
+    v2[0] += fi * fi;
+    v2[1] += fi * hi;
+  }
+  unsigned e = 0;
+  SysState s = {};
+  bool ok = clu_sum<2>(v2, C, rank, e, sh);
+  s.nory = v2[0];
+  s.nom = v2[1];
+  s.ani = -1;
+  if (v2[0] < a.zero) {  // scr.cpp:1117-1120: reported, the iteration goes on
+    s.status = SGPU_ZERO_RHS;
+    s.ares = v2[0];
+    s.ani = 0;
+    s.ani_set = 1;
+  }
+  if (a.ni <= 0) s.done = 1;
+  bool first = true;
+  while (ok && !s.done) {
+    // p = A d over the CTA's rows, d.p
+    double v1[1] = {0.0};
+    for (int j = 0; j < mine; j++) {
+      const int st = j < fixed ? j : fixed + q;
+      if ((j >= fixed || first) && !ring_wait(full + st, j < fixed ? 0u : ph)) {
+        sh.bad = 1;
+        break;
+      }
+      const unsigned char *stage = stages + (size_t)st * sb;
+      const int t0 = (w + kCluWarps * j) * CluTile::kUnits, e0 = sp[t0];
+      const double *vals = reinterpret_cast<const double *>(stage) + (e0 & 1);
+      const int *cols = reinterpret_cast<const int *>(stage + vb) + (e0 & 3);
+      const int sub = lane & 1, u = t0 + (lane >> 1);
+      double y = 0.0, y2 = 0.0;
+      if (u < nu) {
+        const int b = sp[u] - e0, len = sp[u + 1] - e0 - b;
+        // 9 entries of a lane at a time (a plate's row has 18); the CTA's own
+        // d first, then -- few rows, at the range's ends -- the neighbours'
+        constexpr int U = 9;
+        const int *cl = cols + b + sub;
+        const double *vl = vals + b + sub;
+        int left = (len - sub + 1) >> 1;  // entries of the lane
+        for (; left >= U; left -= U, cl += 2 * U, vl += 2 * U) {
+          int at[U], far = 0;
+          double xx[U];
+#pragma unroll
+          for (int z = 0; z < U; z++) {
+            at[z] = cl[2 * z];
+            far |= at[z];
+          }
+#pragma unroll
+          for (int z = 0; z < U; z++) xx[z] = *reinterpret_cast<const double *>(dsb + max(at[z], 0));
+          if (far < 0) {
+#pragma unroll
+            for (int z = 0; z < U; z++) clu_load_if(xx[z], far_address(ds, at[z]), at[z] < 0);
+          }
+#pragma unroll
+          for (int z = 0; z < U; z++) {
+            if (z & 1) y2 = fma(vl[2 * z], xx[z], y2);
+            else y = fma(vl[2 * z], xx[z], y);
+          }
+        }
+        for (; left > 0; left--, cl += 2, vl += 2) {
+          const int at = cl[0];
+          double xx = *reinterpret_cast<const double *>(dsb + max(at, 0));
+          if (at < 0) clu_load_if(xx, far_address(ds, at), true);
+          y = fma(vl[0], xx, y);
+        }
+        y += y2;
+      }
+      __syncwarp();
+      y += __shfl_xor_sync(0xffffffffu, y, 1);
+      if (sub == 0 && u < nu) {
+        ps[u] = y;
+        v1[0] += ds[u] * y;
+      }
+      __syncwarp();  // the stage is read: the warp's next copy may overwrite it
+      if (j >= fixed) {
+        if (lane == 0) {
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          issue(next, st);
+          if (++next == mine) next = fixed;
+        }
+        if (++q == S) {
+          q = 0;
+          ph ^= 1;
+        }
+      }
+    }
+    first = false;
+    // what the update reads from L2, on its way during the sum (a CTA has at
+    // most kCluMine rows a thread: cluster_fits)
+    double xg[kCluMine], dg[kCluMine];
+#pragma unroll
+    for (int z = 0; z < kCluMine; z++) {
+      const int i = (int)threadIdx.x + z * kCluTPB;
+      if (i < nu) {
+        xg[z] = a.x[g0 + i];
+        dg[z] = __ldg(a.diag + g0 + i);
+      }
+    }
+    ok = clu_sum<1>(v1, C, rank, e, sh);
+    if (!ok) break;
+    s.denom = v1[0];
+    if (fabs(v1[0]) < a.zero) {  // scr.cpp:1146-1151
+      s.ani = s.it;
+      s.ares = s.nom;
+      s.ani_set = 1;
+      if (s.status == 0) s.status = SGPU_BREAKDOWN;
+      s.done = 1;
+      break;
+    }
+    const double alpha = s.nom / v1[0];
+    // x += alpha d; r -= alpha p; h = r/diag (kept where p was); r.r and r.h
+    v2[0] = v2[1] = 0.0;
+#pragma unroll
+    for (int z = 0; z < kCluMine; z++) {
+      const int i = (int)threadIdx.x + z * kCluTPB;
+      if (i < nu) {
+        a.x[g0 + i] = xg[z] + alpha * ds[i];
+        const double ri = rs[i] - alpha * ps[i], hi = ri / dg[z];
+        rs[i] = ri;
+        ps[i] = hi;
+        v2[0] += ri * ri;
+        v2[1] += ri * hi;
+      }
+    }
+    ok = clu_sum<2>(v2, C, rank, e, sh);
+    if (!ok) break;
+    s.alpha = alpha;
+    s.rr = v2[0];
+    s.beta = v2[1] / s.nom;
+    s.nom = v2[1];
+    const long long n_it = s.it;
+    s.it = n_it + 1;
+    if (fabs(v2[0] / s.nory) < a.res) {  // scr.cpp:1188
+      s.ani = n_it;
+      s.ares = v2[1] / s.nory;
+      s.ani_set = 1;
+      s.done = 1;
+      break;
+    }
+    if (n_it + 1 >= a.ni) {
+      s.done = 1;
+      if (s.status == 0) s.status = SGPU_NOT_CONVERGED;
+      break;
+    }
+    for (int i = threadIdx.x; i < nu; i += kCluTPB) ds[i] = s.beta * ds[i] + ps[i];
+    if (C > 1) clu_barrier();
+    else __syncthreads();
+  }
+  // the copies that nobody reads (and those of a solve without iterations)
+  if (lane == 0) {
+    for (int z = 0; z < fixed; z++) ring_wait(full + z, 0u);
+    if (fixed < mine)
+      for (int z = 0; z < S; z++) {
+        ring_wait(full + fixed + q, ph);
+        if (++q == S) {
+          q = 0;
+          ph ^= 1;
+        }
+      }
+  }
+  if (rank == 0 && threadIdx.x == 0) {
+    if (!ok) {
+      s.status = SGPU_CUDA_ERROR;
+      s.done = 1;
+    }
+    a.st[k] = s;
+  }
+  if (C > 1) clu_barrier();  // no CTA leaves while another may read its d
+}
+
+// Where a gather finds its d: for an entry of the CTA's own rows the byte
+// offset in its shared d, for a neighbour's the sign bit, the neighbour's rank
+// (3 bits at 24) and the offset there (at most 32 KB).  The product then needs
+// four instructions per entry instead of fifteen (the compares and clamps of
+// the column against the CTA's range were what bound it: 1.28e9 row products
+// of 18 entries took 77 ms with them).  flag = 1 where a row of a system has a
+// column outside the system: then its entry is not used.
+__global__ void k_local_cols(int nsys, const long long *__restrict__ sysptr, const int *__restrict__ rowptr,
+                             const int *__restrict__ col, int *__restrict__ lcol, int *flag) {
+  const int lane = threadIdx.x & 31;
+  for (int k = blockIdx.y; k < nsys; k += gridDim.y) {
+    const int r0 = (int)sysptr[k], n = (int)(sysptr[k + 1] - r0);
+    const int C = n > kCluAlone ? kClu : 1, per = (n + C - 1) / C;
+    for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n; i += (gridDim.x * blockDim.x) >> 5) {
+      const int own = i / per;
+      for (int q = rowptr[r0 + i] + lane; q < rowptr[r0 + i + 1]; q += 32) {
+        const int rel = col[q] - r0;
+        int v = 0;
+        if (rel < 0 || rel >= n) {
+          *flag = 1;
+        } else {
+          const int o = rel / per, off = 8 * (rel - o * per);
+          v = o == own ? off : (int)(0x80000000u | ((unsigned)o << 24) | (unsigned)off);
+        }
+        lcol[q] = v;
+      }
+    }
+  }
+}
+
+// Whether the cluster form takes the batch: the longest row's stage and the
+// largest system's vectors fit a CTA's shared memory with two stages a warp.
+bool cluster_fits(int longest, int64_t most_rows) {
+  if (longest <= 0 || longest > 2048) return false;
+  const int64_t ent = ((int64_t)longest * CluTile::kUnits + 3) & ~3ll;
+  const int64_t per = std::max<int64_t>((most_rows + kClu - 1) / kClu, std::min<int64_t>(most_rows, kCluAlone));
+  return per <= kCluMine * kCluTPB &&
+         28 * per + 256 + 2 * kCluWarps * (int64_t)CluTile::stage_bytes((int)ent) <= kCluSmem;
+}
+
+constexpr int kCoupled = 1000;  // run_cluster: the systems are not the matrix's diagonal blocks
+
+int run_cluster(sgpu_matrix m, const std::vector<int64_t> &rows, int longest, double *x, const double *f, int64_t ni,
+                double res, double zero, std::vector<SysState> &hs, int64_t *iters, float *ms) {
+  cudaStream_t s = m->stream;
+  const Csr &c = m->csr;
+  const int nsys = (int)rows.size();
+  std::vector<long long> ptr(nsys + 1, 0);
+  for (int k = 0; k < nsys; k++) ptr[k + 1] = ptr[k] + rows[k];
+  std::vector<int> order(nsys), items;
+  for (int k = 0; k < nsys; k++) order[k] = k;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return rows[a] > rows[b]; });
+  int at = 0;
+  for (; at < nsys && rows[order[at]] > kCluAlone; at++) items.insert(items.end(), kClu, order[at]);
+  for (; at < nsys; at += kClu)
+    for (int z = 0; z < kClu; z++) items.push_back(at + z < nsys ? order[at + z] : -1);
+  DevBuf<long long> ptr_d;
+  DevBuf<int> items_d;
+  DevBuf<SysState> st;
+  SGPU_TRY(ptr_d.alloc(nsys + 1));
+  SGPU_TRY(items_d.alloc(items.size()));
+  SGPU_TRY(st.alloc(nsys));
+  SGPU_CUDA(cudaMemcpyAsync(ptr_d.p, ptr.data(), (nsys + 1) * sizeof(long long), cudaMemcpyHostToDevice, s));
+  SGPU_CUDA(cudaMemcpyAsync(items_d.p, items.data(), items.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+  // the neighbours whose d a gather may read are the system's own: where the
+  // matrix couples systems, the caller's other form runs
+  DevBuf<int> lcol;
+  SGPU_TRY(lcol.alloc((size_t)c.nnz + 4));
+  int *flag_d = reinterpret_cast<int *>(m->w.counters.p + 8), coupled = 0;
+  SGPU_CUDA(cudaMemsetAsync(flag_d, 0, sizeof(int), s));
+  const dim3 lg((unsigned)std::max<int64_t>(1, std::min<int64_t>((rows[order[0]] + 63) / 64, 16)),
+                (unsigned)std::min(nsys, 2048));
+  k_local_cols<<<lg, TPB, 0, s>>>(nsys, ptr_d.p, c.rowptr.p, c.col.p, lcol.p, flag_d);
+  count_launches(1);
+  SGPU_CUDA(cudaMemcpyAsync(&coupled, flag_d, sizeof(int), cudaMemcpyDeviceToHost, s));
+  SGPU_CUDA(cudaStreamSynchronize(s));
+  if (coupled) return kCoupled;
+  const int ent = (longest * CluTile::kUnits + 3) & ~3;
+  const CluArgs a = {items_d.p, ptr_d.p, c.rowptr.p, lcol.p, c.val.p, c.diag.p, f, x, st.p, ent, (long long)ni, res,
+                     zero};
+  SGPU_CUDA(cudaFuncSetAttribute(k_bcluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kCluSmem));
+  SGPU_CUDA(cudaEventRecord(m->ev0, s));
+  k_bcluster<<<(unsigned)items.size(), kCluTPB, kCluSmem, s>>>(a);
+  count_launches(1);
+  SGPU_CUDA(cudaGetLastError());
+  SGPU_CUDA(cudaEventRecord(m->ev1, s));
+  hs.resize(nsys);
+  SGPU_CUDA(cudaMemcpyAsync(hs.data(), st.p, nsys * sizeof(SysState), cudaMemcpyDeviceToHost, s));
+  SGPU_CUDA(cudaStreamSynchronize(s));
+  if (ms) SGPU_CUDA(cudaEventElapsedTime(ms, m->ev0, m->ev1));
+  int64_t mx = 0;
+  for (const SysState &q : hs) {
+    if (q.status == SGPU_CUDA_ERROR) return fail(SGPU_CUDA_ERROR, "batched PCG: a wait inside a cluster ran out");
+    mx = std::max<int64_t>(mx, q.it);
+  }
+  if (iters) *iters = mx;
+  return SGPU_OK;
+}
+
 // the persistent solve of every system; hs gets the per-system results
 int run_persistent(sgpu_matrix m, const std::vector<int64_t> &rows, int L, double *x, const double *f, double *r,
                    double *h, double *d, double *p, int64_t ni, double res, double zero, std::vector<SysState> &hs,
@@ -608,8 +1075,14 @@ extern "C" SGPU_API int sgpu_matrix_pcg_batch(sgpu_matrix m, int32_t nsys, const
     const double mean = (double)m->csr.nnz / (double)m->n;
     best.L = mean > 40 ? 16 : (mean > 12 ? 8 : 4);
     best.S = 0;
-    SGPU_TRY(run_persistent(m, rows, best.L, w.x.p, w.f.p, w.r.p, w.h.p, w.d.p, w.p.p, ni, res, zero, hs, &its,
-                            &ms));
+    int longest = 0;
+    SGPU_TRY(longest_row(m, &longest));
+    const int64_t most = *std::max_element(rows.begin(), rows.end());
+    int rc = kCoupled;
+    if (cluster_fits(longest, most)) rc = run_cluster(m, rows, longest, w.x.p, w.f.p, ni, res, zero, hs, &its, &ms);
+    if (rc == kCoupled)
+      rc = run_persistent(m, rows, best.L, w.x.p, w.f.p, w.r.p, w.h.p, w.d.p, w.p.p, ni, res, zero, hs, &its, &ms);
+    if (rc != SGPU_OK) return rc;
   } else {
     Batch b;
     SGPU_TRY(build_segments(rows, best.S, b, s));

@@ -1047,7 +1047,7 @@ constexpr long long kPersistChunk = 4096;
 // How an FP64 solve iterates.
 enum class Form { kResident, kTiles, kGraph };
 
-int longest_row(sgpu_matrix m, int units, const int *ptr, int *cached) {
+int longest_unit(sgpu_matrix m, int units, const int *ptr, int *cached) {
   if (*cached > 0) return SGPU_OK;
   int *out = reinterpret_cast<int *>(m->w.counters.p + 8);
   SGPU_CUDA(cudaMemsetAsync(out, 0, sizeof(int), m->stream));
@@ -1077,7 +1077,7 @@ int choose_form(sgpu_matrix m, int sms, Form *form, TileMat *tm, int *longest, i
   Bsr3 &b = m->bsr;
   *tm = b.valid ? TileMat{b.nb, b.browptr.p, b.bcol.p, b.bval.p, 0, 0, 0}
                 : TileMat{c.n, c.rowptr.p, c.col.p, c.val.p, 0, 0, 0};
-  SGPU_TRY(longest_row(m, tm->units, tm->ptr, b.valid ? &b.longest : &m->csr.longest));
+  SGPU_TRY(longest_unit(m, tm->units, tm->ptr, b.valid ? &b.longest : &m->csr.longest));
   *longest = b.valid ? b.longest : c.longest;
   *lanes = b.valid ? tile_lanes<3>(*tm, *longest, sms) : tile_lanes<1>(*tm, *longest, sms);
   if (*lanes > 0) {
@@ -1353,6 +1353,14 @@ int pcg_run(sgpu_matrix m, int64_t ni, double res, double zero, int64_t iv, int 
     info->fallback = fallback;
   }
   return hs.status;
+}
+
+// entries of the longest CSR row
+int longest_row(sgpu_matrix m, int *longest) {
+  SGPU_TRY(ensure_work(m, false));
+  SGPU_TRY(longest_unit(m, m->csr.n, m->csr.rowptr.p, &m->csr.longest));
+  *longest = m->csr.longest;
+  return SGPU_OK;
 }
 
 int pcg_prepare(sgpu_matrix m, bool mixed) { return ensure_work(m, mixed); }
