@@ -85,6 +85,15 @@ struct AmgLevel {
   int lz_slot = -1;
 };
 
+// The coarse levels of a cycle as a list of steps on the device
+// (k_coarse_program), recorded at the start of a solve.
+struct CoarseProgram {
+  bool current = false;  // recorded for the solve under way (nsteps 0: none)
+  int nsteps = 0, block = 0, grid = 0;
+  void *result = nullptr;  // level 1's iterate after it
+  DevBuf<unsigned char> steps;
+};
+
 struct Amg {
   int k0 = 0;             // near-null-space vectors given (0: translations)
   PBuf<double> B0;      // n x k0 as given
@@ -142,6 +151,8 @@ struct Amg {
   int64_t h16_nblk = 0;     // stored blocks, padding included
   DevBuf<int> h16ptr, h16col;
   DevBuf<uint16_t> h16val;  // IEEE binary16 bit patterns
+  CoarseProgram prog32, prog64;
+  DevBuf<unsigned char> prog_sync;  // the programs' grid barrier
   ~Amg() {
     for (AmgLevel *l : pool) delete l;
     if (side) {

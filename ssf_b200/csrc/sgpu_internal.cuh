@@ -35,6 +35,51 @@ void count_launches(int64_t k);
 
 constexpr int kNumSMs = 148;
 
+#ifdef __CUDACC__
+// Sums y[0 .. B) over the L lanes of a group (B = 1, 3 or 6; L a power of two,
+// at least 8 for B > 1) so that each sum ends in lanes of its own: a lane
+// gives away the half of its values that the partner keeps, and only the last
+// steps move one value.  B = 6 over a warp takes 9 shuffles where six
+// butterflies take 30, B = 3 over 8 lanes 4 against 9; the pairs added are the
+// butterfly's, so the bits are too.  Returns the sum of row row_of_lane(sub).
+template <int B, int L>
+struct RowSums {
+  static constexpr int kStep = B == 1 ? L : (B == 3 ? L / 4 : L / 8);  // lanes that share a row
+  // the row whose sum lane sub gets (>= B: none), and whether it is the
+  // group's first such lane
+  static __device__ __forceinline__ int row_of_lane(int sub) { return B == 1 ? 0 : sub / kStep; }
+  static __device__ __forceinline__ bool first(int sub) { return sub % kStep == 0 && sub / kStep < B; }
+  template <typename T>
+  static __device__ __forceinline__ T sum(T (&y)[B], int sub) {
+    T v;
+    if constexpr (B == 1) {
+      v = y[0];
+    } else if constexpr (B == 3) {
+      const bool h = sub & (L / 2), g = sub & (L / 4);
+      const T a = __shfl_xor_sync(0xffffffffu, h ? y[0] : y[2], L / 2);
+      const T b = __shfl_xor_sync(0xffffffffu, h ? y[1] : T(0), L / 2);
+      const T k0 = (h ? y[2] : y[0]) + a, k1 = (h ? T(0) : y[1]) + b;
+      v = (g ? k1 : k0) + __shfl_xor_sync(0xffffffffu, g ? k0 : k1, L / 4);
+    } else {
+      static_assert(B == 6, "rows per block: 1, 3 or 6");
+      const bool h = sub & (L / 2), g = sub & (L / 4), f = sub & (L / 8);
+      T k[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const T up = q < 2 ? y[q + 4 < B ? q + 4 : 0] : T(0);  // rows 4, 5, none, none
+        k[q] = (h ? up : y[q]) + __shfl_xor_sync(0xffffffffu, h ? y[q] : up, L / 2);
+      }
+      const T m0 = (g ? k[2] : k[0]) + __shfl_xor_sync(0xffffffffu, g ? k[0] : k[2], L / 4);
+      const T m1 = (g ? k[3] : k[1]) + __shfl_xor_sync(0xffffffffu, g ? k[1] : k[3], L / 4);
+      v = (f ? m1 : m0) + __shfl_xor_sync(0xffffffffu, f ? m0 : m1, L / 8);
+    }
+#pragma unroll
+    for (int o = kStep / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  }
+};
+#endif
+
 // ---------------------------------------------------------------------------
 // device buffers
 // ---------------------------------------------------------------------------

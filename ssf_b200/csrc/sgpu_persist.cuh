@@ -674,15 +674,10 @@ __global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const T
           }
         }
         __syncwarp();
-#pragma unroll
-        for (int o = LPR / 2; o > 0; o >>= 1) {
-          y0 += __shfl_xor_sync(0xffffffffu, y0, o, LPR);
-          y1 += __shfl_xor_sync(0xffffffffu, y1, o, LPR);
-          y2 += __shfl_xor_sync(0xffffffffu, y2, o, LPR);
-        }
-        if (sub < 3 && u < nu) {
-          const double yv = sub == 0 ? y0 : (sub == 1 ? y1 : y2);
-          const int i = 3 * (u0 + u) + sub;
+        double y[3] = {y0, y1, y2};
+        const double yv = RowSums<3, LPR>::sum(y, sub);
+        if (RowSums<3, LPR>::first(sub) && u < nu) {
+          const int i = 3 * (u0 + u) + RowSums<3, LPR>::row_of_lane(sub);
           a.p[i] = yv;
           acc += a.d[i] * yv;
         }
