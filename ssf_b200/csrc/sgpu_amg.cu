@@ -1184,7 +1184,7 @@ struct BSys {
 // Sum of v over the rows [r0, r1) of one system by the whole CTA: every
 // thread's rows in order, then the warp, then the warps in order (the result
 // is in thread 0).  A warp per system instead (the earlier form) left 256
-// systems on 32 CTAs: at 2.69M rows the three sums of an iteration took 0.35
+// systems on 32 CTAs: at 2.69M rows the three sums of an iteration took 0.41
 // ms, against 0.04 with a CTA each.
 constexpr int kSegTPB = 512;
 template <int NV>
@@ -4568,101 +4568,6 @@ int write_st(sgpu_matrix m, const PcgState *h) {
   return SGPU_OK;
 }
 
-template <typename T>
-int capture_chunk(sgpu_matrix m, int iters, cudaGraphExec_t *exec, int64_t *nodes) {
-  cudaStream_t s = m->stream;
-  Work &w = m->w;
-  const int64_t before = sgpu_kernel_launches();
-  cudaGraph_t g;
-  SGPU_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-  int rc = SGPU_OK;
-  for (int it = 0; it < iters && rc == SGPU_OK; it++) {
-    rc = spmv64_flex(m, w.d.p, w.p.p, s);
-    if (rc == SGPU_OK) rc = fcg_update<T>(m, s);
-    if (rc == SGPU_OK) rc = vcycle_dir<T>(m, s);
-  }
-  cudaError_t e = cudaStreamEndCapture(s, &g);
-  if (rc != SGPU_OK) return rc;
-  if (e != cudaSuccess) return fail(SGPU_CUDA_ERROR, std::string("cudaStreamEndCapture: ") + cudaGetErrorString(e));
-  e = cudaGraphInstantiate(exec, g, 0);
-  cudaGraphDestroy(g);
-  if (e != cudaSuccess) return fail(SGPU_CUDA_ERROR, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-  *nodes = sgpu_kernel_launches() - before;
-  count_launches(-*nodes);  // captured launches run (and are counted) at each replay
-  return SGPU_OK;
-}
-
-// The loop body's last kernel: run the body again while the iteration has
-// not stopped and the launch's iteration cap is not reached.
-__global__ void k_fcg_continue(cudaGraphConditionalHandle h, PcgState *st, int64_t cap) {
-  const int64_t c = ++st->loops;
-  cudaGraphSetConditional(h, (!st->done && c < cap) ? 1u : 0u);
-}
-
-// The flexible CG's iterations as one graph: a conditional WHILE node whose
-// body is one iteration (FP64 SpMV, update, V-cycle and direction) and
-// k_fcg_continue, which ends the loop when the solver's state says done (the
-// stopping test, a breakdown or ni iterations) or after `cap` iterations of
-// one launch, whichever comes first.  The host waits once per launch.
-// Returns SGPU_OK with *exec == nullptr when the runtime offers no
-// conditional nodes (the caller then uses capture_chunk).
-template <typename T>
-int capture_loop(sgpu_matrix m, int64_t cap, cudaGraphExec_t *exec, int64_t *nodes) {
-  cudaStream_t s = m->stream;
-  Work &w = m->w;
-  *exec = nullptr;
-  cudaGraph_t g = nullptr;
-  SGPU_CUDA(cudaGraphCreate(&g, 0));
-  cudaGraphConditionalHandle h;
-  if (cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
-    cudaGetLastError();
-    cudaGraphDestroy(g);
-    return SGPU_OK;
-  }
-  cudaGraphNodeParams cp = {};
-  cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = h;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  cudaGraphNode_t node;
-  if (cudaGraphAddNode(&node, g, nullptr, 0, &cp) != cudaSuccess) {
-    cudaGetLastError();
-    cudaGraphDestroy(g);
-    return SGPU_OK;
-  }
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  const int64_t before = sgpu_kernel_launches();
-  cudaError_t e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
-  if (e != cudaSuccess) {
-    cudaGraphDestroy(g);
-    return fail(SGPU_CUDA_ERROR, std::string("cudaStreamBeginCaptureToGraph: ") + cudaGetErrorString(e));
-  }
-  int rc = spmv64_flex(m, w.d.p, w.p.p, s);
-  if (rc == SGPU_OK) rc = fcg_update<T>(m, s);
-  if (rc == SGPU_OK) rc = vcycle_dir<T>(m, s);
-  if (rc == SGPU_OK) {
-    k_fcg_continue<<<1, 1, 0, s>>>(h, pcg_state(m), cap);
-    count_launches(1);
-  }
-  cudaGraph_t captured = nullptr;
-  e = cudaStreamEndCapture(s, &captured);
-  if (rc != SGPU_OK) {
-    cudaGraphDestroy(g);
-    return rc;
-  }
-  if (e == cudaSuccess) e = cudaGraphInstantiate(exec, g, 0);
-  cudaGraphDestroy(g);
-  *nodes = sgpu_kernel_launches() - before;  // kernels of one iteration
-  count_launches(-*nodes);
-  if (e != cudaSuccess) {  // a body the runtime does not take: the caller captures chunks
-    cudaGetLastError();
-    *exec = nullptr;
-    if (getenv("SGPU_AMG_VERBOSE"))
-      fprintf(stderr, "amg: no device-side loop graph (%s); chunks of iterations\n", cudaGetErrorString(e));
-  }
-  return SGPU_OK;
-}
-
 // r = f - K x with a fresh V-cycle and p = z: (re)start of the recurrence
 template <typename T>
 int fcg_start(sgpu_matrix m, cudaStream_t s) {
@@ -4688,32 +4593,17 @@ int fcg_solve(sgpu_matrix m, int64_t ni, double res, double zero, int64_t iv, in
   program<T>(*m->amg).current = false;
   if (iv == 0) SGPU_CUDA(cudaMemsetAsync(w.x.p, 0, (size_t)n * sizeof(double), s));
   SGPU_TRY(fcg_start<T>(m, s));
-  SGPU_TRY(read_st(m, hs));
-  if (hs->done) return SGPU_OK;
-  const int chunk = 8;
-  cudaGraphExec_t exec = nullptr;
-  int64_t nodes = 0;
-  PhaseClock clk(s);
-  // the device-side loop (SGPU_FCG_LOOP=chunk: graphs of `chunk` iterations
-  // and a host test between them)
-  const char *lm = getenv("SGPU_FCG_LOOP");
-  bool loop = !(lm && !strcmp(lm, "chunk"));
-  if (loop) {
-    // at most the remaining iterations (plus one) per launch
-    SGPU_TRY(capture_loop<T>(m, std::max<int64_t>(2, ni - hs->it + 1), &exec, &nodes));
-    loop = exec != nullptr;
-  }
-  if (!loop) SGPU_TRY(capture_chunk<T>(m, chunk, &exec, &nodes));
-  clk.mark(loop ? "graph capture + instantiate (loop)" : "graph capture + instantiate");
+  Iterations iters;
   int rc = SGPU_OK;
   int restarts = 0;
   for (;;) {
-    if (loop) SGPU_CUDA(cudaMemsetAsync(&pcg_state(m)->loops, 0, sizeof(int64_t), s));
-    cudaError_t e = cudaGraphLaunch(exec, s);
-    if (e != cudaSuccess) { rc = fail(SGPU_CUDA_ERROR, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e)); break; }
-    rc = read_st(m, hs);
+    rc = iters.run(s, m->amg->side, &pcg_state(m)->done, ni + 1, [&]() -> int {
+      SGPU_TRY(spmv64_flex(m, w.d.p, w.p.p, s));
+      SGPU_TRY(fcg_update<T>(m, s));
+      return vcycle_dir<T>(m, s);
+    });
+    if (rc == SGPU_OK) rc = read_st(m, hs);
     if (rc != SGPU_OK) break;
-    count_launches(loop ? nodes * hs->loops : nodes);
     if (!hs->done) continue;
     // converged on the recurrence: with SGPU_CRIT_TRUE the true residual must
     // agree, else the recurrence restarts from it (at most four times; a
@@ -4741,7 +4631,6 @@ int fcg_solve(sgpu_matrix m, int64_t ni, double res, double zero, int64_t iv, in
     if (rc == SGPU_OK) rc = fcg_start<T>(m, s);
     if (rc != SGPU_OK) break;
   }
-  cudaGraphExecDestroy(exec);
   if (rc == SGPU_OK && hs->status == SGPU_CUDA_ERROR)
     rc = fail(SGPU_CUDA_ERROR, "aggregation cycle: a wait of the coarse levels ran out");
   return rc;
@@ -4899,14 +4788,9 @@ int batch_solve(sgpu_matrix m, int nsys, const long long *sysptr, const int *row
   k_bseg_beta<<<gs, kSegTPB, 0, s>>>(nsys, sysptr, A.batch_zr, A.batch_zq, sys);
   count_launches(1);
   // (k_b_dir ran before the first beta: p = S x0, beta = 0 at a start)
-  cudaGraph_t graph;
-  cudaGraphExec_t exec = nullptr;
-  const int64_t before = sgpu_kernel_launches();
-  SGPU_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-  int rc = SGPU_OK;
-  for (int it = 0; it < 8 && rc == SGPU_OK; it++) {
-    rc = batch_spmv64(m, w.d.p, w.p.p, ppq, s);
-    if (rc != SGPU_OK) break;
+  Iterations iters;
+  SGPU_TRY(iters.run(s, A.side, &pcg_state(m)->done, ni + 8, [&]() -> int {
+    SGPU_TRY(batch_spmv64(m, w.d.p, w.p.p, ppq, s));
     k_bseg_alpha<<<gs, kSegTPB, 0, s>>>(nsys, sysptr, ppq, sys);
     k_b_update<T><<<g, TPB, 0, s>>>(n, rowsys, sys, w.x.p, w.r.p, w.d.p, w.p.p, m->csr.dscale.p, V.b.p, V.r.p, V.d.p,
                                     V.x.p, c2, prr, pcg_state(m));
@@ -4914,34 +4798,18 @@ int batch_solve(sgpu_matrix m, int nsys, const long long *sysptr, const int *row
     k_bcount<<<1, TPB, 0, s>>>(nsys, sys, pcg_state(m));
     count_launches(4);
     // the new residual's preconditioned direction: cycle, beta, then p
-    Amg &Ar = *m->amg;
-    const int nl = (int)Ar.lv.size();
+    const int nl = (int)A.lv.size();
     std::vector<Cheb> ch(nl);
     for (int l = 0; l < nl; l++)
-      ch[l] = cheb_coeffs(sizeof(T) == 4 ? Ar.lv[l]->lmax32 : Ar.lv[l]->lmax64, Ar.ratio, Ar.deg);
+      ch[l] = cheb_coeffs(sizeof(T) == 4 ? A.lv[l]->lmax32 : A.lv[l]->lmax64, A.ratio, A.deg);
     std::vector<T *> xcur(nl + 1, nullptr);
-    rc = cycle<T>(m, 0, true, ch, xcur, s);
-    if (rc != SGPU_OK) break;
+    SGPU_TRY(cycle<T>(m, 0, true, ch, xcur, s));
     k_bseg_beta<<<gs, kSegTPB, 0, s>>>(nsys, sysptr, A.batch_zr, A.batch_zq, sys);
     k_b_dir<T><<<g, TPB, 0, s>>>(n, rowsys, sys, w.d.p, xcur[0], m->csr.dscale.p, pcg_state(m));
     count_launches(2);
-  }
-  cudaError_t e = cudaStreamEndCapture(s, &graph);
-  if (rc != SGPU_OK) return rc;
-  if (e != cudaSuccess) return fail(SGPU_CUDA_ERROR, std::string("cudaStreamEndCapture: ") + cudaGetErrorString(e));
-  e = cudaGraphInstantiate(&exec, graph, 0);
-  cudaGraphDestroy(graph);
-  if (e != cudaSuccess) return fail(SGPU_CUDA_ERROR, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-  const int64_t nodes = sgpu_kernel_launches() - before;
-  count_launches(-nodes);
-  for (int64_t it = 0;; it += 8) {
-    SGPU_TRY(read_st(m, hs));
-    if (hs->done || it > ni + 8) break;
-    e = cudaGraphLaunch(exec, s);
-    if (e != cudaSuccess) { rc = fail(SGPU_CUDA_ERROR, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e)); break; }
-    count_launches(nodes);
-  }
-  cudaGraphExecDestroy(exec);
+    return SGPU_OK;
+  }));
+  int rc = read_st(m, hs);
   if (rc == SGPU_OK && hs->status == SGPU_CUDA_ERROR)
     rc = fail(SGPU_CUDA_ERROR, "aggregation cycle: a wait of the coarse levels ran out");
   return rc;

@@ -3,6 +3,9 @@
 // (sgpu_amg_multi.cu).
 #pragma once
 
+#include <cstdlib>
+#include <cstring>
+#include <string>
 #include <vector>
 
 #include "sgpu_internal.cuh"
@@ -223,5 +226,104 @@ inline const double *level_dinv<double>(const AmgLevel &L) { return L.unit_diag 
 // Builds the hierarchy if the handle has none (set-up in FP64) and the copies
 // of the requested cycle precision; set-up device time into *setup_ms.
 int amg_ensure(sgpu_matrix m, bool fp32, float *setup_ms);
+
+// A solve's iterations: the first ones launched one kernel after the other,
+// the rest as a graph of kChunk of them, launched again while the one before
+// it still runs.  The host reads `done` of a finished launch on a second
+// stream meanwhile, so the device never waits for it; the kernels of what is
+// queued past the end return at once.  A conditional WHILE node around one
+// iteration (the form before) puts a gap between iterations, and graphs of 8
+// with the host in between (the batches' form before) one between graphs:
+// 129,480 equations in FP64 9.05 -> 8.67 ms, 1.01M mixed 24.1 -> 23.7, 64
+// load cases 41.0 -> 40.2, 256 plates 63.1 -> 61.4.
+class Iterations {
+ public:
+  Iterations() = default;
+  Iterations(const Iterations &) = delete;
+  Iterations &operator=(const Iterations &) = delete;
+  ~Iterations() {
+    for (cudaEvent_t e : mark_)
+      if (e) cudaEventSynchronize(e), cudaEventDestroy(e);  // the graph may still run
+    if (exec_) cudaGraphExecDestroy(exec_);
+    if (own_) cudaStreamDestroy(own_);
+  }
+
+  // `iteration` launches one iteration on s; done: the solver state's flag
+  // (set by the kernels, never cleared by them), at most max_iters iterations.
+  // poll: a stream that is idle now, or null.  s may still have queued kernels
+  // on return, all of which see `done`.
+  template <class Body>
+  int run(cudaStream_t s, cudaStream_t poll, const int *done, int64_t max_iters, Body iteration) {
+    const char *lm = getenv("SGPU_FCG_LOOP");
+    const bool ahead = !(lm && !strcmp(lm, "chunk"));  // chunk: the host tests before every launch
+    if (!poll) {
+      if (!own_) SGPU_CUDA(cudaStreamCreateWithFlags(&own_, cudaStreamNonBlocking));
+      poll = own_;
+    }
+    for (cudaEvent_t &e : mark_)
+      if (!e) SGPU_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    int64_t queued = 0;
+    bool stop = false;
+    SGPU_CUDA(cudaEventRecord(mark_[0], s));
+    if (!exec_) {
+      if (ahead)
+        for (; queued < 2; queued++) SGPU_TRY(iteration());
+      SGPU_TRY(read(poll, mark_[0], done, &stop));  // converged at the start: no graph
+      if (stop || queued >= max_iters) return SGPU_OK;
+      SGPU_TRY(capture(s, kChunk, iteration));
+    }
+    for (int k = 0; !stop && queued < max_iters; k ^= 1) {
+      if (!ahead) SGPU_TRY(read(poll, mark_[k ^ 1], done, &stop));
+      if (stop) break;
+      SGPU_CUDA(cudaGraphLaunch(exec_, s));
+      count_launches(nodes_);
+      SGPU_CUDA(cudaEventRecord(mark_[k], s));
+      queued += kChunk;
+      if (ahead && queued > 2 + kChunk) SGPU_TRY(read(poll, mark_[k ^ 1], done, &stop));
+    }
+    return SGPU_OK;
+  }
+
+ private:
+  // 1, 2 and 4 take the same time to a percent; a longer graph takes longer to
+  // make and leaves more behind the end
+  static constexpr int kChunk = 2;
+
+  static int read(cudaStream_t poll, cudaEvent_t mark, const int *done, bool *stop) {
+    int flag = 0;
+    SGPU_CUDA(cudaStreamWaitEvent(poll, mark, 0));
+    SGPU_CUDA(cudaMemcpyAsync(&flag, done, sizeof(int), cudaMemcpyDeviceToHost, poll));
+    SGPU_CUDA(cudaStreamSynchronize(poll));
+    *stop = flag != 0;
+    return SGPU_OK;
+  }
+
+  template <class Body>
+  int capture(cudaStream_t s, int count, Body iteration) {
+    cudaGraph_t g;
+    const int64_t before = sgpu_kernel_launches();
+    SGPU_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
+    int rc = SGPU_OK;
+    for (int it = 0; it < count && rc == SGPU_OK; it++) rc = iteration();
+    cudaError_t e = cudaStreamEndCapture(s, &g);
+    nodes_ = sgpu_kernel_launches() - before;
+    count_launches(-nodes_);  // captured launches run (and are counted) at each replay
+    if (e != cudaSuccess)
+      return rc != SGPU_OK ? rc : fail(SGPU_CUDA_ERROR, std::string("cudaStreamEndCapture: ") + cudaGetErrorString(e));
+    if (rc == SGPU_OK) e = cudaGraphInstantiate(&exec_, g, 0);
+    cudaGraphDestroy(g);
+    if (rc != SGPU_OK) return rc;
+    if (e != cudaSuccess) {
+      exec_ = nullptr;
+      return fail(SGPU_CUDA_ERROR, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
+    }
+    return SGPU_OK;
+  }
+
+  cudaGraphExec_t exec_ = nullptr;
+  int64_t nodes_ = 0;
+  cudaEvent_t mark_[2] = {nullptr, nullptr};
+  cudaStream_t own_ = nullptr;
+};
 
 }  // namespace sgpu

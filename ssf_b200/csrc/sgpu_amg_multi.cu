@@ -54,14 +54,40 @@ struct MVecs {
 // per-column grid reduction
 // ---------------------------------------------------------------------------
 
+// Column t's sum of `n` rows of RP values each, in row order; 16 loads in flight.
+template <int RP>
+__device__ __forceinline__ double sum_rows(const double *p, int n) {
+  double s = 0.0;
+  for (int b0 = 0; b0 < n; b0 += 16) {
+    double v[16];
+#pragma unroll
+    for (int b = 0; b < 16; b++) v[b] = b0 + b < n ? __ldcg(p + (size_t)(b0 + b) * RP) : 0.0;
+#pragma unroll
+    for (int b = 0; b < 16; b++) s += v[b];
+  }
+  return s;
+}
+
+constexpr int kRedGroup = 32;                                            // blocks of one group
+constexpr int kRedGroups = (8 * kNumSMs + kRedGroup - 1) / kRedGroup;    // of the largest grid
+constexpr int kTickets = 1 + kRedGroups;                                 // counters of one reduction
+constexpr int kSlots = 8;                                                // kernels with sums
+
 // Sums acc[c][q] (column lane + 32 c) over the grid.  Returns true in the
-// last block, with the sums in tot[q * RP + col].
+// last block, with the sums in tot[q * RP + col].  Blocks are summed in
+// groups of 32 by the group's last block, the groups by the last of those: a
+// chain of 32 + 37 partials.  One block adding all 1184 of each column left the
+// other SMs idle for 37 % of the last smoothing step (80,000 equations, 64
+// columns).  `ticket` has kTickets counters.
 template <int NV, int CPL>
 __device__ bool col_reduce(const double (&acc)[CPL][NV], double *partials, unsigned *ticket, double *tot) {
   constexpr int RP = 32 * CPL;
   __shared__ double sh[NV][CPL][NW][32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nblk = (int)gridDim.x, grp = blockIdx.x / kRedGroup, ngrp = (nblk + kRedGroup - 1) / kRedGroup;
+  const int size = min(kRedGroup, nblk - grp * kRedGroup);
+  double *groups = partials + (size_t)NV * nblk * RP;
 #pragma unroll
   for (int q = 0; q < NV; q++)
 #pragma unroll
@@ -71,19 +97,31 @@ __device__ bool col_reduce(const double (&acc)[CPL][NV], double *partials, unsig
     const int q = t / RP, col = t % RP;
     double s = 0.0;
     for (int w = 0; w < NW; w++) s += sh[q][col / 32][w][col % 32];
-    partials[((size_t)q * gridDim.x + blockIdx.x) * RP + col] = s;
+    partials[((size_t)q * nblk + blockIdx.x) * RP + col] = s;
   }
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
+  if (threadIdx.x == 0) last = (atomicAdd(ticket + 1 + grp, 1u) == (unsigned)size - 1);
   __syncthreads();
   if (!last) return false;
   __threadfence();
   for (int t = threadIdx.x; t < NV * RP; t += blockDim.x) {
     const int q = t / RP, col = t % RP;
-    double s = 0.0;
-    for (int b = 0; b < (int)gridDim.x; b++) s += __ldcg(partials + ((size_t)q * gridDim.x + b) * RP + col);
-    tot[t] = s;
+    groups[((size_t)q * ngrp + grp) * RP + col] =
+        sum_rows<RP>(partials + ((size_t)q * nblk + grp * kRedGroup) * RP + col, size);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ticket[1 + grp] = 0u;
+    last = (atomicAdd(ticket, 1u) == (unsigned)ngrp - 1);
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  for (int t = threadIdx.x; t < NV * RP; t += blockDim.x) {
+    const int q = t / RP, col = t % RP;
+    tot[t] = sum_rows<RP>(groups + (size_t)q * ngrp * RP + col, ngrp);
   }
   __syncthreads();
   if (threadIdx.x == 0) *ticket = 0u;
@@ -231,46 +269,108 @@ struct MOpStore {  // q = K x (start of the recurrence)
 // products of a level matrix with a block of vectors
 // ---------------------------------------------------------------------------
 
-// 3x3 block rows with component-major values (the handle's BSR3); VT values,
-// T vectors
-template <typename VT, typename T, int CPL, class Op>
+// A block's nine values and its column offset, padded to whole 16-byte words.
+template <typename T>
+struct Staged;
+template <>
+struct Staged<float> {
+  float4 w[3];
+  __device__ void put(const float (&v)[9], int off) {
+    float *p = reinterpret_cast<float *>(w);
+#pragma unroll
+    for (int q = 0; q < 9; q++) p[q] = v[q];
+    p[9] = __int_as_float(off);
+  }
+  __device__ int get(float (&v)[9]) const {
+    const float4 a = w[0], b = w[1];
+    const float2 c = *reinterpret_cast<const float2 *>(w + 2);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w, v[8] = c.x;
+    return __float_as_int(c.y);
+  }
+};
+template <>
+struct Staged<double> {
+  double2 w[5];
+  __device__ void put(const double (&v)[9], int off) {
+    double *p = reinterpret_cast<double *>(w);
+#pragma unroll
+    for (int q = 0; q < 9; q++) p[q] = v[q];
+    p[9] = __longlong_as_double(off);
+  }
+  __device__ int get(double (&v)[9]) const {
+    v[0] = w[0].x, v[1] = w[0].y, v[2] = w[1].x, v[3] = w[1].y, v[4] = w[2].x, v[5] = w[2].y;
+    v[6] = w[3].x, v[7] = w[3].y, v[8] = w[4].x;
+    return (int)__double_as_longlong(w[4].y);
+  }
+};
+
+// 3x3 block rows with component-major values (the handle's BSR3), a warp per
+// block row, lanes over columns.  The vectors' rows come from L1 and L2, so
+// what bounds it is L1's wavefronts (75 % in FP64) and, in FP32, the latency
+// of the loads.  A row's values are read coalesced, one block per lane, while
+// the row before is multiplied, and pass through shared memory, from where
+// every lane takes a block in 3 (FP64: 5) 16-byte words instead of 10 loads.
+// 132,300 equations, 64 columns: FP32 139 -> 105 us, FP64 202 -> 159 us.
+template <typename T, int CPL, class Op>
 __global__ void __launch_bounds__(TPB) k_mspmm_bsr3(int nb, const int *__restrict__ browptr,
-                                                    const int *__restrict__ bcol, const VT *__restrict__ bval,
+                                                    const int *__restrict__ bcol, const T *__restrict__ bval,
                                                     const T *__restrict__ X, Op op, MCol *cols, int R, MState *ms,
                                                     double *partials, unsigned *ticket) {
   if (ms->all_done) return;
   constexpr int RP = 32 * CPL;
   constexpr int NVX = Op::NV > 0 ? Op::NV : 1;
-  const int lane = threadIdx.x & 31;
+  __shared__ Staged<T> stage[NW][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
   double acc[CPL][NVX] = {};
-  for (int br = warp; br < nb; br += nw) {
-    const int s = __ldg(browptr + br), nbr = __ldg(browptr + br + 1) - s;
-    const VT *bv = bval + 9ll * s;
-    T y[3][CPL];
+  int br = warp, s = 0, nbr = 0, j0 = 0;  // the piece (32 blocks of a row) whose values are in v
+  T v[9];
+  int col = 0;
+  auto fetch = [&]() {
+    if (br < nb && j0 + lane < nbr) {
+      col = __ldg(bcol + s + j0 + lane);
+      const T *bv = bval + 9ll * s + j0 + lane;
 #pragma unroll
-    for (int q = 0; q < 3; q++)
-#pragma unroll
-      for (int c = 0; c < CPL; c++) y[q][c] = 0;
+      for (int q = 0; q < 9; q++) v[q] = __ldg(bv + q * nbr);
+    }
+  };
+  if (br < nb) s = __ldg(browptr + br), nbr = __ldg(browptr + br + 1) - s;
+  fetch();
+  T y[3][CPL] = {};
+  while (br < nb) {
+    const int row = br, cnt = min(32, nbr - j0);
+    __syncwarp();
+    if (lane < cnt) stage[wid][lane].put(v, col);
+    __syncwarp();
+    j0 += 32;
+    const bool last = j0 >= nbr;
+    if (last) {
+      br += nw;
+      j0 = 0;
+      if (br < nb) s = __ldg(browptr + br), nbr = __ldg(browptr + br + 1) - s;
+    }
+    fetch();
 #pragma unroll 2
-    for (int j = 0; j < nbr; j++) {
-      const int col = __ldg(bcol + s + j);
-      T v[9];
-#pragma unroll
-      for (int q = 0; q < 9; q++) v[q] = (T)__ldg(bv + q * nbr + j);  // same address in every lane
-      const T *x0 = X + (size_t)(3 * col) * RP + lane;
+    for (int j = 0; j < cnt; j++) {
+      T a[9];
+      const T *x0 = X + (size_t)(3 * stage[wid][j].get(a)) * RP + lane;
 #pragma unroll
       for (int c = 0; c < CPL; c++) {
         const T a0 = __ldg(x0 + 32 * c), a1 = __ldg(x0 + RP + 32 * c), a2 = __ldg(x0 + 2 * RP + 32 * c);
-        y[0][c] += v[0] * a0 + v[1] * a1 + v[2] * a2;
-        y[1][c] += v[3] * a0 + v[4] * a1 + v[5] * a2;
-        y[2][c] += v[6] * a0 + v[7] * a1 + v[8] * a2;
+        y[0][c] += a[0] * a0 + a[1] * a1 + a[2] * a2;
+        y[1][c] += a[3] * a0 + a[4] * a1 + a[5] * a2;
+        y[2][c] += a[6] * a0 + a[7] * a1 + a[8] * a2;
       }
     }
+    if (last) {
 #pragma unroll
-    for (int q = 0; q < 3; q++)
+      for (int q = 0; q < 3; q++)
 #pragma unroll
-      for (int c = 0; c < CPL; c++) op.row(3 * br + q, lane + 32 * c, y[q][c], acc[c]);
+        for (int c = 0; c < CPL; c++) {
+          op.row(3 * row + q, lane + 32 * c, y[q][c], acc[c]);
+          y[q][c] = 0;
+        }
+    }
   }
   op_finish<Op, CPL>(op, acc, partials, ticket, cols, R, ms);
 }
@@ -329,14 +429,17 @@ __device__ __forceinline__ void load_block(const T *__restrict__ a, T (&v)[B * B
 // B x B row-major blocks (coarse levels).  A coarse level has few block rows,
 // so each is split over SPLIT warps of a CTA (each takes every SPLIT-th
 // block); the partial sums meet in shared memory and the first warp of the
-// group applies the row operator.
-template <typename T, int B, int CPL, class Op>
+// group applies the row operator.  Four warps a row, eight where the level has
+// fewer rows than the GPU has CTA slots: a chain of blocks is what such a
+// level waits for (64 columns, the coarse levels of 132,300 equations on
+// average 17 -> 10 us).
+template <typename T, int B, int CPL, int SPLIT, class Op>
 __global__ void __launch_bounds__(TPB) k_mspmm_bsrb(int nb, const int *__restrict__ browptr,
                                                     const int *__restrict__ bcol, const T *__restrict__ bval,
                                                     const T *__restrict__ X, Op op, MCol *cols, int R, MState *ms,
                                                     double *partials, unsigned *ticket) {
   if (ms->all_done) return;
-  constexpr int RP = 32 * CPL, SPLIT = 4, GROUPS = NW / SPLIT;
+  constexpr int RP = 32 * CPL, GROUPS = NW / SPLIT;
   constexpr int NVX = Op::NV > 0 ? Op::NV : 1;
   __shared__ T part[GROUPS][SPLIT][B][RP];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -396,9 +499,12 @@ __global__ void __launch_bounds__(TPB) k_mspmm_bsrb(int nb, const int *__restric
 // transfers, coarsest solve
 // ---------------------------------------------------------------------------
 
-// B_c = Q^T Res: one warp per coarse equation (aggregate G, component q),
-// lanes over columns, rows of the aggregate summed in order; with START the
-// coarse smoothing starts from x = 0 (r = D^-1 b, d = x = c2 r)
+// B_c = Q^T Res: one CTA per aggregate, its nodes dealt to the warps, lanes
+// over columns; a warp reads a residual row once for all K components, and
+// the warps' sums meet in shared memory in warp order.  With START the coarse
+// smoothing starts from x = 0 (r = D^-1 b, d = x = c2 r).  A warp per coarse
+// equation, which read every residual row K times, took 24 us a coarse level
+// (64 columns, 132,300 equations on the finest), now 9.
 template <typename T, int B, int K, int CPL, bool START>
 __global__ void __launch_bounds__(TPB) k_mrestrict(int na, const int *__restrict__ aggptr,
                                                    const int *__restrict__ aggnodes, const T *__restrict__ Q,
@@ -407,36 +513,56 @@ __global__ void __launch_bounds__(TPB) k_mrestrict(int na, const int *__restrict
                                                    const T *__restrict__ dinvc, T c2, const MState *ms) {
   if (ms->all_done) return;
   constexpr int RP = 32 * CPL;
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-  for (int p = warp; p < na * K; p += nw) {
-    const int G = p / K, q = p % K;
-    T acc[CPL];
+  // FP64 with 4 columns a lane would not fit all warps' sums: fewer partial sums then
+  constexpr int PW = (size_t)NW * K * RP * sizeof(T) <= 40 * 1024 ? NW : NW / 4;
+  __shared__ T part[PW][K][RP];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int G = blockIdx.x; G < na; G += gridDim.x) {
+    T acc[K][CPL];
 #pragma unroll
-    for (int c = 0; c < CPL; c++) acc[c] = 0;
-    const int t0 = __ldg(aggptr + G), t1 = __ldg(aggptr + G + 1);
-#pragma unroll 2
-    for (int t = t0; t < t1; t++) {
-      const int i = __ldg(aggnodes + t);
+    for (int q = 0; q < K; q++)
 #pragma unroll
-      for (int e = 0; e < B; e++) {
-        const T qv = __ldg(Q + ((size_t)B * i + e) * K + q);
-        const T *rr = res + ((size_t)B * i + e) * RP + lane;
+      for (int c = 0; c < CPL; c++) acc[q][c] = 0;
+    const int t1 = __ldg(aggptr + G + 1);
+    if (wid < PW)
+      for (int t = __ldg(aggptr + G) + wid; t < t1; t += PW) {
+        const int i = __ldg(aggnodes + t);
 #pragma unroll
-        for (int c = 0; c < CPL; c++) acc[c] += qv * rr[32 * c];
+        for (int e = 0; e < B; e++) {
+          const T *qr = Q + ((size_t)B * i + e) * K;
+          const T *rr = res + ((size_t)B * i + e) * RP + lane;
+          T rv[CPL];
+#pragma unroll
+          for (int c = 0; c < CPL; c++) rv[c] = __ldg(rr + 32 * c);
+#pragma unroll
+          for (int q = 0; q < K; q++) {
+            const T qv = __ldg(qr + q);
+#pragma unroll
+            for (int c = 0; c < CPL; c++) acc[q][c] += qv * rv[c];
+          }
+        }
       }
-    }
+    if (wid < PW)
 #pragma unroll
-    for (int c = 0; c < CPL; c++) {
-      const size_t k = (size_t)p * RP + lane + 32 * c;
-      bc[k] = acc[c];
+      for (int q = 0; q < K; q++)
+#pragma unroll
+        for (int c = 0; c < CPL; c++) part[wid][q][lane + 32 * c] = acc[q][c];
+    __syncthreads();
+    for (int t = threadIdx.x; t < K * RP; t += TPB) {
+      const int q = t / RP, col = t % RP, p = K * G + q;
+      T v = part[0][q][col];
+#pragma unroll
+      for (int w = 1; w < PW; w++) v += part[w][q][col];
+      const size_t k = (size_t)p * RP + col;
+      bc[k] = v;
       if (START) {
-        const T ri = dinvc[p] * acc[c];
+        const T ri = dinvc[p] * v;
         rc[k] = ri;
         dc[k] = c2 * ri;
         xc[k] = c2 * ri;
       }
     }
+    __syncthreads();
   }
 }
 
@@ -465,55 +591,48 @@ __global__ void __launch_bounds__(TPB) k_mprolong(int n, const int *__restrict__
   }
 }
 
-// X_c = M^-1 B_c, a small dense product tiled through shared memory: a CTA
-// owns 32 rows of M (4 per warp), stages 32 columns of M and the matching 32
-// rows of B_c per step; lanes own the right-hand sides
+// X_c = M^-1 B_c, M^-1 dense: a CTA owns 4 rows, its warps every 8th column
+// of them (lanes own the right-hand sides), and the warps' sums meet in shared
+// memory in warp order.  With nc of 6 to 1024 rows the wait for the loads is
+// what it costs, so the chain of a warp is an eighth of a row (32 x 32 tiles
+// through shared memory, 3 CTAs for the last level of 132,300 equations: 13 us
+// against 3.2).
 template <typename T, int CPL>
 __global__ void __launch_bounds__(TPB) k_mdense(int nc, const T *__restrict__ M, const T *__restrict__ b,
                                                 T *__restrict__ x, const MState *ms) {
   if (ms->all_done) return;
-  constexpr int RP = 32 * CPL, TR = 32, TJ = 32;
-  __shared__ T ms_[TR][TJ + 1];
-  __shared__ T bs[TJ][RP];
+  constexpr int RP = 32 * CPL, ROWS = 4;
+  __shared__ T part[NW][ROWS][RP];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int i0 = blockIdx.x * TR; i0 < nc; i0 += gridDim.x * TR) {
-    T s[4][CPL];
+  const int i0 = blockIdx.x * ROWS;
+  T s[ROWS][CPL] = {};
+  const T *row[ROWS];
 #pragma unroll
-    for (int r = 0; r < 4; r++)
+  for (int r = 0; r < ROWS; r++) row[r] = M + (size_t)min(i0 + r, nc - 1) * nc;
+#pragma unroll 4
+  for (int j = wid; j < nc; j += NW) {
+    T bv[CPL];
 #pragma unroll
-      for (int c = 0; c < CPL; c++) s[r][c] = 0;
-    for (int j0 = 0; j0 < nc; j0 += TJ) {
-      for (int t = threadIdx.x; t < TR * TJ; t += blockDim.x) {
-        const int r = t / TJ, j = t % TJ;
-        ms_[r][j] = (i0 + r < nc && j0 + j < nc) ? M[(size_t)(i0 + r) * nc + j0 + j] : T(0);
-      }
-      for (int t = threadIdx.x; t < TJ * RP; t += blockDim.x) {
-        const int j = t / RP, c = t % RP;
-        bs[j][c] = (j0 + j < nc) ? b[(size_t)(j0 + j) * RP + c] : T(0);
-      }
-      __syncthreads();
-#pragma unroll 8
-      for (int j = 0; j < TJ; j++) {
-        T bv[CPL];
+    for (int c = 0; c < CPL; c++) bv[c] = __ldg(b + (size_t)j * RP + lane + 32 * c);
 #pragma unroll
-        for (int c = 0; c < CPL; c++) bv[c] = bs[j][lane + 32 * c];
+    for (int r = 0; r < ROWS; r++) {
+      const T a = __ldg(row[r] + j);
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-          const T a = ms_[4 * wid + r][j];
-#pragma unroll
-          for (int c = 0; c < CPL; c++) s[r][c] += a * bv[c];
-        }
-      }
-      __syncthreads();
+      for (int c = 0; c < CPL; c++) s[r][c] += a * bv[c];
     }
+  }
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const int i = i0 + 4 * wid + r;
-      if (i < nc) {
+  for (int r = 0; r < ROWS; r++)
 #pragma unroll
-        for (int c = 0; c < CPL; c++) x[(size_t)i * RP + lane + 32 * c] = s[r][c];
-      }
-    }
+    for (int c = 0; c < CPL; c++) part[wid][r][lane + 32 * c] = s[r][c];
+  __syncthreads();
+  for (int t = threadIdx.x; t < ROWS * RP; t += TPB) {
+    const int r = t / RP, col = t % RP;
+    if (i0 + r >= nc) break;
+    T v = part[0][r][col];
+#pragma unroll
+    for (int w = 1; w < NW; w++) v += part[w][r][col];
+    x[(size_t)(i0 + r) * RP + col] = v;
   }
 }
 
@@ -527,8 +646,8 @@ template <typename T, int CPL>
 __global__ void __launch_bounds__(TPB) k_mfcg_init(int n, const double *__restrict__ F, const double *__restrict__ Q,
                                                    double *__restrict__ Rv, const double *__restrict__ dscale,
                                                    T *__restrict__ b0, T *__restrict__ r0, T *__restrict__ d0,
-                                                   T *__restrict__ x0, T c2, MCol *cols, int R, MState *ms,
-                                                   double *partials, unsigned *ticket) {
+                                                   T *__restrict__ x0, T c2, int more, MCol *cols, int R,
+                                                   MState *ms, double *partials, unsigned *ticket) {
   constexpr int RP = 32 * CPL;
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
@@ -544,9 +663,11 @@ __global__ void __launch_bounds__(TPB) k_mfcg_init(int n, const double *__restri
       acc[c][1] += ri * ri;
       const T bi = (T)(si * ri);
       b0[k] = bi;
-      r0[k] = bi;
-      d0[k] = c2 * bi;
       x0[k] = c2 * bi;
+      if (more) {
+        r0[k] = bi;
+        d0[k] = c2 * bi;
+      }
     }
   }
   __shared__ double tot[2 * RP];
@@ -579,7 +700,7 @@ __global__ void __launch_bounds__(TPB) k_mfcg_update(int n, double *__restrict__
                                                      const double *__restrict__ P, const double *__restrict__ Q,
                                                      const double *__restrict__ dscale, T *__restrict__ b0,
                                                      T *__restrict__ r0, T *__restrict__ d0, T *__restrict__ x0, T c2,
-                                                     MCol *cols, int R, MState *ms, double *partials,
+                                                     int more, MCol *cols, int R, MState *ms, double *partials,
                                                      unsigned *ticket) {
   if (ms->all_done) return;
   constexpr int RP = 32 * CPL;
@@ -603,9 +724,11 @@ __global__ void __launch_bounds__(TPB) k_mfcg_update(int n, double *__restrict__
       acc[c][0] += ri * ri;
       const T bi = (T)(si * ri);
       b0[k] = bi;
-      r0[k] = bi;
-      d0[k] = c2 * bi;
       x0[k] = c2 * bi;
+      if (more) {
+        r0[k] = bi;
+        d0[k] = c2 * bi;
+      }
     }
   }
   __shared__ double tot[RP];
@@ -726,25 +849,34 @@ struct Multi {
 
   static constexpr int RP = 32 * CPL;
 
+  template <int B, class Op>
+  void bsrb_product(const AmgLevel &L, const T *val, const T *v, const Op &op, unsigned *tk) {
+    if (L.nb <= 4 * kNumSMs)
+      k_mspmm_bsrb<T, B, CPL, 8, Op><<<L.nb, TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, cols, R, ms, partials,
+                                                          tk);
+    else  // 2 block rows per CTA
+      k_mspmm_bsrb<T, B, CPL, 4, Op><<<(int)std::min<int64_t>(((int64_t)L.nb + 1) / 2, 8 * kNumSMs), TPB, 0, s>>>(
+          L.nb, L.browptr, L.bcol, val, v, op, cols, R, ms, partials, tk);
+  }
+
   template <class Op>
   int level_product(int l, const T *v, const Op &op, int slot) {
     const AmgLevel &L = *A->lv[l];
     const T *val = level_vals<T>(m, L);
     const int g = grid_warps(L.nb);
-    const int gb = (int)std::min<int64_t>(((int64_t)L.nb + 1) / 2, 8 * kNumSMs);  // 2 block rows per CTA
-    unsigned *tk = tickets + slot;
+    unsigned *tk = tickets + slot * kTickets;
     if (L.layout == 1)
-      k_mspmm_bsr3<T, T, CPL, Op><<<g, TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, cols, R, ms, partials, tk);
+      k_mspmm_bsr3<T, CPL, Op><<<g, TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, cols, R, ms, partials, tk);
     else if (L.layout == 2)
       k_mspmm_csr<T, T, CPL, Op><<<g, TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, cols, R, ms, partials, tk);
     else if constexpr (Op::NV > 0)  // (operators with column sums run on level 0 only)
       return fail(SGPU_BAD_INPUT, "reduction on a coarse level");
     else if (L.b == 6)
-      k_mspmm_bsrb<T, 6, CPL, Op><<<gb, TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, cols, R, ms, partials, tk);
+      bsrb_product<6>(L, val, v, op, tk);
     else if (L.b == 3)
-      k_mspmm_bsrb<T, 3, CPL, Op><<<gb, TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, cols, R, ms, partials, tk);
+      bsrb_product<3>(L, val, v, op, tk);
     else if (L.b == 1)
-      k_mspmm_bsrb<T, 1, CPL, Op><<<gb, TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, cols, R, ms, partials, tk);
+      bsrb_product<1>(L, val, v, op, tk);
     else
       return fail(SGPU_BAD_INPUT, "unsupported coarse block size");
     count_launches(1);
@@ -756,9 +888,9 @@ struct Multi {
   template <class Op>
   int outer_product(const double *v, const Op &op, int slot) {
     const int g = grid_warps(m->bsr.valid ? m->bsr.nb : m->n);
-    unsigned *tk = tickets + slot;
+    unsigned *tk = tickets + slot * kTickets;
     if (m->bsr.valid)
-      k_mspmm_bsr3<double, double, CPL, Op><<<g, TPB, 0, s>>>(m->bsr.nb, m->bsr.browptr.p, m->bsr.bcol.p,
+      k_mspmm_bsr3<double, CPL, Op><<<g, TPB, 0, s>>>(m->bsr.nb, m->bsr.browptr.p, m->bsr.bcol.p,
                                                               m->bsr.bval.p, v, op, cols, R, ms, partials, tk);
     else
       k_mspmm_csr<double, double, CPL, Op><<<g, TPB, 0, s>>>(n, m->csr.rowptr.p, m->csr.col.p, m->csr.val.p, v, op,
@@ -770,7 +902,7 @@ struct Multi {
 
   template <int B, int K>
   void restrict_bk(const AmgLevel &L, const T *res, T *bc, T *rc, T *dc, T *xc, const T *dinvc, T c2, bool start) {
-    const int g = grid_warps((int64_t)L.na * K);
+    const int g = std::min(L.na, 8 * kNumSMs);
     if (start)
       k_mrestrict<T, B, K, CPL, true><<<g, TPB, 0, s>>>(L.na, L.aggptr.p, L.aggnodes.p, qm<T>(L), res, bc, rc, dc, xc,
                                                         dinvc, c2, ms);
@@ -837,7 +969,7 @@ struct Multi {
     const int deg = A->deg;
     if (l == nl) {
       const T *M = sizeof(T) == 4 ? (const T *)A->M32.p : (const T *)A->M64.p;
-      k_mdense<T, CPL><<<(A->nc + 31) / 32, TPB, 0, s>>>(A->nc, M, cb, cx, ms);
+      k_mdense<T, CPL><<<(A->nc + 3) / 4, TPB, 0, s>>>(A->nc, M, cb, cx, ms);
       count_launches(1);
       xcur[l] = cx;
       return SGPU_OK;
@@ -924,12 +1056,17 @@ struct Multi {
 
   T c2_level0() const { return (T)ch[0].c2_first; }
 
+  // level 0's first smoothing step is followed by others, which read r and d
+  // (the only level being also the bottom one included); writing both without
+  // a reader was an eighth of the update's traffic
+  int more_steps() const { return A->deg > 1 || (A->lv.size() == 1 && A->nc == 0); }
+
   int start() {  // R = F - K X, a cycle, P = S x0
     MOpStore op{Q, RP};
     SGPU_TRY(outer_product(X, op, 0));
     MVecs<T> &V = lv[0];
     k_mfcg_init<T, CPL><<<grid_warps(n), TPB, 0, s>>>(n, F, Q, Rv, m->csr.dscale.p, V.b, V.r, V.d, V.x, c2_level0(),
-                                                      cols, R, ms, partials, tickets + 2);
+                                                      more_steps(), cols, R, ms, partials, tickets + 2 * kTickets);
     count_launches(1);
     return cycle_dir();
   }
@@ -939,7 +1076,7 @@ struct Multi {
     SGPU_TRY(outer_product(P, op, 1));
     MVecs<T> &V = lv[0];
     k_mfcg_update<T, CPL><<<grid_warps(n), TPB, 0, s>>>(n, X, Rv, P, Q, m->csr.dscale.p, V.b, V.r, V.d, V.x,
-                                                        c2_level0(), cols, R, ms, partials, tickets + 2);
+                                                        c2_level0(), more_steps(), cols, R, ms, partials, tickets + 2 * kTickets);
     count_launches(1);
     return cycle_dir();
   }
@@ -965,8 +1102,8 @@ int run_multi(sgpu_matrix m, int R, double *Xh, const double *Fh, int64_t ni, do
   Buf<unsigned> tickets(s);
   SGPU_TRY(cols.alloc(R));
   SGPU_TRY(ms.alloc(1));
-  SGPU_TRY(partials.alloc((size_t)2 * RP * 8 * kNumSMs));
-  SGPU_TRY(tickets.alloc(8));
+  SGPU_TRY(partials.alloc((size_t)2 * RP * (8 * kNumSMs + kRedGroups)));
+  SGPU_TRY(tickets.alloc(kSlots * kTickets));
   for (Buf<double> *b : {&X, &Rv, &P, &Q, &F}) SGPU_TRY(b->alloc((size_t)n * RP));
   SGPU_TRY(stage.alloc((size_t)n * R));
   std::vector<Buf<T> *> owned;
@@ -1010,8 +1147,9 @@ int run_multi(sgpu_matrix m, int R, double *Xh, const double *Fh, int64_t ni, do
   hm.res = res;
   int rc = SGPU_OK;
   const int g = grid_warps((int64_t)n * RP / 32 + 1);
+  Iterations iters;
   auto go = [&]() -> int {
-    SGPU_CUDA(cudaMemsetAsync(tickets.p, 0, 8 * sizeof(unsigned), s));
+    SGPU_CUDA(cudaMemsetAsync(tickets.p, 0, kSlots * kTickets * sizeof(unsigned), s));
     SGPU_CUDA(cudaMemcpyAsync(cols.p, hc.data(), R * sizeof(MCol), cudaMemcpyHostToDevice, s));
     SGPU_CUDA(cudaMemcpyAsync(ms.p, &hm, sizeof(MState), cudaMemcpyHostToDevice, s));
     SGPU_CUDA(cudaMemcpyAsync(stage.p, Fh, (size_t)n * R * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -1027,34 +1165,9 @@ int run_multi(sgpu_matrix m, int R, double *Xh, const double *Fh, int64_t ni, do
     count_launches(iv ? 2 : 1);
     SGPU_CUDA(cudaEventRecord(m->ev0, s));
     SGPU_TRY(M.start());
-    // iterations in graphs of 8; the host reads the small state between them
-    cudaGraph_t graph;
-    cudaGraphExec_t exec = nullptr;
-    const int64_t before = sgpu_kernel_launches();
-    SGPU_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-    int crc = SGPU_OK;
-    for (int k = 0; k < 8 && crc == SGPU_OK; k++) crc = M.iteration();
-    cudaError_t e = cudaStreamEndCapture(s, &graph);
-    if (crc != SGPU_OK) return crc;
-    if (e != cudaSuccess) return fail(SGPU_CUDA_ERROR, std::string("cudaStreamEndCapture: ") + cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) return fail(SGPU_CUDA_ERROR, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-    const int64_t nodes = sgpu_kernel_launches() - before;
-    count_launches(-nodes);
-    int lrc = SGPU_OK;
-    for (int64_t it = 0;; it += 8) {
-      MState cur{};
-      SGPU_CUDA(cudaMemcpyAsync(&cur, ms.p, sizeof(MState), cudaMemcpyDeviceToHost, s));
-      SGPU_CUDA(cudaStreamSynchronize(s));
-      if (cur.all_done || it > ni + 8) break;
-      e = cudaGraphLaunch(exec, s);
-      if (e != cudaSuccess) { lrc = fail(SGPU_CUDA_ERROR, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e)); break; }
-      count_launches(nodes);
-    }
-    cudaGraphExecDestroy(exec);
+    SGPU_TRY(iters.run(s, A.side, &ms.p->all_done, ni + 8, [&]() { return M.iteration(); }));
     SGPU_CUDA(cudaEventRecord(m->ev1, s));
-    return lrc;
+    return SGPU_OK;
   };
   rc = go();
   if (rc == SGPU_OK) {

@@ -199,7 +199,6 @@ struct PcgState {
   // control
   int done, pause, status;
   double last_dot;
-  int64_t loops;  // iterations run by one launch of a device-side loop graph
 };
 
 // Per-handle scratch vectors of the iteration.
