@@ -2929,8 +2929,8 @@ int amg_set_rigid_body_modes(sgpu_matrix m, int64_t nn, int ndofn, const double 
   PBuf<int64_t> cn;
   SGPU_TRY(xyz.alloc((size_t)nn * 3));
   SGPU_TRY(cn.alloc((size_t)nn * ndofn));
-  SGPU_CUDA(cudaMemcpyAsync(xyz.p, coords_h, (size_t)nn * 3 * sizeof(double), cudaMemcpyHostToDevice, m->stream));
-  SGPU_CUDA(cudaMemcpyAsync(cn.p, cn_h, (size_t)nn * ndofn * sizeof(int64_t), cudaMemcpyHostToDevice, m->stream));
+  SGPU_CUDA(copy_in(xyz.p, coords_h, (size_t)nn * 3 * sizeof(double), m->stream));
+  SGPU_CUDA(copy_in(cn.p, cn_h, (size_t)nn * ndofn * sizeof(int64_t), m->stream));
   SGPU_CUDA(cudaMemsetAsync(A.B0.p, 0, (size_t)m->n * k * sizeof(double), m->stream));
   k_rigid_body_modes<<<(unsigned)((nn + 255) / 256), 256, 0, m->stream>>>(nn, ndofn, k, xyz.p, cn.p, c[0], c[1],
                                                                            c[2], A.B0.p, m->n);
@@ -2947,7 +2947,7 @@ int amg_set_nullspace(sgpu_matrix m, int k, const double *B_host) {
   A.clear();
   A.k0 = k;
   SGPU_TRY(A.B0.alloc((size_t)m->n * k));
-  SGPU_CUDA(cudaMemcpyAsync(A.B0.p, B_host, (size_t)m->n * k * sizeof(double), cudaMemcpyHostToDevice, m->stream));
+  SGPU_CUDA(copy_in(A.B0.p, B_host, (size_t)m->n * k * sizeof(double), m->stream));
   SGPU_CUDA(cudaStreamSynchronize(m->stream));
   return SGPU_OK;
 }
@@ -4849,7 +4849,7 @@ int amg_batch_run(sgpu_matrix m, int nsys, const int64_t *sys_rows, double *x, c
   std::vector<BSys> hsys(nsys);
   for (auto &b : hsys) { memset(&b, 0, sizeof(b)); b.ani = -1; }
   SGPU_CUDA(cudaMemcpyAsync(sys.p, hsys.data(), nsys * sizeof(BSys), cudaMemcpyHostToDevice, s));
-  SGPU_CUDA(cudaMemcpyAsync(m->w.f.p, f, n * sizeof(double), cudaMemcpyHostToDevice, s));
+  SGPU_CUDA(copy_in(m->w.f.p, f, n * sizeof(double), s));
   k_b_rowsys<<<grid_for((int64_t)nsys * 32), TPB, 0, s>>>(nsys, sysptr.p, rowsys.p);
   count_launches(1);
   A.batch_zr = pzr.p;
@@ -4861,7 +4861,7 @@ int amg_batch_run(sgpu_matrix m, int nsys, const int64_t *sys_rows, double *x, c
   A.batch_zr = A.batch_zq = nullptr;
   SGPU_CUDA(cudaEventRecord(m->ev1, s));
   if (rc != SGPU_OK) return rc;
-  SGPU_CUDA(cudaMemcpyAsync(x, m->w.x.p, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+  SGPU_CUDA(copy_out(x, m->w.x.p, n * sizeof(double), s));
   SGPU_CUDA(cudaMemcpyAsync(hsys.data(), sys.p, nsys * sizeof(BSys), cudaMemcpyDeviceToHost, s));
   SGPU_CUDA(cudaStreamSynchronize(s));
   float solve_ms = 0.f;

@@ -1152,10 +1152,10 @@ int run_multi(sgpu_matrix m, int R, double *Xh, const double *Fh, int64_t ni, do
     SGPU_CUDA(cudaMemsetAsync(tickets.p, 0, kSlots * kTickets * sizeof(unsigned), s));
     SGPU_CUDA(cudaMemcpyAsync(cols.p, hc.data(), R * sizeof(MCol), cudaMemcpyHostToDevice, s));
     SGPU_CUDA(cudaMemcpyAsync(ms.p, &hm, sizeof(MState), cudaMemcpyHostToDevice, s));
-    SGPU_CUDA(cudaMemcpyAsync(stage.p, Fh, (size_t)n * R * sizeof(double), cudaMemcpyHostToDevice, s));
+    SGPU_CUDA(copy_in(stage.p, Fh, (size_t)n * R * sizeof(double), s));
     k_to_rows<<<g, TPB, 0, s>>>(n, R, RP, stage.p, F.p);
     if (iv) {
-      SGPU_CUDA(cudaMemcpyAsync(stage.p, Xh, (size_t)n * R * sizeof(double), cudaMemcpyHostToDevice, s));
+      SGPU_CUDA(copy_in(stage.p, Xh, (size_t)n * R * sizeof(double), s));
       k_to_rows<<<g, TPB, 0, s>>>(n, R, RP, stage.p, X.p);
     } else {
       SGPU_CUDA(cudaMemsetAsync(X.p, 0, (size_t)n * RP * sizeof(double), s));
@@ -1173,9 +1173,10 @@ int run_multi(sgpu_matrix m, int R, double *Xh, const double *Fh, int64_t ni, do
   if (rc == SGPU_OK) {
     k_to_cols<<<g, TPB, 0, s>>>(n, R, RP, X.p, stage.p);
     count_launches(1);
-    cudaMemcpyAsync(Xh, stage.p, (size_t)n * R * sizeof(double), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(hc.data(), cols.p, R * sizeof(MCol), cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) rc = fail(SGPU_CUDA_ERROR, "copy-back failed");
+    if (copy_out(Xh, stage.p, (size_t)n * R * sizeof(double), s) != cudaSuccess ||
+        cudaMemcpyAsync(hc.data(), cols.p, R * sizeof(MCol), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+      rc = fail(SGPU_CUDA_ERROR, "copy-back failed");
   }
   float solve_ms = 0.f;
   if (rc == SGPU_OK) cudaEventElapsedTime(&solve_ms, m->ev0, m->ev1);

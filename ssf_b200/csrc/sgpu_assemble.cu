@@ -16,9 +16,10 @@
 //     row) equation pairs as 64-bit keys, and one radix sort + unique gives
 //     the SCR pattern (symcomprow::initiate, GEFEL/scr.cpp:556), from which
 //     the full CSR is built (sgpu_matrix.cu);
-//  2. colouring: greedy first-fit on the host over node masks -- elements of
-//     one colour share no node, so their element matrices can be added into
-//     the CSR without atomics, and the sum order is fixed (deterministic);
+//  2. colouring: greedy first-fit on the host over node masks, beside the
+//     copies and the pattern -- elements of one colour share no node, so their
+//     element matrices can be added into the CSR without atomics, and the sum
+//     order is fixed (deterministic);
 //  3. one launch per colour: one warp per element; lanes 0..G-1 compute the
 //     Jacobian and Cartesian shape-function gradients of one Gauss point each
 //     (derivatives_3d, GEFEL/difcalc.cpp:487) into shared memory, then every
@@ -31,6 +32,8 @@
 #include <climits>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
+#include <thread>
 #include <vector>
 
 #include "sgpu_internal.cuh"
@@ -1990,16 +1993,21 @@ int read_err(const unsigned *err_d, cudaStream_t s, unsigned *out) {
 }
 
 // greedy first-fit colouring over per-node colour masks: an element takes the
-// lowest colour no element sharing one of its nodes already has
-int colour_elements(int64_t nn, int64_t ne, int nne, const int64_t *elems, std::vector<int> &order,
-                    std::vector<int> &offsets) {
+// lowest colour no element sharing one of its nodes already has.  Returns an
+// error's text, or null.
+const char *colour_elements(int64_t nn, int64_t ne, int nne, const int64_t *elems, std::vector<int> &order,
+                            std::vector<int> &offsets) {
   std::vector<uint64_t> mask((size_t)nn, 0);
   std::vector<int> colour((size_t)ne);
   int ncol = 0;
   for (int64_t e = 0; e < ne; e++) {
     uint64_t used = 0;
-    for (int a = 0; a < nne; a++) used |= mask[(size_t)elems[e * nne + a]];
-    if (used == ~0ull) return fail(SGPU_BAD_INPUT, "mesh needs more than 64 element colours");
+    for (int a = 0; a < nne; a++) {
+      const int64_t node = elems[e * nne + a];
+      if (node < 0 || node >= nn) return "element node out of range";
+      used |= mask[(size_t)node];
+    }
+    if (used == ~0ull) return "mesh needs more than 64 element colours";
     const int c = __builtin_ctzll(~used);
     colour[(size_t)e] = c;
     ncol = std::max(ncol, c + 1);
@@ -2011,7 +2019,7 @@ int colour_elements(int64_t nn, int64_t ne, int nne, const int64_t *elems, std::
   order.resize((size_t)ne);
   std::vector<int> fill(offsets.begin(), offsets.end() - 1);
   for (int64_t e = 0; e < ne; e++) order[(size_t)fill[colour[(size_t)e]]++] = (int)e;
-  return SGPU_OK;
+  return nullptr;
 }
 
 // stream-ordered temporaries of the pattern build (the device pool keeps the
@@ -2166,6 +2174,39 @@ struct AssemblyData {
   // precondition
   DevBuf<int> iptr, inc;
   bool node_rows = false;
+};
+
+// The colouring (3 ms for 330,000 elements, one after the other by its
+// definition) in a thread of its own beside the copies and the pattern's
+// construction; joined before its lists are read and on every way out.
+struct Colouring {
+  std::thread t;
+  const char *error = nullptr;
+  void run(int64_t nn, int64_t ne, int nne, const int64_t *elems, AssemblyData &ad) noexcept {
+    try {
+      error = colour_elements(nn, ne, nne, elems, ad.order, ad.offsets);
+    } catch (const std::exception &) {
+      error = "out of host memory for the element colours";
+    }
+  }
+  void start(int64_t nn, int64_t ne, int nne, const int64_t *elems, AssemblyData &ad) {
+    if (ne < kAside) return;
+    try {
+      t = std::thread([=, &ad]() { run(nn, ne, nne, elems, ad); });
+    } catch (const std::exception &) {  // no thread to be had: done by finish
+    }
+  }
+  const char *finish(int64_t nn, int64_t ne, int nne, const int64_t *elems, AssemblyData &ad) {
+    if (t.joinable()) t.join();
+    else run(nn, ne, nne, elems, ad);
+    return error;
+  }
+  void stop() {
+    if (t.joinable()) t.join();
+  }
+  ~Colouring() { stop(); }
+  // a thread costs about as much as colouring this many elements
+  static constexpr int64_t kAside = 8192;
 };
 
 // SGPU_HEX8_FULL=1: isotropic hexahedra through the full B^T D B product of
@@ -2383,7 +2424,9 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   const int ndofe = nne * ndofn;
   sgpu_matrix m = new sgpu_matrix_s();
   m->src_sym = 1;
+  Colouring colouring;
   auto bail = [&](int st) {
+    colouring.stop();  // it writes into m's lists
     if (m->stream) cudaStreamSynchronize(m->stream);
     cudaStream_t s = m->own_stream;
     cudaEvent_t a = m->ev0, b = m->ev1;
@@ -2401,6 +2444,7 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   m->asm_data = new sgpu_assembly_s();
   AssemblyData &ad = m->asm_data->d;
   ad.kind = kind; ad.nne = nne; ad.ndofn = ndofn; ad.nn = nn; ad.ne = ne;
+  colouring.start(nn, ne, nne, mesh->elems, ad);
   int st;
   cudaEvent_t t0, t1;
   cudaEventCreate(&t0);
@@ -2423,18 +2467,17 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   DevBuf<int64_t> cn_d;
   BAIL_ON(cn_d.alloc(nn * ndofn));
   BAIL_ON(ad.cne.alloc(ne * ndofe));
-  cudaMemcpyAsync(ad.coords.p, mesh->coords, nn * 3 * sizeof(double), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(ad.elems.p, mesh->elems, ne * nne * sizeof(int64_t), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(ad.emat.p, ad.general ? mesh->dmat : mesh->emat, ne * nmatp * sizeof(double),
-                  cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(cn_d.p, mesh->cn, nn * ndofn * sizeof(int64_t), cudaMemcpyHostToDevice, s);
+  copy_in(ad.coords.p, mesh->coords, nn * 3 * sizeof(double), s);
+  copy_in(ad.elems.p, mesh->elems, ne * nne * sizeof(int64_t), s);
+  copy_in(ad.emat.p, ad.general ? mesh->dmat : mesh->emat, ne * nmatp * sizeof(double), s);
+  copy_in(cn_d.p, mesh->cn, nn * ndofn * sizeof(int64_t), s);
   if (mesh->thick) {
     BAIL_ON(ad.thick.alloc(ne));
-    cudaMemcpyAsync(ad.thick.p, mesh->thick, ne * sizeof(double), cudaMemcpyHostToDevice, s);
+    copy_in(ad.thick.p, mesh->thick, ne * sizeof(double), s);
   }
   if (mesh->rho) {
     BAIL_ON(ad.rho.alloc(ne));
-    cudaMemcpyAsync(ad.rho.p, mesh->rho, ne * sizeof(double), cudaMemcpyHostToDevice, s);
+    copy_in(ad.rho.p, mesh->rho, ne * sizeof(double), s);
   }
   DevBuf<unsigned> err;
   BAIL_ON(err.alloc(1));
@@ -2523,11 +2566,10 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   cudaEventDestroy(t0);
   cudaEventDestroy(t1);
 
-  // colouring (host) and the per-colour element lists
-  st = colour_elements(nn, ne, nne, mesh->elems, ad.order, ad.offsets);
-  if (st != SGPU_OK) return bail(st);
+  // the per-colour element lists
+  if (const char *why = colouring.finish(nn, ne, nne, mesh->elems, ad)) return bail(fail(SGPU_BAD_INPUT, why));
   if (ad.elist.alloc(ne) != SGPU_OK) return bail(SGPU_CUDA_ERROR);
-  cudaMemcpyAsync(ad.elist.p, ad.order.data(), ne * sizeof(int), cudaMemcpyHostToDevice, s);
+  copy_in(ad.elist.p, ad.order.data(), ne * sizeof(int), s);
   float asm_ms = 0.f;
   st = assemble_values(m, ad, kind, &asm_ms);
   if (st != SGPU_OK) return bail(st);
@@ -2558,8 +2600,8 @@ SGPU_API int sgpu_assembly_lift(sgpu_matrix m, const double *rnode, double *rhs)
   const int64_t nr = ad.nn * ad.ndofn;
   SGPU_TRY(rn.alloc(nr));
   SGPU_TRY(f.alloc(m->n));
-  SGPU_CUDA(cudaMemcpyAsync(rn.p, rnode, nr * sizeof(double), cudaMemcpyHostToDevice, s));
-  SGPU_CUDA(cudaMemcpyAsync(f.p, rhs, m->n * sizeof(double), cudaMemcpyHostToDevice, s));
+  SGPU_CUDA(copy_in(rn.p, rnode, nr * sizeof(double), s));
+  SGPU_CUDA(copy_in(f.p, rhs, m->n * sizeof(double), s));
   const int ncol = (int)ad.offsets.size() - 1;
   for (int col = 0; col < ncol; col++) {
     const int beg = ad.offsets[col], cnt = ad.offsets[col + 1] - beg;
@@ -2645,12 +2687,11 @@ SGPU_API int sgpu_assemble_copy(sgpu_matrix src, int32_t kind, const double *ema
   m->bsr.valid = false;
   m->bsr.nb = -1;  // examined on first use
   m->bsr.known = src->bsr.known;
-  if (emat && cudaMemcpyAsync(ad.emat.p, emat, ad.ne * (ad.general ? 36 : 2) * sizeof(double),
-                              cudaMemcpyHostToDevice, s) != cudaSuccess)
+  if (emat && copy_in(ad.emat.p, emat, ad.ne * (ad.general ? 36 : 2) * sizeof(double), s) != cudaSuccess)
     return bail(fail(SGPU_CUDA_ERROR, "copy of emat failed"));
   if (rho) {
     if (ad.rho.alloc(ad.ne) != SGPU_OK) return bail(SGPU_CUDA_ERROR);
-    if (cudaMemcpyAsync(ad.rho.p, rho, ad.ne * sizeof(double), cudaMemcpyHostToDevice, s) != cudaSuccess)
+    if (copy_in(ad.rho.p, rho, ad.ne * sizeof(double), s) != cudaSuccess)
       return bail(fail(SGPU_CUDA_ERROR, "copy of rho failed"));
   }
   float ms = 0.f;
@@ -2678,11 +2719,10 @@ SGPU_API int sgpu_reassemble(sgpu_matrix m, int32_t kind, const double *emat, co
   if (kind != ad.kind && !scalar_ok) return fail(SGPU_BAD_INPUT, "element kind differs from the pattern's");
   cudaStream_t s = m->stream;
   if (emat)
-    SGPU_CUDA(cudaMemcpyAsync(ad.emat.p, emat, ad.ne * (ad.general ? 36 : 2) * sizeof(double),
-                              cudaMemcpyHostToDevice, s));
+    SGPU_CUDA(copy_in(ad.emat.p, emat, ad.ne * (ad.general ? 36 : 2) * sizeof(double), s));
   if (rho) {
     SGPU_TRY(ad.rho.alloc(ad.ne));
-    SGPU_CUDA(cudaMemcpyAsync(ad.rho.p, rho, ad.ne * sizeof(double), cudaMemcpyHostToDevice, s));
+    SGPU_CUDA(copy_in(ad.rho.p, rho, ad.ne * sizeof(double), s));
   }
   float ms = 0.f;
   SGPU_TRY(assemble_values(m, ad, kind, &ms));

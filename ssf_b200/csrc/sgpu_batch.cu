@@ -1045,7 +1045,7 @@ extern "C" SGPU_API int sgpu_matrix_pcg_batch(sgpu_matrix m, int32_t nsys, const
   cudaStream_t s = m->stream;
   const size_t n = (size_t)m->n;
   Work &w = m->w;
-  SGPU_CUDA(cudaMemcpyAsync(w.f.p, f, n * sizeof(double), cudaMemcpyHostToDevice, s));
+  SGPU_CUDA(copy_in(w.f.p, f, n * sizeof(double), s));
   // the plan: segment rows S and lanes per row L; tuned on ~32 iterations of
   // this batch when asked (the iterate is reset for the real solve)
   // SGPU_BATCH_FORM=graph: the segmented graph-of-launches form below;
@@ -1089,7 +1089,7 @@ extern "C" SGPU_API int sgpu_matrix_pcg_batch(sgpu_matrix m, int32_t nsys, const
     SGPU_CUDA(cudaMemsetAsync(w.x.p, 0, n * sizeof(double), s));
     SGPU_TRY(run_batch(m, b, best, w.x.p, w.f.p, w.r.p, w.h.p, w.d.p, w.p.p, ni, res, zero, hs, &its, &ms));
   }
-  SGPU_CUDA(cudaMemcpyAsync(x, w.x.p, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+  SGPU_CUDA(copy_out(x, w.x.p, n * sizeof(double), s));
   SGPU_CUDA(cudaStreamSynchronize(s));
   int worst = SGPU_OK;
   for (int k = 0; k < nsys; k++) {

@@ -91,6 +91,20 @@ struct RowSums {
 cudaError_t devmem_get(void **p, size_t *bytes);
 void devmem_put(void *p, size_t bytes);
 
+// Blocks released by this thread within the scope wait for the device once,
+// here, instead of once each.  For the end of a handle: nothing is launched
+// meanwhile that uses them.
+struct DevIdle {
+  DevIdle();
+  ~DevIdle();
+};
+
+// Copies between a caller's host array and the device, ordered on s
+// (sgpu_transfer.cu).  As with cudaMemcpyAsync, a pageable array may be reused
+// (copy_in) or holds the result (copy_out) on return.
+cudaError_t copy_in(void *dst, const void *src, size_t bytes, cudaStream_t s);
+cudaError_t copy_out(void *dst, const void *src, size_t bytes, cudaStream_t s);
+
 template <class T>
 struct DevBuf {
   T *p = nullptr;

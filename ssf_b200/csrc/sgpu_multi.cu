@@ -329,10 +329,10 @@ extern "C" SGPU_API int sgpu_matrix_pcg_multi(sgpu_matrix m, int32_t nrhs, doubl
   SGPU_CUDA(cudaMemsetAsync(cs.p, 0, RP * sizeof(ColState), s));
   SGPU_CUDA(cudaEventRecord(m->ev0, s));
   // upload (host column blocks -> row-major blocks)
-  SGPU_CUDA(cudaMemcpyAsync(hostcols.p, F, (size_t)n * R * sizeof(double), cudaMemcpyHostToDevice, s));
+  SGPU_CUDA(copy_in(hostcols.p, F, (size_t)n * R * sizeof(double), s));
   k_pack<<<kNumSMs * 8, TPB, 0, s>>>(n, R, RP, hostcols.p, Fd.p);
   if (iv) {
-    SGPU_CUDA(cudaMemcpyAsync(hostcols.p, X, (size_t)n * R * sizeof(double), cudaMemcpyHostToDevice, s));
+    SGPU_CUDA(copy_in(hostcols.p, X, (size_t)n * R * sizeof(double), s));
     k_pack<<<kNumSMs * 8, TPB, 0, s>>>(n, R, RP, hostcols.p, Xd.p);
   } else {
     SGPU_CUDA(cudaMemsetAsync(Xd.p, 0, nn * sizeof(double), s));
@@ -360,7 +360,7 @@ extern "C" SGPU_API int sgpu_matrix_pcg_multi(sgpu_matrix m, int32_t nrhs, doubl
   SGPU_CUDA(cudaEventRecord(m->ev1, s));
   k_unpack<<<kNumSMs * 8, TPB, 0, s>>>(n, R, RP, Xd.p, hostcols.p);
   count_launches(1);
-  SGPU_CUDA(cudaMemcpyAsync(X, hostcols.p, (size_t)n * R * sizeof(double), cudaMemcpyDeviceToHost, s));
+  SGPU_CUDA(copy_out(X, hostcols.p, (size_t)n * R * sizeof(double), s));
   std::vector<ColState> h(RP);
   SGPU_CUDA(cudaMemcpyAsync(h.data(), cs.p, RP * sizeof(ColState), cudaMemcpyDeviceToHost, s));
   SGPU_CUDA(cudaStreamSynchronize(s));

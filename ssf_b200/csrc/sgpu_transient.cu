@@ -102,7 +102,10 @@ int transient(sgpu_matrix K, sgpu_matrix C, const double *rhs, double *d, double
     cudaStream_t s = A->own_stream;
     cudaEvent_t e0 = A->ev0, e1 = A->ev1;
     cudaStreamSynchronize(A->stream);
-    delete A;
+    {
+      DevIdle idle;
+      delete A;
+    }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (s) cudaStreamDestroy(s);
@@ -116,9 +119,9 @@ int transient(sgpu_matrix K, sgpu_matrix C, const double *rhs, double *d, double
   cudaStream_t c_stream_saved = C->stream, k_stream_saved = K->stream;
   C->stream = s;  // C's (d-form) or K's (v-form) products run on A's stream for ordering
   K->stream = s;
-  cudaMemcpyAsync(d_d.p, d, n * sizeof(double), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(v_d.p, v, n * sizeof(double), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(rhs_d.p, rhs, n * sizeof(double), cudaMemcpyHostToDevice, s);
+  copy_in(d_d.p, d, n * sizeof(double), s);
+  copy_in(v_d.p, v, n * sizeof(double), s);
+  copy_in(rhs_d.p, rhs, n * sizeof(double), s);
   const int vb = blocks_for(n);
   int64_t total_its = 0;
   double total_ms = 0.0, last_true = 0.0, setup_ms = 0.0;
@@ -166,8 +169,8 @@ int transient(sgpu_matrix K, sgpu_matrix C, const double *rhs, double *d, double
   C->stream = c_stream_saved;
   K->stream = k_stream_saved;
   if (st != SGPU_OK) return cleanup(st);
-  cudaMemcpyAsync(d, d_d.p, n * sizeof(double), cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(v, v_d.p, n * sizeof(double), cudaMemcpyDeviceToHost, s);
+  copy_out(d, d_d.p, n * sizeof(double), s);
+  copy_out(v, v_d.p, n * sizeof(double), s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return cleanup(fail(SGPU_CUDA_ERROR, "transient copy-back failed"));
   if (info) {
     info->iterations = total_its;

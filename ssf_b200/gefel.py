@@ -253,9 +253,7 @@ def pcg_multi_blocks(dm: "DeviceMatrix", Fc, ni=100000, res=1e-20, zero=1e-30, X
         Xc = np.zeros_like(Fc) if X0c is None else np.array(X0c, dtype=np.float64)
     elif X0c is not None:
         Xc[...] = X0c
-    else:
-        Xc[...] = 0.0
-    X0 = X0c
+    X0 = X0c  # without it the solve starts from zero by itself and writes every column
     ani = np.full(R, -1, dtype=np.int64)
     ares = np.full(R, np.nan)
     st = np.zeros(R, dtype=np.int32)
@@ -267,7 +265,10 @@ def pcg_multi_blocks(dm: "DeviceMatrix", Fc, ni=100000, res=1e-20, zero=1e-30, X
     else:
         rc = L.lib().sgpu_matrix_pcg_multi(dm.h, R, Xc, Fc, int(ni), float(res), float(zero), 0 if X0 is None else 1,
                                            ani.ctypes.data, ares.ctypes.data, st.ctypes.data, C.byref(info))
-    L.check(rc, (L.OK, L.NOT_CONVERGED, L.BREAKDOWN, L.ZERO_RHS))
+    ok = (L.OK, L.NOT_CONVERGED, L.BREAKDOWN, L.ZERO_RHS)
+    if rc not in ok and X0 is None:
+        Xc[...] = 0.0
+    L.check(rc, ok)
     out = [Result(int(st[c]), int(ani[c]) if ani[c] >= 0 else None, float(ares[c]) if ani[c] >= 0 else None,
                   info.as_dict()) for c in range(R)]
     return Xc, out
