@@ -468,9 +468,9 @@ inline cudaError_t launch_resident(ResidentArgs a, int64_t nnz, int grid, cudaSt
 // rows.  Per iteration:
 //   product  p = A d over the CTA's rows, d.p
 //   barrier  alpha
-//   update   x, r, h over the CTA's rows; r.r, r.h
+//   update   r, h over the CTA's rows; r.r, r.h
 //   barrier  beta, stopping test
-//   d = beta d + h
+//   x += alpha d (the last iteration's too), d = beta d + h
 //   barrier
 //
 // The matrix arrives by bulk copies (cp.async.bulk on an mbarrier) into
@@ -483,14 +483,16 @@ inline cudaError_t launch_resident(ResidentArgs a, int64_t nnz, int grid, cudaSt
 // copies leave L2 to the vectors.
 //
 // Measured per iteration (B200), against three launches per iteration in a
-// graph: 1,008,600 equations in 3x3 blocks (683 MB) 149.7 -> 129.4 us, of
-// which the bytes take 104.5 and the barriers and vectors about 12; 132,300
-// equations (84 MB, in L2) 33.1 -> 21.8 us; 481,200 equations of CSR (104
-// MB) 39.4 -> 27.8 us; 2,130,048 of CSR (640 MB) 196 -> 178 us.  Variants that
-// lost: plain loads instead of bulk copies (152 us on the first), 12 or 24
-// warps there (133 to 139), evict-last copies (157).  A second stage per warp
-// (LPR 16) lost to wider tiles (139): a tile's gathers, not its copy, are
-// what a warp waits for.
+// graph: 1,008,600 equations in 3x3 blocks (683 MB) 149.7 -> 123 us, of which
+// the bytes take 104.5; 132,300 equations (84 MB, in L2) 33.1 -> 21.9 us;
+// 481,200 equations of CSR (104 MB) 39.4 -> 27.1 us; 2,130,048 of CSR (640 MB)
+// 196 -> 165 us.  x is updated with d, which both read, and not with r, which
+// d has to wait for.  Variants that lost: plain loads instead of bulk copies
+// (152 us on the first), evict-last copies (157), 12 or 24 warps (133 to 139
+// there; on CSR of 2,130,048 equations 12 warps 178, 20 warps 165 to 168), the
+// vector phases as functions of their own (CSR of 481,200 equations 31.8).  A
+// second stage per warp (LPR 16) lost to wider tiles (139): a tile's gathers,
+// not its copy, are what a warp waits for.
 __device__ __forceinline__ unsigned ring_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool ring_test(unsigned long long *bar, unsigned parity) {
   unsigned ok;
@@ -540,6 +542,59 @@ struct TileArgs {
   GridSync *gs;
   long long most;
 };
+
+// The vector phases over the rows [r0, r1) of the CTA.  A thread's loads of
+// two rows are in flight together (its stores may alias its next loads for all
+// the compiler knows, so a plain loop has one row's); of four, the registers
+// cost the product more than it gives (1,008,600 equations in 3x3 blocks 128
+// us an iteration, with one row 126.5, with two 121.5).
+constexpr int kRowBatch = 2;
+template <int TPBX>
+__device__ __forceinline__ double2 tiles_residual(double *r, double *h, const double *p, const double *diag, double alpha,
+                                               int r0, int r1) {  // r -= alpha p, h = r / diag; r.r, r.h
+  double2 v = {0.0, 0.0};
+  for (int i0 = r0 + threadIdx.x; i0 < r1; i0 += kRowBatch * TPBX) {
+    double rv[kRowBatch], pv[kRowBatch], g[kRowBatch];
+#pragma unroll
+    for (int z = 0; z < kRowBatch; z++) {
+      const int i = i0 + z * TPBX;
+      if (i < r1) rv[z] = r[i], pv[z] = p[i], g[z] = diag ? __ldg(diag + i) : 1.0;
+    }
+#pragma unroll
+    for (int z = 0; z < kRowBatch; z++) {
+      const int i = i0 + z * TPBX;
+      if (i < r1) {
+        const double ri = fma(-alpha, pv[z], rv[z]);
+        const double hi = diag ? ri / g[z] : ri;
+        r[i] = ri;
+        h[i] = hi;
+        v.x += ri * ri;
+        v.y += ri * hi;
+      }
+    }
+  }
+  return v;
+}
+template <int TPBX>
+__device__ __forceinline__ void tiles_direction(double *x, double *d, const double *h, double alpha, double beta,
+                                             bool stop, int r0, int r1) {  // x += alpha d, d = beta d + h
+  for (int i0 = r0 + threadIdx.x; i0 < r1; i0 += kRowBatch * TPBX) {
+    double xv[kRowBatch], dv[kRowBatch], hv[kRowBatch];
+#pragma unroll
+    for (int z = 0; z < kRowBatch; z++) {
+      const int i = i0 + z * TPBX;
+      if (i < r1) xv[z] = x[i], dv[z] = d[i], hv[z] = h[i];
+    }
+#pragma unroll
+    for (int z = 0; z < kRowBatch; z++) {
+      const int i = i0 + z * TPBX;
+      if (i < r1) {
+        x[i] = fma(alpha, dv[z], xv[z]);
+        if (!stop) d[i] = fma(beta, dv[z], hv[z]);
+      }
+    }
+  }
+}
 
 template <int ROWS, int LPR, int TPBX>
 __global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const TileMat m) {
@@ -624,7 +679,7 @@ __global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const T
           const int b = sp[u] - e0, len = sp[u + 1] - e0 - b;
           const double *v = vals + b;
           const int *c = cols + b;
-          constexpr int U = LPR == 2 ? 7 : 4;
+          constexpr int U = LPR == 2 ? 9 : 4;
           for (int e = sub; e < len; e += LPR * U) {
             double xx[U];
 #pragma unroll
@@ -696,21 +751,12 @@ __global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const T
     double dp[1] = {acc}, alpha;
     ok = grid_barrier_sum<1>(dp, a.gs, ++epoch, sums) && !bad;
     if (!ok || cg.direction(dp[0], nom, alpha)) break;
-    double v[2] = {0.0, 0.0};
-#pragma unroll 4
-    for (int i = r0 + threadIdx.x; i < r1; i += TPBX) {
-      a.x[i] = fma(alpha, a.d[i], a.x[i]);
-      const double ri = fma(-alpha, a.p[i], a.r[i]);
-      const double hi = prec ? ri / __ldg(a.diag + i) : ri;
-      a.r[i] = ri;
-      a.h[i] = hi;
-      v[0] += ri * ri;
-      v[1] += ri * hi;
-    }
+    const double2 t = tiles_residual<TPBX>(a.r, a.h, a.p, prec ? a.diag : nullptr, alpha, r0, r1);
+    double v[2] = {t.x, t.y};
     ok = grid_barrier_sum<2>(v, a.gs, ++epoch, sums);
-    if (!ok || cg.updated(v[0], v[1], it, nom, beta)) break;
-#pragma unroll 4
-    for (int i = r0 + threadIdx.x; i < r1; i += TPBX) a.d[i] = fma(beta, a.d[i], a.h[i]);
+    const bool stop = !ok || cg.updated(v[0], v[1], it, nom, beta);
+    tiles_direction<TPBX>(a.x, a.d, a.h, alpha, beta, stop, r0, r1);
+    if (stop) break;
     ok = grid_barrier(a.gs, ++epoch, sums);
     if (!ok) break;
   }
@@ -735,26 +781,30 @@ __global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const T
 // The rule of the launch: the fewest lanes per unit whose stages (one per
 // warp at least) fit.  Fewer lanes mean wider tiles, fewer shuffles and more
 // gathers in flight per lane; the longest unit decides whether they fit
-// (8 lanes up to 43 blocks a row, 32 up to 166 of BSR3; 2 lanes up to 43
-// entries a row, 32 up to 700 of CSR).  BSR3 runs 16 warps of up to 128
-// registers, CSR, whose lanes hold less, 24.
+// (8 lanes up to 43 blocks a row, 32 up to 166 of BSR3; 2 lanes up to 66
+// entries a row, 8 up to 265, 32 up to 700 of CSR).  16 warps of up to 128
+// registers; the rows that 32 lanes share, in which every warp has only its
+// own row's gathers in flight, run 24 (60,000 rows of 401 entries 89.3 us an
+// iteration with 16 warps, 79.4 with 24).  With 24 warps throughout, whose
+// stages are shorter, 300,000 rows of 55 entries took 63.2 us (8 lanes)
+// against 50.7 (2 lanes), 100,000 of 201 entries 89.8 (32) against 69.7 (8).
 constexpr int kTileRing = 200 * 1024;    // stages
 constexpr int kTileSmem = 225 * 1024;    // with the unit pointers
-template <int ROWS>
-constexpr int kTileTPB = ROWS == 3 ? 512 : 768;
+template <int ROWS, int LPR>
+constexpr int kTileTPB = ROWS == 1 && LPR == 32 ? 768 : 512;
 
 template <int ROWS, int LPR>
 inline bool tiles_fit(const TileMat &m, int longest, int sms) {
   using K = TileKind<ROWS, LPR>;
   const int ent = (longest * K::kUnits + 3) & ~3, per = (m.units + sms - 1) / sms;
-  const int64_t stage = (int64_t)kTileTPB<ROWS> / 32 * (K::stage_bytes(ent) + 8);
+  const int64_t stage = (int64_t)kTileTPB<ROWS, LPR> / 32 * (K::stage_bytes(ent) + 8);
   return longest > 0 && longest < 4096 && stage <= kTileRing && stage + 4ll * (per + 1) <= kTileSmem;
 }
 
 template <int ROWS, int LPR>
 inline cudaError_t launch_tiles_as(const TileArgs &a, TileMat m, int longest, int sms, cudaStream_t s) {
   using K = TileKind<ROWS, LPR>;
-  constexpr int TPBX = kTileTPB<ROWS>, W = TPBX / 32;
+  constexpr int TPBX = kTileTPB<ROWS, LPR>, W = TPBX / 32;
   m.ent = (longest * K::kUnits + 3) & ~3;
   m.per = (m.units + sms - 1) / sms;
   const int grid = (m.units + m.per - 1) / m.per;  // no CTA without units

@@ -139,7 +139,9 @@ SYSTEMS = {
     "csr_2": (lambda: banded(200003, [1, 7, 300], 2), (0, 2)),
     "csr_2_uneven": (lambda: banded(160001, [1, 7, 300, 9000], 2, True), (0, 2)),
     "csr_8": (lambda: banded(40000, range(1, 41), 3), (0, 8)),
-    "csr_32": (lambda: banded(15001, range(1, 101), 4), (0, 32)),
+    "csr_32": (lambda: banded(15001, range(1, 101), 4), (0, 8)),  # 201 entries a row: 8 lanes take up to 265
+    "csr_32_long": (lambda: banded(15001, range(1, 151), 4), (0, 32)),
+    "csr_2_long": (lambda: banded(90001, range(1, 33), 5), (0, 2)),  # 65 entries, one below the line
     "general": (lambda: arrow(200003, 5000, 5), (0, None)),
     "bsr_8": (lambda: blocked(60001, [1, 7, 300], 6), (3, 8)),
     "bsr_16": (lambda: blocked(6001, range(1, 26), 7), (3, 16)),
