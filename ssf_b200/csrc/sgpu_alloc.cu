@@ -15,8 +15,9 @@
 // library start from that, so a reused block is cleared (and the clear
 // finished) before it is handed out: on a stream of the cache's own, so that
 // what else the device does is not waited for, and for a handle's small blocks
-// when the handle ends.  Solving a 10,000-equation system on a new handle
-// (38 blocks) paid 0.5 of its 2.3 ms for clears and waits of the device.
+// when the handle ends.  Solving a system of 1,500 equations on a new handle
+// (38 blocks) took 2.36 ms with a clear and two waits of the device for each,
+// 1.97 without.
 #include <map>
 #include <mutex>
 

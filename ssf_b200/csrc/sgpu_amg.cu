@@ -625,23 +625,47 @@ __global__ void __launch_bounds__(TPB) k_lv_bsr3_tma(int nb, int cap_blocks, con
   op_reduce<Op>(op, acc, st, partials, ticket);
 }
 
-// level 0 in scalar CSR: L lanes per row
+// level 0 in scalar CSR: L lanes per row.  FP64 has the gathers of U entries a
+// lane in flight and 4 lanes on short rows (2.69M rows of 18 entries 137 ->
+// 100 us, of which the bytes take 85); FP32, whose 4 lanes read half a sector
+// a step, keeps the other half in L1 (118 -> 104 us, bytes 57; 5 entries in
+// flight took 128).  Both read a row's bounds one row ahead.  A warp's entries
+// as one run through shared memory took 156 (FP32) and 244 us (FP64).
 template <typename T, int L, class Op>
 __global__ void __launch_bounds__(TPB) k_lv_csr(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
                                                 const T *__restrict__ val, const T *__restrict__ v, Op op,
                                                 PcgState *st, double *partials, unsigned *ticket) {
   if (st->done) return;
-  constexpr int GPW = 32 / L;
+  constexpr int GPW = 32 / L, U = L == 4 ? 5 : 4;
   const int lane = threadIdx.x & 31, g = lane / L, sub = lane % L;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   double acc[Op::NV > 0 ? Op::NV : 1] = {};
+  int b_next = 0, e_next = 0;  // a row's bounds are on their way while the row before is multiplied
+  if (warp * GPW + g < n) b_next = __ldg(rowptr + warp * GPW + g), e_next = __ldg(rowptr + warp * GPW + g + 1);
   for (int base = warp * GPW; base < n; base += nwarps * GPW) {
-    const int i = base + g;
-    int b = 0, e = 0;
-    if (i < n) { b = __ldg(rowptr + i); e = __ldg(rowptr + i + 1); }
+    const int i = base + g, b = b_next, e = e_next;
+    b_next = e_next = 0;
+    if (i + nwarps * GPW < n) b_next = __ldg(rowptr + i + nwarps * GPW), e_next = __ldg(rowptr + i + nwarps * GPW + 1);
     T s = 0;
-    for (int k = b + sub; k < e; k += L) s += __ldcs(val + k) * __ldg(v + __ldcs(col + k));
+    if constexpr (sizeof(T) == 4) {
+      for (int k = b + sub; k < e; k += L) s += __ldg(val + k) * __ldg(v + __ldg(col + k));
+    } else {
+      for (int k = b + sub; k < e; k += L * U) {
+        int c[U];
+        T w[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (k + L * u < e) c[u] = __ldcs(col + k + L * u), w[u] = __ldcs(val + k + L * u);
+        T x[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (k + L * u < e) x[u] = __ldg(v + c[u]);
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (k + L * u < e) s += w[u] * x[u];
+      }
+    }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, L);
     if (sub == 0 && i < n) op.row(i, s, acc);
@@ -671,23 +695,30 @@ __device__ __forceinline__ void load_block(const T *__restrict__ a, T (&v)[B * B
   }
 }
 
-// coarse levels: B x B blocks stored row-major, one warp per block row
-template <typename T, int B, class Op>
+// coarse levels: B x B blocks stored row-major, LPR lanes per block row
+// (launch_bsrb)
+template <typename T, int B, class Op, int LPR = 32>
 __global__ void __launch_bounds__(TPB) k_lv_bsrb(int nb, const int *__restrict__ browptr,
                                                  const int *__restrict__ bcol, const T *__restrict__ bval,
                                                  const T *__restrict__ v, Op op, PcgState *st, double *partials,
                                                  unsigned *ticket) {
   if (st->done) return;
-  const int lane = threadIdx.x & 31;
+  constexpr int RPW = 32 / LPR;
+  const int lane = threadIdx.x & 31, g = lane / LPR, sub = lane % LPR;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   double acc[Op::NV > 0 ? Op::NV : 1] = {};
-  for (int br = warp; br < nb; br += nwarps) {
-    const int s = __ldg(browptr + br), e = __ldg(browptr + br + 1);
+  int s_next = 0, e_next = 0;
+  if (warp * RPW + g < nb) s_next = __ldg(browptr + warp * RPW + g), e_next = __ldg(browptr + warp * RPW + g + 1);
+  for (int base = warp * RPW; base < nb; base += nwarps * RPW) {
+    const int br = base + g, s = s_next, e = e_next;
+    s_next = e_next = 0;
+    if (br + nwarps * RPW < nb)
+      s_next = __ldg(browptr + br + nwarps * RPW), e_next = __ldg(browptr + br + nwarps * RPW + 1);
     T y[B];
 #pragma unroll
     for (int c = 0; c < B; c++) y[c] = 0;
-    for (int k = s + lane; k < e; k += 32) {
+    for (int k = s + sub; k < e; k += LPR) {
       const int c = __ldg(bcol + k);
       T a[B * B];
       load_block<T, B>(bval + (size_t)k * B * B, a);
@@ -700,8 +731,8 @@ __global__ void __launch_bounds__(TPB) k_lv_bsrb(int nb, const int *__restrict__
         for (int q = 0; q < B; q++) y[r] += a[r * B + q] * xv[q];
       }
     }
-    const T yv = RowSums<B, 32>::sum(y, lane);
-    if (RowSums<B, 32>::first(lane)) op.row(B * br + RowSums<B, 32>::row_of_lane(lane), yv, acc);
+    const T yv = RowSums<B, LPR>::sum(y, sub);
+    if (RowSums<B, LPR>::first(sub) && br < nb) op.row(B * br + RowSums<B, LPR>::row_of_lane(sub), yv, acc);
   }
   op_reduce<Op>(op, acc, st, partials, ticket);
 }
@@ -1079,9 +1110,11 @@ __global__ void __launch_bounds__(TPB) k_fcg_init(int n, const double *__restric
     v[1] += ri * ri;
     const T bi = (T)(dscale[i] * ri);
     b0[i] = bi;
-    r0[i] = bi;
-    d0[i] = c2 * bi;
     x0[i] = c2 * bi;
+    if (r0) {  // a later smoothing step reads them
+      r0[i] = bi;
+      d0[i] = c2 * bi;
+    }
   }
   double t[2];
   if (reduce_grid<2>(v, partials, ticket, t)) {
@@ -1121,9 +1154,11 @@ __global__ void __launch_bounds__(TPB) k_fcg_update(int n, double *__restrict__ 
     v[0] += ri * ri;
     const T bi = (T)(dscale[i] * ri);
     b0[i] = bi;
-    r0[i] = bi;
-    d0[i] = c2 * bi;
     x0[i] = c2 * bi;
+    if (r0) {  // a later smoothing step reads them
+      r0[i] = bi;
+      d0[i] = c2 * bi;
+    }
   }
   double t[1];
   if (reduce_grid<1>(v, partials, ticket, t)) {
@@ -1335,9 +1370,11 @@ __global__ void __launch_bounds__(TPB) k_b_init_rows(int n, const double *__rest
     prr[i] = ri * ri;
     const T bi = (T)(dscale[i] * ri);
     b0[i] = bi;
-    r0[i] = bi;
-    d0[i] = c2 * bi;
     x0[i] = c2 * bi;
+    if (r0) {  // a later smoothing step reads them
+      r0[i] = bi;
+      d0[i] = c2 * bi;
+    }
   }
 }
 
@@ -1357,9 +1394,11 @@ __global__ void __launch_bounds__(TPB) k_b_update(int n, const int *__restrict__
     prr[i] = ri * ri;
     const T bi = (T)(dscale[i] * ri);
     b0[i] = bi;
-    r0[i] = bi;
-    d0[i] = c2 * bi;
     x0[i] = c2 * bi;
+    if (r0) {  // a later smoothing step reads them
+      r0[i] = bi;
+      d0[i] = c2 * bi;
+    }
   }
 }
 
@@ -3680,6 +3719,33 @@ int level0_lanes(const sgpu_matrix m, bool fp32) {
   return v;
 }
 
+// The largest level-1 matrix that a program takes.  A graph's kernels follow
+// one another about as fast as a grid barrier opens, so a program gains only
+// where the steps are short; a large level's steps run longer in one CTA per
+// SM than in the separate kernels' grids.  Measured whole solves: 129,480
+// equations (level 1 of 16 MB, FP64) 9.3 -> 8.9 ms; the 1.01M-equation
+// cantilever (57 MB) and 256 plates (41 MB) unchanged where only their deeper
+// levels ran as programs, slower (0.80 against 0.60 ms a cycle) with level 1.
+constexpr double kProgLevelBytes = 20e6;
+
+// A coarse level's product: a warp per block row, or 8 lanes where a row has
+// few blocks (plane problems: 9, which leave 23 lanes of a warp idle) and the
+// level is too large to be a step of a program, whose rows a warp sums.  256
+// plates (level 1 of 41 MB) 59.4 ms with a warp, 55.5 with 8 lanes.
+template <typename T, int B, class Op>
+void launch_bsrb(const AmgLevel &L, const T *val, const T *v, const Op &op, cudaStream_t s, PcgState *st, double *part,
+                 unsigned *tk) {
+  if constexpr (B <= 3) {
+    if (L.nblk <= (int64_t)12 * L.nb && (double)L.nblk * B * B * sizeof(T) > kProgLevelBytes) {
+      auto k = k_lv_bsrb<T, B, Op, 8>;
+      k<<<resident_grid(k, (L.nb + 3) / 4), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk);
+      return;
+    }
+  }
+  auto k = k_lv_bsrb<T, B, Op>;
+  k<<<resident_grid(k, L.nb), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk);
+}
+
 template <typename T, class Op>
 int launch_level(sgpu_matrix m, const AmgLevel &L, const T *v, const Op &op, cudaStream_t s, int slot) {
   PcgState *st = pcg_state(m);
@@ -3725,12 +3791,9 @@ int launch_level(sgpu_matrix m, const AmgLevel &L, const T *v, const Op &op, cud
   } else {
     if (record_level(m, L, v, op)) return SGPU_OK;
     switch (L.b) {
-      case 1: { auto k = k_lv_bsrb<T, 1, Op>;
-        k<<<resident_grid(k, L.nb), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk); break; }
-      case 3: { auto k = k_lv_bsrb<T, 3, Op>;
-        k<<<resident_grid(k, L.nb), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk); break; }
-      case 6: { auto k = k_lv_bsrb<T, 6, Op>;
-        k<<<resident_grid(k, L.nb), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk); break; }
+      case 1: launch_bsrb<T, 1>(L, val, v, op, s, st, part, tk); break;
+      case 3: launch_bsrb<T, 3>(L, val, v, op, s, st, part, tk); break;
+      case 6: launch_bsrb<T, 6>(L, val, v, op, s, st, part, tk); break;
       default:
         return fail(SGPU_BAD_INPUT, "unsupported coarse block size");
     }
@@ -4346,15 +4409,6 @@ constexpr int kProgMaxSteps = 1024;
 template <typename T>
 int cycle(sgpu_matrix m, int l, bool zero_init, const std::vector<Cheb> &ch, std::vector<T *> &xcur, cudaStream_t s);
 
-// The largest level-1 matrix that a program takes.  A graph's kernels follow
-// one another about as fast as a grid barrier opens, so a program gains only
-// where the steps are short; a large level's steps run longer in one CTA per
-// SM than in the separate kernels' grids.  Measured whole solves: 129,480
-// equations (level 1 of 16 MB, FP64) 9.3 -> 8.9 ms; the 1.01M-equation
-// cantilever (57 MB) and 256 plates (41 MB) unchanged where only their deeper
-// levels ran as programs, slower (0.80 against 0.60 ms a cycle) with level 1.
-constexpr double kProgLevelBytes = 20e6;
-
 // The `visits` of level l as a program (level 1 and all below it), recorded
 // from the cycle itself on the first cycle of a solve (never during a graph
 // capture) and kept for its others: the arrays and coefficients do not change
@@ -4527,6 +4581,15 @@ int vcycle_dir(sgpu_matrix m, cudaStream_t s) {
   return SGPU_OK;
 }
 
+// The smoothed residual that level 0's first step from zero leaves for later
+// steps, or null where it has none: one smoothing step, and another level or
+// the dense solve below (the bottom level smooths on).  Written without a
+// reader, it and the direction were an eighth of the update's traffic.
+template <typename T>
+T *first_r(const Amg &A, LevelVecs<T> &V) {
+  return A.deg > 1 || (A.lv.size() == 1 && A.nc == 0) ? V.r.p : nullptr;
+}
+
 template <typename T>
 int fcg_update(sgpu_matrix m, cudaStream_t s) {
   Amg &A = *m->amg;
@@ -4536,7 +4599,7 @@ int fcg_update(sgpu_matrix m, cudaStream_t s) {
   const double l0 = sizeof(T) == 4 ? L0.lmax32 : L0.lmax64;
   const T c2 = (T)cheb_coeffs(l0, A.ratio, A.deg).c2_first;
   k_fcg_update<T><<<grid_for(m->n), TPB, 0, s>>>((int)m->n, w.x.p, w.r.p, w.d.p, w.p.p, m->csr.dscale.p, V.b.p,
-                                                  V.r.p, V.d.p, V.x.p, c2, pcg_state(m), w.partials.p,
+                                                  first_r(A, V), V.d.p, V.x.p, c2, pcg_state(m), w.partials.p,
                                                   w.counters.p + 2);
   count_launches(1);
   return SGPU_OK;
@@ -4550,7 +4613,7 @@ int fcg_init(sgpu_matrix m, cudaStream_t s) {
   Work &w = m->w;
   const double l0 = sizeof(T) == 4 ? L0.lmax32 : L0.lmax64;
   const T c2 = (T)cheb_coeffs(l0, A.ratio, A.deg).c2_first;
-  k_fcg_init<T><<<grid_for(m->n), TPB, 0, s>>>((int)m->n, w.f.p, w.p.p, w.r.p, m->csr.dscale.p, V.b.p, V.r.p, V.d.p,
+  k_fcg_init<T><<<grid_for(m->n), TPB, 0, s>>>((int)m->n, w.f.p, w.p.p, w.r.p, m->csr.dscale.p, V.b.p, first_r(A, V), V.d.p,
                                                 V.x.p, c2, pcg_state(m), w.partials.p, w.counters.p + 2);
   count_launches(1);
   return SGPU_OK;
@@ -4751,9 +4814,14 @@ int batch_spmv64(sgpu_matrix m, const double *p, double *q, double *prod, cudaSt
     k<<<resident_grid(k, m->bsr.nb), TPB, 0, s>>>(m->bsr.nb, m->bsr.browptr.p, m->bsr.bcol.p, m->bsr.bval.p, p, op,
                                                   st, m->w.partials.p, m->w.counters.p);
   } else {
-    auto k = k_lv_csr<double, 8, OpStorePQ>;
-    k<<<resident_grid(k, (m->n + 3) / 4), TPB, 0, s>>>((int)m->n, m->csr.rowptr.p, m->csr.col.p, m->csr.val.p, p, op,
-                                                        st, m->w.partials.p, m->w.counters.p);
+    // 4 lanes on rows of up to 5 entries a lane, which all are in flight then
+    auto launch = [&](auto k, int rows) {
+      k<<<resident_grid(k, (m->n + rows - 1) / rows), TPB, 0, s>>>((int)m->n, m->csr.rowptr.p, m->csr.col.p,
+                                                                   m->csr.val.p, p, op, st, m->w.partials.p,
+                                                                   m->w.counters.p);
+    };
+    if (m->csr.nnz <= (int64_t)20 * m->n) launch(k_lv_csr<double, 4, OpStorePQ>, 8);
+    else launch(k_lv_csr<double, 8, OpStorePQ>, 4);
   }
   count_launches(1);
   SGPU_CUDA(cudaGetLastError());
@@ -4779,7 +4847,7 @@ int batch_solve(sgpu_matrix m, int nsys, const long long *sysptr, const int *row
   SGPU_CUDA(cudaMemsetAsync(w.x.p, 0, (size_t)n * sizeof(double), s));
   SGPU_CUDA(cudaMemsetAsync(w.p.p, 0, (size_t)n * sizeof(double), s));
   SGPU_CUDA(cudaMemsetAsync(w.d.p, 0, (size_t)n * sizeof(double), s));
-  k_b_init_rows<T><<<g, TPB, 0, s>>>(n, w.f.p, w.p.p, w.r.p, m->csr.dscale.p, V.b.p, V.r.p, V.d.p, V.x.p, c2, pff,
+  k_b_init_rows<T><<<g, TPB, 0, s>>>(n, w.f.p, w.p.p, w.r.p, m->csr.dscale.p, V.b.p, first_r(A, V), V.d.p, V.x.p, c2, pff,
                                      prr);
   k_bseg_init<<<gs, kSegTPB, 0, s>>>(nsys, sysptr, pff, prr, sys, res);
   k_bcount<<<1, TPB, 0, s>>>(nsys, sys, pcg_state(m));
@@ -4792,7 +4860,7 @@ int batch_solve(sgpu_matrix m, int nsys, const long long *sysptr, const int *row
   SGPU_TRY(iters.run(s, A.side, &pcg_state(m)->done, ni + 8, [&]() -> int {
     SGPU_TRY(batch_spmv64(m, w.d.p, w.p.p, ppq, s));
     k_bseg_alpha<<<gs, kSegTPB, 0, s>>>(nsys, sysptr, ppq, sys);
-    k_b_update<T><<<g, TPB, 0, s>>>(n, rowsys, sys, w.x.p, w.r.p, w.d.p, w.p.p, m->csr.dscale.p, V.b.p, V.r.p, V.d.p,
+    k_b_update<T><<<g, TPB, 0, s>>>(n, rowsys, sys, w.x.p, w.r.p, w.d.p, w.p.p, m->csr.dscale.p, V.b.p, first_r(A, V), V.d.p,
                                     V.x.p, c2, prr, pcg_state(m));
     k_bseg_rr<<<gs, kSegTPB, 0, s>>>(nsys, sysptr, prr, sys, (long long)ni, res);
     k_bcount<<<1, TPB, 0, s>>>(nsys, sys, pcg_state(m));

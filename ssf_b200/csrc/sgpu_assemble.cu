@@ -2176,7 +2176,7 @@ struct AssemblyData {
   bool node_rows = false;
 };
 
-// The colouring (3 ms for 330,000 elements, one after the other by its
+// The colouring (3 ms for 320,000 elements, one after the other by its
 // definition) in a thread of its own beside the copies and the pattern's
 // construction; joined before its lists are read and on every way out.
 struct Colouring {

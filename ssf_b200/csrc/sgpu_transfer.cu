@@ -4,7 +4,8 @@
 // driver, filled by the calling thread: 11 GB/s on B200's host, a fifth of
 // what the link takes from pinned memory.  Large arrays go through pinned
 // slots of our own, which a few threads fill (or empty) while the slots
-// before are on the link.
+// before are on the link: 28 GB/s (78 MB of a matrix's storage 7.1 -> 2.8 ms).
+// Pinning the 8 MB takes 3.7 ms, once in a process.
 //
 // The slots belong to the process, one set per device, and are given back
 // when it ends; a thread that finds them in use copies the plain way.
