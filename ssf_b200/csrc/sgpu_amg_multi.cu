@@ -311,11 +311,13 @@ struct Staged<double> {
 // the row before is multiplied, and pass through shared memory, from where
 // every lane takes a block in 3 (FP64: 5) 16-byte words instead of 10 loads.
 // 132,300 equations, 64 columns: FP32 139 -> 105 us, FP64 202 -> 159 us.
+// FP32 up to 64 columns has three blocks in flight and four CTAs a SM (a whole
+// solve of 64 load cases 33.5 -> 32.6 ms against two blocks and no bound; four
+// blocks 34.0, two with five CTAs 37.8).  FP64 would spill under that bound.
 template <typename T, int CPL, class Op>
-__global__ void __launch_bounds__(TPB) k_mspmm_bsr3(int nb, const int *__restrict__ browptr,
-                                                    const int *__restrict__ bcol, const T *__restrict__ bval,
-                                                    const T *__restrict__ X, Op op, MCol *cols, int R, MState *ms,
-                                                    double *partials, unsigned *ticket) {
+__global__ void __launch_bounds__(TPB, sizeof(T) == 4 && CPL <= 2 ? 4 : 1)
+    k_mspmm_bsr3(int nb, const int *__restrict__ browptr, const int *__restrict__ bcol, const T *__restrict__ bval,
+                 const T *__restrict__ X, Op op, MCol *cols, int R, MState *ms, double *partials, unsigned *ticket) {
   if (ms->all_done) return;
   constexpr int RP = 32 * CPL;
   constexpr int NVX = Op::NV > 0 ? Op::NV : 1;
@@ -350,7 +352,7 @@ __global__ void __launch_bounds__(TPB) k_mspmm_bsr3(int nb, const int *__restric
       if (br < nb) s = __ldg(browptr + br), nbr = __ldg(browptr + br + 1) - s;
     }
     fetch();
-#pragma unroll 2
+#pragma unroll (sizeof(T) == 4 && CPL <= 2 ? 3 : 2)
     for (int j = 0; j < cnt; j++) {
       T a[9];
       const T *x0 = X + (size_t)(3 * stage[wid][j].get(a)) * RP + lane;
