@@ -108,7 +108,8 @@ void pieces(Stage &st, Job &j, int t) {
 cudaError_t copy(void *dst, const void *src, size_t bytes, cudaStream_t s, bool in) {
   const cudaMemcpyKind kind = in ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
   int dev = 0;
-  if (bytes < kLeast || cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices || !pageable(in ? src : dst))
+  // the per-thread default stream is another stream in each of the copying threads
+  if (bytes < kLeast || s == cudaStreamPerThread || cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices || !pageable(in ? src : dst))
     return cudaMemcpyAsync(dst, src, bytes, kind, s);
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)

@@ -1,0 +1,61 @@
+"""The library's host code against a stand-in for the CUDA runtime (fake_cudart.cpp): which thread issues a copy on
+which stream, and what a call that fails leads to.  No device is needed."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+SOURCES = ["sgpu_transfer.cu", "sgpu_alloc.cu", "sgpu_capi.cu"]
+LARGE = 5 * (4 << 20) // 8 + 7  # values: several rounds of every copying thread
+PER_THREAD = 2                  # cudaStreamPerThread
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    """The host sources and the stand-in as one library; what they call in files of kernels returns 0 at once."""
+    d = tmp_path_factory.mktemp("host")
+    objs = []
+    for src in [os.path.join(ROOT, "ssf_b200", "csrc", s) for s in SOURCES] + [os.path.join(HERE, "fake_cudart.cpp")]:
+        objs.append(str(d / (os.path.basename(src) + ".o")))
+        subprocess.run(["g++", "-x", "c++", "-std=c++17", "-O1", "-fPIC", "-I", os.path.join(CUDA, "include"), "-c", src,
+                        "-o", objs[-1]], check=True)
+    names = subprocess.run(["nm", "-g", *objs], check=True, capture_output=True, text=True).stdout.split("\n")
+    names = [line.split()[-2:] for line in names if len(line.split()) >= 2 and not line.endswith(":")]
+    defined = {n for kind, n in names if kind != "U"}
+    missing = sorted({n for kind, n in names if kind == "U" and "sgpu" in n} - defined)
+    stubs = d / "stubs.s"
+    stubs.write_text(".text\n" + "".join(f".globl {n}\n{n}:\n" for n in missing) + "xorl %eax, %eax\nret\n"
+                     ".section .note.GNU-stack,\"\",@progbits\n")
+    out = str(d / "libhost.so")
+    subprocess.run(["g++", "-shared", "-o", out, *objs, str(stubs), "-lpthread"], check=True)
+    lib = C.CDLL(out)
+    yield lib
+
+
+@pytest.fixture
+def copies(host):
+    """copy_in and copy_out, as (destination, source, bytes, stream) -> error"""
+    host.fake_reset()
+    out = []
+    for name in ("_ZN4sgpu7copy_inEPvPKvmP11CUstream_st", "_ZN4sgpu8copy_outEPvPKvmP11CUstream_st"):
+        fn = getattr(host, name)
+        fn.argtypes, fn.restype = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p], C.c_int
+        out.append(fn)
+    yield out
+    host.fake_reset()
+
+
+@pytest.mark.parametrize("stream", [PER_THREAD, 0x1000])
+@pytest.mark.parametrize("n", [1, (4 << 20) // 8, LARGE])
+def test_every_piece_lands_on_the_callers_stream(host, copies, stream, n):
+    """The per-thread default stream is another stream in another thread: only the caller may copy on it."""
+    for fn in copies:
+        src, dst = np.random.default_rng(n).standard_normal(n), np.zeros(n)
+        assert fn(dst.ctypes.data, src.ctypes.data, 8 * n, stream) == 0
+        assert np.array_equal(dst, src)
+    assert stream != PER_THREAD or host.fake_foreign_copies(C.c_void_p(stream)) == 0
