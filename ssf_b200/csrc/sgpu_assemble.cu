@@ -2495,8 +2495,10 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   BAIL_ON(examine_codes(cn_d.p, ncode, ndofn, code.p, err.p, &nfree, &flags, s));
   const bool monotone = !(flags & 32u);
   int64_t n = nfree;
-  if (!monotone)  // number of equations = largest code number
+  if (!monotone) {  // the largest code number: fewer than the positive ones where nodes share equations
+    n = 0;
     for (int64_t q = 0; q < ncode; q++) n = std::max<int64_t>(n, mesh->cn[q]);
+  }
   if (n <= 0) return bail(fail(SGPU_BAD_INPUT, "no free equations"));
   if (flags & 1u) return bail(fail(SGPU_BAD_INPUT, "element node out of range"));
   if (n >= (1LL << 31) - 1) return bail(fail(SGPU_BAD_INPUT, "n out of range for int32 device indices"));
