@@ -384,12 +384,28 @@ __device__ __forceinline__ void hex_gauss_point(int lane, const double *x, const
   }
 }
 
+// Where element kernels report, and whether nodes share equations.  Elements
+// of a launch share no node and the lanes of an element have (node, component)
+// pairs of their own, so plain additions do; where nodes share equations
+// (tied), both meet again, and the additions are atomic.
+struct Report {
+  unsigned *err;
+  int tied;
+  __device__ operator unsigned *() const { return err; }
+};
+
 // add v into CSR entry (r, c); both >= 0
 __device__ __forceinline__ void csr_add(const int *__restrict__ rowptr, const int *__restrict__ col,
-                                        double *__restrict__ val, int r, int c, double v, unsigned *err) {
+                                        double *__restrict__ val, int r, int c, double v, Report err) {
   const int p = find_col(col, __ldg(rowptr + r), __ldg(rowptr + r + 1), c);
-  if (p >= 0) val[p] += v;
-  else atomicOr(err, 4u);
+  if (p < 0) atomicOr(err, 4u);
+  else if (err.tied) atomicAdd(val + p, v);
+  else val[p] += v;
+}
+
+__device__ __forceinline__ void rhs_sub(double *rhs, double v, int tied) {
+  if (tied) atomicAdd(rhs, -v);
+  else *rhs -= v;
 }
 
 // adds the 3 x 3 block k at rows r[0..2], columns c[0..2] (< 0: no
@@ -399,8 +415,9 @@ __device__ __forceinline__ void csr_add(const int *__restrict__ rowptr, const in
 // offsets -- each checked before it is used; otherwise nine searches.
 __device__ __forceinline__ void block3_add(const int *__restrict__ rowptr, const int *__restrict__ col,
                                            double *__restrict__ val, const int r[3], const int c[3],
-                                           const double k[3][3], unsigned *err) {
-  if (r[0] >= 0 && r[1] == r[0] + 1 && r[2] == r[0] + 2 && c[0] >= 0 && c[1] == c[0] + 1 && c[2] == c[0] + 2) {
+                                           const double k[3][3], Report err) {
+  if (!err.tied && r[0] >= 0 && r[1] == r[0] + 1 && r[2] == r[0] + 2 && c[0] >= 0 && c[1] == c[0] + 1 &&
+      c[2] == c[0] + 2) {
     const int b0 = __ldg(rowptr + r[0]), e0 = __ldg(rowptr + r[0] + 1);
     const int p = find_col(col, b0, e0, c[0]);
     if (p >= 0 && p + 2 < e0) {
@@ -442,7 +459,7 @@ __global__ void __launch_bounds__(TPB) k_hex8_elastic(int ne_c, const int *__res
                                                       const int64_t *__restrict__ elems,
                                                       const int *__restrict__ cne, const double *__restrict__ emat,
                                                       const int *__restrict__ rowptr, const int *__restrict__ col,
-                                                      double *__restrict__ val, unsigned *err) {
+                                                      double *__restrict__ val, Report err) {
   __shared__ HexShared shm[WPB];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   HexShared &sh = shm[wib];
@@ -582,7 +599,7 @@ __device__ __forceinline__ int find_in_shared(const int *cols, int len, int c) {
 template <bool ROWCACHE>
 __device__ __forceinline__ void iso_scatter(const HexIsoShared &sh, int A, const int rr[3], const int cc[3],
                                             const double k[3][3], const int *__restrict__ rowptr,
-                                            const int *__restrict__ col, double *__restrict__ val, unsigned *err) {
+                                            const int *__restrict__ col, double *__restrict__ val, Report err) {
   if (ROWCACHE) {
     const int len = sh.rl[A];
     if (len > 0 && cc[0] >= 0 && cc[1] == cc[0] + 1 && cc[2] == cc[0] + 2) {
@@ -639,7 +656,7 @@ __global__ void __launch_bounds__(TPB, 3) k_hex8_iso(int ne_c, const int *__rest
                                                      const int64_t *__restrict__ elems,
                                                      const int *__restrict__ cne, const double *__restrict__ emat,
                                                      const int *__restrict__ rowptr, const int *__restrict__ col,
-                                                     double *__restrict__ val, unsigned *err,
+                                                     double *__restrict__ val, Report err,
                                                      double *__restrict__ kbuf) {
   __shared__ HexIsoShared shm[WPB];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1189,7 +1206,7 @@ __global__ void __launch_bounds__(TPB) k_tet4_elastic(int ne_c, const int *__res
                                                       const int64_t *__restrict__ elems,
                                                       const int *__restrict__ cne, const double *__restrict__ emat,
                                                       const int *__restrict__ rowptr, const int *__restrict__ col,
-                                                      double *__restrict__ val, unsigned *err) {
+                                                      double *__restrict__ val, Report err) {
   const int lane = threadIdx.x & 31, half = lane >> 4, hl = lane & 15;
   const int warp = (int)((blockIdx.x * (unsigned)TPB + threadIdx.x) >> 5);
   const int nwarps = gridDim.x * WPB;
@@ -1292,7 +1309,7 @@ __global__ void __launch_bounds__(TPB) k_quad4_elastic(int ne_c, const int *__re
                                                        const int *__restrict__ cne, const double *__restrict__ emat,
                                                        const double *__restrict__ thick,
                                                        const int *__restrict__ rowptr, const int *__restrict__ col,
-                                                       double *__restrict__ val, unsigned *err) {
+                                                       double *__restrict__ val, Report err) {
   __shared__ QuadShared shm[WPB];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   QuadShared &sh = shm[wib];
@@ -1434,7 +1451,7 @@ __global__ void __launch_bounds__(TPB20) k_hex20_elastic(int ne_c, const int *__
                                                          const int64_t *__restrict__ elems,
                                                          const int *__restrict__ cne, const double *__restrict__ emat,
                                                          const int *__restrict__ rowptr, const int *__restrict__ col,
-                                                         double *__restrict__ val, unsigned *err) {
+                                                         double *__restrict__ val, Report err) {
   extern __shared__ double smem20[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   Hex20Shared &sh = reinterpret_cast<Hex20Shared *>(smem20)[wib];
@@ -1544,7 +1561,7 @@ __global__ void __launch_bounds__(TPB) k_quad8_elastic(int ne_c, const int *__re
                                                        const int *__restrict__ cne, const double *__restrict__ emat,
                                                        const double *__restrict__ thick,
                                                        const int *__restrict__ rowptr, const int *__restrict__ col,
-                                                       double *__restrict__ val, unsigned *err) {
+                                                       double *__restrict__ val, Report err) {
   __shared__ Quad8Shared shm[WPB];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   Quad8Shared &sh = shm[wib];
@@ -1645,7 +1662,7 @@ __global__ void __launch_bounds__(TPB) k_tri3_elastic(int ne_c, const int *__res
                                                       const int *__restrict__ cne, const double *__restrict__ emat,
                                                       const double *__restrict__ thick,
                                                       const int *__restrict__ rowptr, const int *__restrict__ col,
-                                                      double *__restrict__ val, unsigned *err) {
+                                                      double *__restrict__ val, Report err) {
   for (int t = blockIdx.x * TPB + threadIdx.x; t < ne_c; t += gridDim.x * TPB) {
     const int e = elist[t];
     double x[3], y[3];
@@ -1700,7 +1717,7 @@ __global__ void __launch_bounds__(TPB) k_hex8_scalar(int ne_c, const int *__rest
                                                      const int *__restrict__ cne, const double *__restrict__ emat,
                                                      const double *__restrict__ rho,
                                                      const int *__restrict__ rowptr, const int *__restrict__ col,
-                                                     double *__restrict__ val, unsigned *err) {
+                                                     double *__restrict__ val, Report err) {
   __shared__ HexShared shm[WPB];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   HexShared &sh = shm[wib];
@@ -1755,7 +1772,8 @@ __global__ void __launch_bounds__(TPB) k_hex8t_lift(int ne_c, const int *__restr
                                                     const double *__restrict__ coords,
                                                     const int64_t *__restrict__ elems,
                                                     const int *__restrict__ cne, const double *__restrict__ emat,
-                                                    const double *__restrict__ rnode, double *__restrict__ rhs) {
+                                                    const double *__restrict__ rnode, double *__restrict__ rhs,
+                                                    int tied) {
   __shared__ HexShared shm[WPB];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   HexShared &sh = shm[wib];
@@ -1793,7 +1811,7 @@ __global__ void __launch_bounds__(TPB) k_hex8t_lift(int ne_c, const int *__restr
         f += kab * r[b];
       }
       const int row = __ldg(cne + (int64_t)e * 8 + a);
-      if (row >= 0) rhs[row] -= f;
+      if (row >= 0) rhs_sub(rhs + row, f, tied);
     }
     __syncwarp();
   }
@@ -1812,7 +1830,7 @@ __global__ void __launch_bounds__(TPB) k_hex8_lift(int ne_c, const int *__restri
                                                    const double *__restrict__ coords,
                                                    const int64_t *__restrict__ elems, const int *__restrict__ cne,
                                                    const double *__restrict__ emat, const double *__restrict__ rnode,
-                                                   double *__restrict__ rhs) {
+                                                   double *__restrict__ rhs, int tied) {
   __shared__ HexShared shm[WPB];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   HexShared &sh = shm[wib];
@@ -1894,7 +1912,7 @@ __global__ void __launch_bounds__(TPB) k_hex8_lift(int ne_c, const int *__restri
 #pragma unroll
         for (int i = 0; i < 3; i++) {
           const int row = __ldg(cne + (int64_t)e * 24 + 3 * a + i);
-          if (row >= 0) rhs[row] -= f[h][i];
+          if (row >= 0) rhs_sub(rhs + row, f[h][i], tied);
         }
       }
     }
@@ -1908,7 +1926,8 @@ __global__ void __launch_bounds__(TPB) k_quad4_lift(int ne_c, const int *__restr
                                                     const double *__restrict__ coords,
                                                     const int64_t *__restrict__ elems, const int *__restrict__ cne,
                                                     const double *__restrict__ emat, const double *__restrict__ thick,
-                                                    const double *__restrict__ rnode, double *__restrict__ rhs) {
+                                                    const double *__restrict__ rnode, double *__restrict__ rhs,
+                                                    int tied) {
   __shared__ QuadShared shm[WPB];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   QuadShared &sh = shm[wib];
@@ -1979,8 +1998,8 @@ __global__ void __launch_bounds__(TPB) k_quad4_lift(int ne_c, const int *__restr
     if (lane < 16 && (lane & 3) == 0) {
       const int a = lane >> 2;
       const int row0 = __ldg(cne + (int64_t)e * 8 + 2 * a), row1 = __ldg(cne + (int64_t)e * 8 + 2 * a + 1);
-      if (row0 >= 0) rhs[row0] -= f0;
-      if (row1 >= 0) rhs[row1] -= f1;
+      if (row0 >= 0) rhs_sub(rhs + row0, f0, tied);
+      if (row1 >= 0) rhs_sub(rhs + row1, f1, tied);
     }
     __syncwarp();
   }
@@ -2174,6 +2193,7 @@ struct AssemblyData {
   // precondition
   DevBuf<int> iptr, inc;
   bool node_rows = false;
+  bool tied = false;  // several (node, component) pairs have one equation
 };
 
 // The colouring (3 ms for 320,000 elements, one after the other by its
@@ -2236,6 +2256,7 @@ int assemble_values(sgpu_matrix m, AssemblyData &ad, int kind, float *ms_out) {
   DevBuf<unsigned> err;
   SGPU_TRY(err.alloc(1));
   SGPU_CUDA(cudaMemsetAsync(err.p, 0, sizeof(unsigned), s));
+  const Report report = {err.p, ad.tied ? 1 : 0};
   SGPU_CUDA(cudaEventRecord(m->ev0, s));
   // isotropic hex8 elasticity on gencodnum's numbering, SGPU_ASSEMBLY_ROWS=1:
   // rows formed per node and written once.  Not the default: on the 1.01M-DOF
@@ -2270,7 +2291,7 @@ int assemble_values(sgpu_matrix m, AssemblyData &ad, int kind, float *ms_out) {
     SGPU_CUDA(cudaMemsetAsync(c.val.p, 0, (size_t)c.nnz * sizeof(double), s));
     const int g1 = (int)std::min<int64_t>((ad.ne + WPB - 1) / WPB, (int64_t)kNumSMs * 16);
     k_hex8_iso<false, true><<<g1, TPB, 0, s>>>((int)ad.ne, nullptr, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p,
-                                                c.rowptr.p, c.col.p, c.val.p, err.p, kbuf.p);
+                                                c.rowptr.p, c.col.p, c.val.p, report, kbuf.p);
     const int g2 = (int)std::min<int64_t>((ad.nn + kRowWarps - 1) / kRowWarps, (int64_t)kNumSMs * 64);
     k_hex8_gather<<<g2, kRowWarps * 32, 0, s>>>(ad.nn, ad.iptr.p, ad.inc.p, ad.elems.p, ad.cne.p, kbuf.p,
                                                 c.rowptr.p, c.col.p, c.val.p, err.p);
@@ -2312,29 +2333,29 @@ int assemble_values(sgpu_matrix m, AssemblyData &ad, int kind, float *ms_out) {
       case 0:
         if (ad.general)
           k_hex8_elastic<true><<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p,
-                                                    c.rowptr.p, c.col.p, c.val.p, err.p);
+                                                    c.rowptr.p, c.col.p, c.val.p, report);
         else if (hex8_full_product())
           k_hex8_elastic<false><<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p,
-                                                     c.rowptr.p, c.col.p, c.val.p, err.p);
-        else if (hex8_row_cache())
+                                                     c.rowptr.p, c.col.p, c.val.p, report);
+        else if (hex8_row_cache() && !ad.tied)  // a shared equation's row has more columns than its node's others
           k_hex8_iso<true, false><<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p,
-                                                       c.rowptr.p, c.col.p, c.val.p, err.p, nullptr);
+                                                       c.rowptr.p, c.col.p, c.val.p, report, nullptr);
         else
           k_hex8_iso<false, false><<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p,
-                                                        c.rowptr.p, c.col.p, c.val.p, err.p, nullptr);
+                                                        c.rowptr.p, c.col.p, c.val.p, report, nullptr);
         break;
       case 1:
         k_quad4_elastic<<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, ad.thick.p,
-                                             c.rowptr.p, c.col.p, c.val.p, err.p);
+                                             c.rowptr.p, c.col.p, c.val.p, report);
         break;
       case 4: {
         const int g4 = std::min((cnt + 2 * WPB - 1) / (2 * WPB), kNumSMs * 16);
         if (ad.general)
           k_tet4_elastic<true><<<g4, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p,
-                                                  c.rowptr.p, c.col.p, c.val.p, err.p);
+                                                  c.rowptr.p, c.col.p, c.val.p, report);
         else
           k_tet4_elastic<false><<<g4, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p,
-                                                   c.rowptr.p, c.col.p, c.val.p, err.p);
+                                                   c.rowptr.p, c.col.p, c.val.p, report);
         break;
       }
       case 6: {
@@ -2343,32 +2364,32 @@ int assemble_values(sgpu_matrix m, AssemblyData &ad, int kind, float *ms_out) {
         if (ad.general) {
           SGPU_CUDA(cudaFuncSetAttribute(k_hex20_elastic<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
           k_hex20_elastic<true><<<g6, TPB20, sm, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p,
-                                                      c.rowptr.p, c.col.p, c.val.p, err.p);
+                                                      c.rowptr.p, c.col.p, c.val.p, report);
         } else {
           SGPU_CUDA(cudaFuncSetAttribute(k_hex20_elastic<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
           k_hex20_elastic<false><<<g6, TPB20, sm, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p,
-                                                       c.rowptr.p, c.col.p, c.val.p, err.p);
+                                                       c.rowptr.p, c.col.p, c.val.p, report);
         }
         break;
       }
       case 7:
         k_quad8_elastic<<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, ad.thick.p,
-                                             c.rowptr.p, c.col.p, c.val.p, err.p);
+                                             c.rowptr.p, c.col.p, c.val.p, report);
         break;
       case 5: {
         const int g5 = std::min((cnt + TPB - 1) / TPB, kNumSMs * 16);
         k_tri3_elastic<<<g5, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, ad.thick.p,
-                                          c.rowptr.p, c.col.p, c.val.p, err.p);
+                                          c.rowptr.p, c.col.p, c.val.p, report);
         break;
       }
       case 2:
         k_hex8_scalar<false><<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, nullptr,
-                                                  c.rowptr.p, c.col.p, c.val.p, err.p);
+                                                  c.rowptr.p, c.col.p, c.val.p, report);
         break;
       default:
         k_hex8_scalar<true><<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p,
                                                  ad.rho.p ? ad.rho.p : nullptr, c.rowptr.p, c.col.p, c.val.p,
-                                                 err.p);
+                                                 report);
         break;
     }
     count_launches(1);
@@ -2503,6 +2524,7 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   if (flags & 1u) return bail(fail(SGPU_BAD_INPUT, "element node out of range"));
   if (n >= (1LL << 31) - 1) return bail(fail(SGPU_BAD_INPUT, "n out of range for int32 device indices"));
   m->n = n;
+  ad.tied = n < nfree;
   cudaMemsetAsync(err.p, 0, sizeof(unsigned), s);
 
   // pattern: from the node adjacency when the code numbers are gencodnum's,
@@ -2604,20 +2626,21 @@ SGPU_API int sgpu_assembly_lift(sgpu_matrix m, const double *rnode, double *rhs)
   SGPU_TRY(f.alloc(m->n));
   SGPU_CUDA(copy_in(rn.p, rnode, nr * sizeof(double), s));
   SGPU_CUDA(copy_in(f.p, rhs, m->n * sizeof(double), s));
-  const int ncol = (int)ad.offsets.size() - 1;
+  const int ncol = (int)ad.offsets.size() - 1, tied = ad.tied ? 1 : 0;
   for (int col = 0; col < ncol; col++) {
     const int beg = ad.offsets[col], cnt = ad.offsets[col + 1] - beg;
     if (cnt == 0) continue;
     const int grid = std::min((cnt + WPB - 1) / WPB, kNumSMs * 16);
     const int *el = ad.elist.p + beg;
     if (scalar)
-      k_hex8t_lift<<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, rn.p, f.p);
+      k_hex8t_lift<<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, rn.p, f.p, tied);
     else if (ad.kind == SGPU_ELEM_QUAD4)
-      k_quad4_lift<<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, ad.thick.p, rn.p, f.p);
+      k_quad4_lift<<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, ad.thick.p, rn.p, f.p,
+                                         tied);
     else if (ad.general)
-      k_hex8_lift<true><<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, rn.p, f.p);
+      k_hex8_lift<true><<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, rn.p, f.p, tied);
     else
-      k_hex8_lift<false><<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, rn.p, f.p);
+      k_hex8_lift<false><<<grid, TPB, 0, s>>>(cnt, el, ad.coords.p, ad.elems.p, ad.cne.p, ad.emat.p, rn.p, f.p, tied);
     count_launches(1);
   }
   SGPU_CUDA(cudaGetLastError());
@@ -2683,6 +2706,7 @@ SGPU_API int sgpu_assemble_copy(sgpu_matrix src, int32_t kind, const double *ema
   DUP(ad.iptr, sa.iptr);
   DUP(ad.inc, sa.inc);
   ad.node_rows = sa.node_rows;
+  ad.tied = sa.tied;
 #undef DUP
   if (st != SGPU_OK) return bail(st);
   if (c.val.alloc(c.nnz + 2) != SGPU_OK || c.diag.alloc(c.n) != SGPU_OK) return bail(SGPU_CUDA_ERROR);

@@ -94,3 +94,45 @@ def test_the_largest_code_number_is_the_number_of_equations(gpu_lib, kind, ties)
         assert A.n == cn.max() < F.n
         adr, ci, _ = A.download(0)
         assert np.array_equal(np.repeat(np.arange(A.n), np.diff(adr)) * A.n + ci, want)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("ties", [ends, faces, chain])
+@pytest.mark.parametrize("whole", [True, False])
+def test_shared_equations(gpu_lib, kind, ties, whole):
+    kid, make = KINDS[kind]
+    mesh = make()
+    comps = range(mesh.ndofn) if whole else range(1)
+    pairs = [(s, m, c) for s, m in ties(mesh) for c in comps]
+    assert pairs
+    cn, to = tie(mesh, pairs)
+    with mefel.stiffness_matrix(mesh) as F:
+        K = dense(F)
+    T = np.zeros((K.shape[0], to.max() + 1))
+    T[np.arange(K.shape[0]), to] = 1.0
+    want = T.T @ K @ T
+    with assemble(mesh, kid, cn) as A:
+        assert A.n == to.max() + 1 < K.shape[0]
+        got = dense(A)
+    # sums of the same element terms in another order; an entry has at most (tied nodes x elements)^2 terms
+    terms = int(np.bincount(to).max()) ** 2 * 64
+    assert np.abs(got - want).max() <= terms * 2.3e-16 * np.abs(K).max() * terms
+
+
+@pytest.mark.parametrize("kind", ["hex8", "quad4"])
+@pytest.mark.parametrize("ties", [ends, faces, chain])
+def test_lifting_onto_shared_equations(gpu_lib, kind, ties):
+    kid, make = KINDS[kind]
+    mesh = make()
+    cn, to = tie(mesh, [(s, m, c) for s, m in ties(mesh) for c in range(mesh.ndofn)])
+    r = np.random.default_rng(4).standard_normal((mesh.nn, mesh.ndofn))
+    with mefel.stiffness_matrix(mesh) as F, assemble(mesh, kid, cn) as A:
+        f, g = np.zeros(F.n), np.zeros(A.n)
+        L.check(gpu_lib.sgpu_assembly_lift(F.h, r, f))
+        L.check(gpu_lib.sgpu_assembly_lift(A.h, r, g))
+        entry = np.abs(F.download(0)[2]).max()
+    want = np.zeros(A.n)
+    np.add.at(want, to, f)
+    # sums of at most 24 x 8 products for each of the tied nodes
+    terms = 192 * int(np.bincount(to).max())
+    assert np.abs(g - want).max() <= terms * 2.3e-16 * terms * entry * np.abs(r).max()
