@@ -805,13 +805,35 @@ double spmv_bytes(sgpu_matrix m, int format, int precision) {
   return (double)m->csr.nnz * (sv + 4.0) + (n + 1.0) * 4.0 + 2.0 * n * sv;
 }
 
+// The kernel of a plain product: the tuned one, else (no tuning run for the
+// handful of launches of a solve, or in a capture) the usual winner of its
+// format.
+SpmvPlan plain_plan(sgpu_matrix m) {
+  if (m->plan64.tuned) return m->plan64;
+  SpmvPlan p;
+  if (m->bsr.nb >= 0 && m->bsr.valid) {
+    p.format = 3;
+    p.variant = 132;
+  } else {
+    const double mean = (double)m->csr.nnz / (double)m->n;
+    p.variant = mean > 40 ? 16 : (mean > 12 ? 8 : 4);
+  }
+  return p;
+}
+
 }  // namespace
 
 // Plain FP64 SpMV with the tuned kernel (public: sgpu_matrix_mxv_d).
 int spmv64(sgpu_matrix m, const double *x, double *y, cudaStream_t s) {
   SGPU_TRY(ensure_work(m, false));
-  if (!m->plan64.tuned) SGPU_TRY(spmv_autotune(m, 64));
-  return launch_spmv64<EpiNone>(m, m->plan64.format, m->plan64.variant, x, y, s, 0);
+  if (!m->plan64.tuned) {
+    // nothing can be timed on a capturing stream; FP64 Jacobi solves do not tune
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    SGPU_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (cap == cudaStreamCaptureStatusNone) SGPU_TRY(spmv_autotune(m, 64));
+  }
+  const SpmvPlan pl = plain_plan(m);
+  return launch_spmv64<EpiNone>(m, pl.format, pl.variant, x, y, s, 0);
 }
 
 // The flexible CG of the multilevel preconditioner (sgpu_amg.cu): q = K p with
@@ -1011,21 +1033,6 @@ int capture_fp32_chunk(sgpu_matrix m, int iters, cudaGraphExec_t *exec, int64_t 
   if (e != cudaSuccess) return fail(SGPU_CUDA_ERROR, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
   *nodes = 3LL * iters;
   return SGPU_OK;
-}
-
-// The kernel of a solve's few plain products: the tuned one, else (no tuning
-// run for a handful of launches) the usual winner of its format.
-SpmvPlan plain_plan(sgpu_matrix m) {
-  if (m->plan64.tuned) return m->plan64;
-  SpmvPlan p;
-  if (m->bsr.nb >= 0 && m->bsr.valid) {
-    p.format = 3;
-    p.variant = 132;
-  } else {
-    const double mean = (double)m->csr.nnz / (double)m->n;
-    p.variant = mean > 40 ? 16 : (mean > 12 ? 8 : 4);
-  }
-  return p;
 }
 
 // true residual of the current w.x against w.f, into st->true_rel
