@@ -614,17 +614,14 @@ __global__ void __cluster_dims__(kClu, 1, 1) __launch_bounds__(kCluTPB, 1) k_bcl
     double v1[1] = {0.0};
     for (int j = 0; j < mine; j++) {
       const int st = j < fixed ? j : fixed + q;
-      if ((j >= fixed || first) && !ring_wait(full + st, j < fixed ? 0u : ph)) {
-        sh.bad = 1;
-        break;
-      }
+      const bool landed = (j < fixed && !first) || ring_wait(full + st, j < fixed ? 0u : ph);
       const unsigned char *stage = stages + (size_t)st * sb;
       const int t0 = (w + kCluWarps * j) * CluTile::kUnits, e0 = sp[t0];
       const double *vals = reinterpret_cast<const double *>(stage) + (e0 & 1);
       const int *cols = reinterpret_cast<const int *>(stage + vb) + (e0 & 3);
       const int sub = lane & 1, u = t0 + (lane >> 1);
       double y = 0.0, y2 = 0.0;
-      if (u < nu) {
+      if (landed && u < nu) {
         const int b = sp[u] - e0, len = sp[u + 1] - e0 - b;
         // 9 entries of a lane at a time (a plate's row has 18); the CTA's own
         // d first, then -- few rows, at the range's ends -- the neighbours'
@@ -660,7 +657,10 @@ __global__ void __cluster_dims__(kClu, 1, 1) __launch_bounds__(kCluTPB, 1) k_bcl
         }
         y += y2;
       }
-      __syncwarp();
+      if (!ring_landed(landed)) {
+        sh.bad = 1;
+        break;
+      }
       y += __shfl_xor_sync(0xffffffffu, y, 1);
       if (sub == 0 && u < nu) {
         ps[u] = y;

@@ -503,12 +503,19 @@ __device__ __forceinline__ bool ring_test(unsigned long long *bar, unsigned pari
       : "memory");
   return ok != 0;
 }
-// bounded wait (a try_wait suspends for up to about a microsecond)
-__device__ __forceinline__ bool ring_wait(unsigned long long *bar, unsigned parity) {
-  for (int tries = 0; tries < kPollLimit; tries++)
+// Bounded wait of a thread (a try_wait suspends for up to about a microsecond).
+// The lanes of a warp may get different answers, since a copy can land between
+// the last polls of two of them: they vote before they part (ring_landed).
+__device__ __forceinline__ bool ring_wait(unsigned long long *bar, unsigned parity, int limit = kPollLimit) {
+  for (int tries = 0; tries < limit; tries++)
     if (ring_test(bar, parity)) return true;
   return false;
 }
+// Whether a copy has landed for every lane of the warp.  It stands where the
+// lanes meet anyway, behind the work on the copy (that of the lanes that saw it
+// land): a vote at the wait itself took 25.8 us an iteration on 262,144 rows of
+// 27 entries, this 22.3.
+__device__ __forceinline__ bool ring_landed(bool mine) { return __all_sync(0xffffffffu, mine); }
 
 // A matrix as units of rows: block rows of 3 (BSR3, values component-major
 // per block row) or single rows (CSR).  The arrays are readable for 16 bytes
@@ -664,10 +671,7 @@ __global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const T
     double acc = 0.0;
     for (int j = 0; j < mine; j++) {
       const int t = w + kTileWarps * j;
-      if (!ring_wait(full + q, ph)) {
-        bad = 1;
-        break;
-      }
+      const bool landed = ring_wait(full + q, ph);
       const unsigned char *stage = stages + (size_t)q * sb;
       const int t0 = t * K::kUnits, e0 = sp[t0];
       const double *vals = reinterpret_cast<const double *>(stage) + ((K::kVals * e0) & 1);
@@ -675,7 +679,7 @@ __global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const T
       const int sub = lane % LPR, u = t0 + lane / LPR;
       if constexpr (ROWS == 1) {
         double y = 0.0, y2 = 0.0;
-        if (u < nu) {
+        if (landed && u < nu) {
           const int b = sp[u] - e0, len = sp[u + 1] - e0 - b;
           const double *v = vals + b;
           const int *c = cols + b;
@@ -694,7 +698,10 @@ __global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const T
           }
           y += y2;
         }
-        __syncwarp();
+        if (!ring_landed(landed)) {
+          bad = 1;
+          break;
+        }
 #pragma unroll
         for (int o = LPR / 2; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o, LPR);
         if (sub == 0 && u < nu) {
@@ -703,7 +710,7 @@ __global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const T
         }
       } else {
         double y0 = 0.0, y1 = 0.0, y2 = 0.0;
-        if (u < nu) {
+        if (landed && u < nu) {
           const int s = sp[u] - e0, nbr = sp[u + 1] - e0 - s;
           const double *v = vals + 9 * s;
           const int *c = cols + s;
@@ -728,7 +735,10 @@ __global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const T
             }
           }
         }
-        __syncwarp();
+        if (!ring_landed(landed)) {
+          bad = 1;
+          break;
+        }
         double y[3] = {y0, y1, y2};
         const double yv = RowSums<3, LPR>::sum(y, sub);
         if (RowSums<3, LPR>::first(sub) && u < nu) {
