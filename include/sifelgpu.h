@@ -406,7 +406,7 @@ SGPU_API int sgpu_transient_vform(sgpu_matrix K, sgpu_matrix C, const double *rh
  * *iterations (may be NULL) gets the iterations done.
  *
  * The work vectors live in one static device array of the library (about
- * 4 MiB, held by every GPU that loads it until exit), so n <=
+ * 5 MiB, held by every GPU that loads it until exit), so n <=
  * SGPU_NOALLOC_MAX_N (SGPU_BAD_INPUT beyond).  Nothing is allocated.  Every
  * call uses the same array: calls that overlap on the GPU race and must be
  * serialised.  The first call on each device looks up the array's device

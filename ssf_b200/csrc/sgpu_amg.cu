@@ -4373,23 +4373,24 @@ CoarseProgram &program(Amg &A) {
 
 // one launch of a whole coarse correction; B: the levels' block size
 template <typename T, int B>
-int launch_program_b(sgpu_matrix m, const CoarseProgram &p, cudaStream_t s) {
+cudaError_t launch_program_b(sgpu_matrix m, const CoarseProgram &p, cudaStream_t s) {
   Amg &A = *m->amg;
   auto k = k_coarse_program<T, B>;
   const size_t smem = (size_t)p.nsteps * sizeof(CoarseStep<T>);
-  if (smem > 48 * 1024)
-    SGPU_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
   const CoarseStep<T> *steps = reinterpret_cast<const CoarseStep<T> *>(p.steps.p);
   int n = p.nsteps;
   PcgState *st = pcg_state(m);
   ProgSync *ps = reinterpret_cast<ProgSync *>(A.prog_sync.p);
   void *args[] = {&steps, &n, &st, &ps};
-  SGPU_CUDA(cudaLaunchCooperativeKernel((const void *)k, dim3(p.grid), dim3(kProgTPB<T>), args, smem, s));
   count_launches(1);
-  return SGPU_OK;
+  return cudaLaunchCooperativeKernel((const void *)k, dim3(p.grid), dim3(kProgTPB<T>), args, smem, s);
 }
 template <typename T>
-int launch_program(sgpu_matrix m, const CoarseProgram &p, cudaStream_t s) {
+cudaError_t launch_program(sgpu_matrix m, const CoarseProgram &p, cudaStream_t s) {
   if (p.block == 6) return launch_program_b<T, 6>(m, p, s);
   if (p.block == 3) return launch_program_b<T, 3>(m, p, s);
   return launch_program_b<T, 1>(m, p, s);
@@ -4421,7 +4422,8 @@ int coarse_program(sgpu_matrix m, int l, int visits, const std::vector<Cheb> &ch
   CoarseProgram &p = program<T>(A);
   *ran = false;
   if (recorder<T>() || l != 1) return SGPU_OK;
-  if (!p.current) {
+  const bool first = !p.current;
+  if (first) {
     const AmgLevel &C = *A.lv[l];
     p.current = true;
     p.nsteps = 0;
@@ -4448,7 +4450,13 @@ int coarse_program(sgpu_matrix m, int l, int visits, const std::vector<Cheb> &ch
     p.result = xcur[l];
   }
   if (p.nsteps == 0) return SGPU_OK;
-  SGPU_TRY(launch_program<T>(m, p, s));
+  const cudaError_t e = launch_program<T>(m, p, s);
+  if (e != cudaSuccess && first) {  // refused (fewer SMs for this process than the device has): the kernels then
+    cudaGetLastError();
+    p.nsteps = 0;
+    return SGPU_OK;
+  }
+  SGPU_CUDA(e);
   xcur[l] = static_cast<T *>(p.result);
   *ran = true;
   return SGPU_OK;

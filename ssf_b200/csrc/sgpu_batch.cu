@@ -803,7 +803,22 @@ bool cluster_fits(int longest, int64_t most_rows) {
          28 * per + 256 + 2 * kCluWarps * (int64_t)CluTile::stage_bytes((int)ent) <= kCluSmem;
 }
 
-constexpr int kCoupled = 1000;  // run_cluster: the systems are not the matrix's diagonal blocks
+constexpr int kOther = 1000;  // run_cluster: not for this batch or device
+
+// Whether the device schedules a cluster with a CTA's shared memory each.
+bool cluster_runs(int sms) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kClu);
+  cfg.blockDim = dim3(kCluTPB);
+  cfg.dynamicSmemBytes = kCluSmem;
+  int most = 0;
+  if (sms >= kClu &&
+      cudaFuncSetAttribute(k_bcluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kCluSmem) == cudaSuccess &&
+      cudaOccupancyMaxActiveClusters(&most, k_bcluster, &cfg) == cudaSuccess)
+    return most > 0;
+  cudaGetLastError();
+  return false;
+}
 
 int run_cluster(sgpu_matrix m, const std::vector<int64_t> &rows, int longest, double *x, const double *f, int64_t ni,
                 double res, double zero, std::vector<SysState> &hs, int64_t *iters, float *ms) {
@@ -839,11 +854,10 @@ int run_cluster(sgpu_matrix m, const std::vector<int64_t> &rows, int longest, do
   count_launches(1);
   SGPU_CUDA(cudaMemcpyAsync(&coupled, flag_d, sizeof(int), cudaMemcpyDeviceToHost, s));
   SGPU_CUDA(cudaStreamSynchronize(s));
-  if (coupled) return kCoupled;
+  if (coupled) return kOther;
   const int ent = (longest * CluTile::kUnits + 3) & ~3;
   const CluArgs a = {items_d.p, ptr_d.p, c.rowptr.p, lcol.p, c.val.p, c.diag.p, f, x, st.p, ent, (long long)ni, res,
                      zero};
-  SGPU_CUDA(cudaFuncSetAttribute(k_bcluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kCluSmem));
   SGPU_CUDA(cudaEventRecord(m->ev0, s));
   k_bcluster<<<(unsigned)items.size(), kCluTPB, kCluSmem, s>>>(a);
   count_launches(1);
@@ -1078,9 +1092,10 @@ extern "C" SGPU_API int sgpu_matrix_pcg_batch(sgpu_matrix m, int32_t nsys, const
     int longest = 0;
     SGPU_TRY(longest_row(m, &longest));
     const int64_t most = *std::max_element(rows.begin(), rows.end());
-    int rc = kCoupled;
-    if (cluster_fits(longest, most)) rc = run_cluster(m, rows, longest, w.x.p, w.f.p, ni, res, zero, hs, &its, &ms);
-    if (rc == kCoupled)
+    int rc = kOther;
+    if (cluster_fits(longest, most) && cluster_runs(resident_grid()))
+      rc = run_cluster(m, rows, longest, w.x.p, w.f.p, ni, res, zero, hs, &its, &ms);
+    if (rc == kOther)
       rc = run_persistent(m, rows, best.L, w.x.p, w.f.p, w.r.p, w.h.p, w.d.p, w.p.p, ni, res, zero, hs, &its, &ms);
     if (rc != SGPU_OK) return rc;
   } else {

@@ -13,11 +13,11 @@
 // event creation).
 //
 // Limits and sharing:
-//  - at most SGPU_NOALLOC_MAX_N equations (131072): the array holds four
-//    FP64 vectors of that length plus reduction slots, about 4 MiB;
+//  - at most SGPU_NOALLOC_MAX_N equations (131072): the array holds five
+//    FP64 vectors of that length plus reduction slots, about 5 MiB;
 //  - every call uses the same array, which keeps the last call's contents;
 //    the entry point clears what must start at zero (the grid barrier, the
-//    iteration state) on every call;
+//    reduction tickets, the iteration state) on every call;
 //  - calls whose work overlaps on the GPU (two host threads, or two streams
 //    of one process, at the same time on the same device) race on the
 //    array: serialise them.
@@ -40,9 +40,11 @@
 // entries: the checks keep every read inside [0, rowptr[n]).
 //
 // The iteration (k_pcg_resident, one cooperative launch of a CTA per SM with
-// a thread or more per row, hence the largest size) is the reference's
-// symcomprow::cg_prec with the diagonal preconditioner (GEFEL/scr.cpp:1093-1205): stop on (r.r)/(f.f) < res, and
-// *ani = i, *ares = (r.h)/(f.f) written only on convergence.
+// a thread or more per row, hence the largest size; three launches an
+// iteration where the device refuses that one or has too few SMs) is the
+// reference's symcomprow::cg_prec with the diagonal preconditioner
+// (GEFEL/scr.cpp:1093-1205): stop on (r.r)/(f.f) < res, and *ani = i,
+// *ares = (r.h)/(f.f) written only on convergence.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -58,27 +60,33 @@ namespace {
 
 constexpr int kTPB = 256;
 constexpr int kMaxN = SGPU_NOALLOC_MAX_N;
-constexpr int kBlocks = 148 * 4;  // grid of the input check
+constexpr int kBlocks = 148 * 4;  // grid of the input check and of the general form
 // iterations of one launch, between two reads of the state: under 50 ms at
 // the largest size, and few enough waits that they cost nothing
 constexpr long long kChunk = 2048;
+constexpr int kGeneralChunk = 16;  // the same of the general form
 
 // byte layout of the scratch array
 constexpr size_t kVecBytes = sizeof(double) * (size_t)kMaxN;
 constexpr size_t kOffDiag = 0;
 constexpr size_t kOffR = kOffDiag + kVecBytes;
 constexpr size_t kOffDh = kOffR + kVecBytes;  // pairs {direction, preconditioned residual}
-constexpr size_t kOffSync = kOffDh + 2 * kVecBytes;
+constexpr size_t kOffD = kOffDh + 2 * kVecBytes;
+constexpr size_t kOffPart = kOffD + kVecBytes;                          // 2 * kBlocks doubles
+constexpr size_t kOffSync = kOffPart + 2 * kBlocks * sizeof(double);
 constexpr size_t kOffState = kOffSync + sizeof(GridSync);
-constexpr size_t kScratchBytes = kOffState + ((sizeof(PcgState) + 255) & ~(size_t)255);
+constexpr size_t kOffTicket = kOffState + ((sizeof(PcgState) + 255) & ~(size_t)255);  // 4 unsigned
+constexpr size_t kScratchBytes = kOffTicket + 256;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 struct Scratch {
   double *diag, *r;
-  double2 *dh;
+  double2 *dh;  // the general form's product and preconditioned residual
+  double *d, *part;
   GridSync *gs;
   PcgState *st;
+  unsigned *ticket;
 };
 
 Scratch carve(unsigned char *base) {
@@ -86,8 +94,11 @@ Scratch carve(unsigned char *base) {
   s.diag = reinterpret_cast<double *>(base + kOffDiag);
   s.r = reinterpret_cast<double *>(base + kOffR);
   s.dh = reinterpret_cast<double2 *>(base + kOffDh);
+  s.d = reinterpret_cast<double *>(base + kOffD);
+  s.part = reinterpret_cast<double *>(base + kOffPart);
   s.gs = reinterpret_cast<GridSync *>(base + kOffSync);
   s.st = reinterpret_cast<PcgState *>(base + kOffState);
+  s.ticket = reinterpret_cast<unsigned *>(base + kOffTicket);
   return s;
 }
 
@@ -112,7 +123,8 @@ int scratch_address(unsigned char **out) {
   return SGPU_OK;
 }
 
-// clears the state (one thread: nothing else of the call runs before it)
+// clears the state and the reduction tickets (one thread: nothing else of the
+// call runs before it)
 __global__ void k_na_clear(Scratch s, long long ni, double res, double zero) {
   PcgState z = {};
   z.ni = ni;
@@ -122,6 +134,7 @@ __global__ void k_na_clear(Scratch s, long long ni, double res, double zero) {
   z.prec = 1;
   z.ani = -1;
   *s.st = z;
+  for (int k = 0; k < 4; k++) s.ticket[k] = 0u;
 }
 
 // checks every row and extracts the diagonal; a malformed row stops the call
@@ -177,8 +190,7 @@ extern "C" SGPU_API int sgpu_csr_pcg_noalloc_d(int32_t n, const int32_t *rowptr_
   if (rc != SGPU_OK) return rc;
   const Scratch s = carve(base);
   const int grid = resident_grid();
-  if (!resident_rows_fit(n, grid))  // fewer than 128 SMs
-    return sgpu::fail(SGPU_CUDA_ERROR, "the device has too few SMs for the no-allocation solver's resident grid");
+  bool resident = resident_rows_fit(n, grid);
   k_na_clear<<<1, 1, 0, st>>>(s, (long long)ni, res, zero);
   k_na_setup<<<kBlocks, kTPB, 0, st>>>(n, rowptr_d, col_d, val_d, s);
   sgpu::count_launches(2);
@@ -196,16 +208,35 @@ extern "C" SGPU_API int sgpu_csr_pcg_noalloc_d(int32_t n, const int32_t *rowptr_
   a.gs = s.gs;
   a.iv = iv != 0;
   a.most = kChunk;
+  const GeneralPcg g = {n,      rowptr_d, col_d, val_d, s.diag, f_d, x_d, s.r, reinterpret_cast<double *>(s.dh) + kMaxN,
+                        s.d,    reinterpret_cast<double *>(s.dh), s.st, s.part, s.ticket, kBlocks};
   PcgState h = {};
-  for (a.start = 1;; a.start = 0) {
-    cudaError_t e = cudaMemsetAsync(s.gs, 0, sizeof(GridSync), st);
-    if (e == cudaSuccess) e = launch_resident(a, 0, grid, st);
-    sgpu::count_launches(1);
+  auto read = [&](cudaError_t e) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, s.st, sizeof(h), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return sgpu::fail(SGPU_CUDA_ERROR, std::string("no-allocation PCG: ") + cudaGetErrorString(e));
-    if (h.done) break;
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+  };
+  cudaError_t e = cudaSuccess;
+  for (a.start = 1; resident && e == cudaSuccess && !h.done; a.start = 0) {
+    e = cudaMemsetAsync(s.gs, 0, sizeof(GridSync), st);
+    if (e == cudaSuccess) e = launch_resident(a, 0, grid, st);
+    if (e != cudaSuccess && a.start) {  // refused: fewer SMs for this process than the device has
+      cudaGetLastError();
+      resident = false;
+      e = cudaSuccess;
+      break;
+    }
+    sgpu::count_launches(1);
+    e = read(e);
   }
+  if (!resident) {
+    e = read(e);  // the input check's verdict
+    if (e == cudaSuccess && !h.done) general_start(g, iv != 0, st);
+    while (e == cudaSuccess && !h.done) {
+      general_iterations(g, kGeneralChunk, st);
+      e = read(cudaGetLastError());
+    }
+  }
+  if (e != cudaSuccess) return sgpu::fail(SGPU_CUDA_ERROR, std::string("no-allocation PCG: ") + cudaGetErrorString(e));
   if (h.status == SGPU_CUDA_ERROR) return sgpu::fail(SGPU_CUDA_ERROR, "no-allocation PCG: the grid's barrier ran out");
   if (iterations) *iterations = h.it;
   if (h.ani_set) {

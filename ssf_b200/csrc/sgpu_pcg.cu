@@ -6,8 +6,9 @@
 //   d = beta d + h.
 // The whole iteration runs inside one cooperative launch (sgpu_persist.cuh):
 // with the matrix in shared memory where it fits the SMs, else streamed
-// through it.  Rows too long or too many for its stages, and a product pinned
-// by the caller, take the general form, three kernels per iteration:
+// through it.  Rows too long or too many for its stages, a product pinned by
+// the caller and a device that refuses such a launch take the general form,
+// three kernels per iteration:
 //   K_A  spmv + d.p  (last block: alpha, breakdown test)
 //   K_B  x,r update, h = r/diag, r.r and r.h (last block: beta, stop test)
 //   K_C  d = beta d + h
@@ -990,7 +991,7 @@ int write_state(sgpu_matrix m, const PcgState *h) {
 }
 
 // Builds a graph of `iters` FP64 iterations (3 kernels each).
-int capture_fp64_chunk(sgpu_matrix m, int iters, cudaGraphExec_t *exec, int64_t *nodes) {
+int capture_fp64_chunk(sgpu_matrix m, const SpmvPlan &pl, int iters, cudaGraphExec_t *exec, int64_t *nodes) {
   cudaStream_t s = m->stream;
   Work &w = m->w;
   const int n = (int)m->n;
@@ -999,7 +1000,7 @@ int capture_fp64_chunk(sgpu_matrix m, int iters, cudaGraphExec_t *exec, int64_t 
   cudaGraph_t g;
   SGPU_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
   for (int it = 0; it < iters; it++) {
-    int rc = launch_spmv64<EpiAlpha64>(m, m->plan64.format, m->plan64.variant, w.d.p, w.p.p, s, 1);
+    int rc = launch_spmv64<EpiAlpha64>(m, pl.format, pl.variant, w.d.p, w.p.p, s, 1);
     if (rc != SGPU_OK) { cudaStreamEndCapture(s, &g); return rc; }
     k_pcg64_update<<<vg, TPB, 0, s>>>(n, w.x.p, w.r.p, w.h.p, w.d.p, w.p.p, m->csr.diag.p, st, w.partials.p,
                                       w.counters.p + 2);
@@ -1121,36 +1122,51 @@ int solve_fp64(sgpu_matrix m, int64_t ni, double res, double zero, int64_t iv, i
   SGPU_TRY(write_state(m, &init));
   if (iv == 0) SGPU_CUDA(cudaMemsetAsync(w.x.p, 0, (size_t)n * sizeof(double), s));
   const SpmvPlan pl = plain_plan(m);
-  if (form != Form::kResident) {  // the resident grid starts its solve itself
+  auto begin = [&]() -> int {
     // p = A x0: zero for x0 = 0 (iv == 0, where the reference zeroes x and multiplies)
     if (iv == 0) SGPU_CUDA(cudaMemsetAsync(w.p.p, 0, (size_t)n * sizeof(double), s));
     else SGPU_TRY(launch_spmv64<EpiNone>(m, pl.format, pl.variant, w.x.p, w.p.p, s, 0));
     k_pcg64_init<<<vg, TPB, 0, s>>>(n, w.f.p, w.p.p, m->csr.diag.p, w.r.p, w.h.p, w.d.p, state_of(m), w.partials.p,
                                     w.counters.p + 2);
     count_launches(1);
-  }
+    return SGPU_OK;
+  };
+  if (form != Form::kResident) SGPU_TRY(begin());  // the resident grid starts its solve itself
   GridSync *gs = reinterpret_cast<GridSync *>(w.gsync.p);
   ResidentArgs ra = {n,     m->csr.rowptr.p, m->csr.col.p, m->csr.val.p, m->csr.diag.p, w.f.p, w.x.p, w.r.p,
                      reinterpret_cast<double2 *>(w.pair.p), state_of(m), gs, 0, 0, 1, (int)(iv != 0), kPersistChunk};
   const TileArgs ta = {n, m->csr.diag.p, w.x.p, w.r.p, w.h.p, w.d.p, w.p.p, state_of(m), gs, kPersistChunk};
   cudaGraphExec_t exec = nullptr;
   int64_t nodes = 0;
-  if (form == Form::kGraph) SGPU_TRY(capture_fp64_chunk(m, kChunk, &exec, &nodes));
   int rc = SGPU_OK;
   std::vector<double> confirms;
   for (;;) {
     cudaError_t e = cudaSuccess;
-    if (form == Form::kGraph) {
-      e = cudaGraphLaunch(exec, s);
-      count_launches(nodes);
-    } else {
+    if (form != Form::kGraph) {
       e = cudaMemsetAsync(gs, 0, sizeof(GridSync), s);
       if (e == cudaSuccess && form == Form::kResident) e = launch_resident(ra, m->csr.nnz, sms, s);
       else if (e == cudaSuccess)
         e = m->used64.format == 3 ? launch_tiles<3>(ta, tm, longest, lanes, sms, s)
                                   : launch_tiles<1>(ta, tm, longest, lanes, sms, s);
-      ra.start = 0;
-      count_launches(1);
+      if (e == cudaSuccess) {
+        ra.start = 0;
+        count_launches(1);
+      } else if (ra.start || form == Form::kTiles) {
+        // refused (fewer SMs for this process than the device has): the
+        // general form takes the solve as it stands
+        cudaGetLastError();
+        if (form == Form::kResident) rc = begin();
+        if (rc != SGPU_OK) break;
+        form = Form::kGraph;
+        m->used64 = pl;
+        e = cudaSuccess;
+      }
+    }
+    if (form == Form::kGraph) {
+      if (!exec) rc = capture_fp64_chunk(m, m->used64, kChunk, &exec, &nodes);
+      if (rc != SGPU_OK) break;
+      e = cudaGraphLaunch(exec, s);
+      count_launches(nodes);
     }
     if (e != cudaSuccess) { rc = fail(SGPU_CUDA_ERROR, std::string("PCG launch: ") + cudaGetErrorString(e)); break; }
     rc = read_state(m, hs);
@@ -1360,6 +1376,29 @@ int pcg_run(sgpu_matrix m, int64_t ni, double res, double zero, int64_t iv, int 
     info->fallback = fallback;
   }
   return hs.status;
+}
+
+void general_start(const GeneralPcg &a, bool iv, cudaStream_t s) {
+  const size_t bytes = (size_t)a.n * sizeof(double);
+  if (iv) {
+    k_spmv_csr<double, double, double, 16, EpiNone><<<a.blocks, TPB, 0, s>>>(a.n, a.rowptr, a.col, a.val, a.x, a.p, a.st,
+                                                                             a.partials, a.tickets);
+    count_launches(1);
+  } else {
+    cudaMemsetAsync(a.x, 0, bytes, s);
+    cudaMemsetAsync(a.p, 0, bytes, s);
+  }
+  k_pcg64_init<<<a.blocks, TPB, 0, s>>>(a.n, a.f, a.p, a.diag, a.r, a.h, a.d, a.st, a.partials, a.tickets + 1);
+  count_launches(1);
+}
+void general_iterations(const GeneralPcg &a, int count, cudaStream_t s) {
+  for (int k = 0; k < count; k++) {
+    k_spmv_csr<double, double, double, 16, EpiAlpha64><<<a.blocks, TPB, 0, s>>>(a.n, a.rowptr, a.col, a.val, a.d, a.p,
+                                                                                a.st, a.partials, a.tickets);
+    k_pcg64_update<<<a.blocks, TPB, 0, s>>>(a.n, a.x, a.r, a.h, a.d, a.p, a.diag, a.st, a.partials, a.tickets + 1);
+    k_pcg64_dir<<<a.blocks, TPB, 0, s>>>(a.n, a.d, a.h, a.st);
+  }
+  count_launches(3 * count);
 }
 
 // entries of the longest CSR row

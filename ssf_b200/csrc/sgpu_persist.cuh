@@ -10,6 +10,7 @@
 #pragma once
 
 #include <algorithm>
+#include <cstdlib>
 
 #include "sgpu_internal.cuh"
 
@@ -418,13 +419,15 @@ __global__ void __launch_bounds__(kResidentTPB, 1) k_pcg_resident(const Resident
   }
 }
 
-// CTAs of a resident grid on the current device (one per SM), and the entries
-// its shared memory holds
+// CTAs of a resident grid on the current device: one per SM.  SGPU_SMS=<n>
+// states how many SMs the process may count on where it has only a share of
+// the device's (read at every solve).
 inline int resident_grid() {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return 0;
+  if (const char *e = getenv("SGPU_SMS")) sms = std::max(0, atoi(e));
   return sms < kMaxGrid ? sms : kMaxGrid;
 }
 constexpr int kResidentSmem = 220 * 1024;  // beside about 1.2 KB of static shared memory
@@ -857,5 +860,23 @@ inline cudaError_t launch_tiles(const TileArgs &a, const TileMat &m, int longest
     return launch_tiles_as<1, 32>(a, m, longest, sms, s);
   }
 }
+
+// ---------------------------------------------------------------------------
+// the general form without a handle (sgpu_pcg.cu)
+// ---------------------------------------------------------------------------
+// Where the device refuses a resident grid: three launches an iteration on
+// plain CSR, with the state's scalars and tests.
+struct GeneralPcg {
+  int n;
+  const int *rowptr, *col;
+  const double *val, *diag, *f;
+  double *x, *r, *h, *d, *p;
+  PcgState *st;
+  double *partials;   // 2 * blocks
+  unsigned *tickets;  // 3, zero
+  int blocks;
+};
+void general_start(const GeneralPcg &a, bool iv, cudaStream_t s);        // r = f - A x0 and the first direction
+void general_iterations(const GeneralPcg &a, int count, cudaStream_t s);
 
 }  // namespace sgpu
