@@ -29,9 +29,11 @@ namespace sgpu {
 // the CTA's own reduction 0.7; polling 148 flagged partials directly (no
 // counter) took 4.1 us, with 148 x 148 polls in flight.
 //
-// The launch is cooperative, so all CTAs are resident; the poll still has a
-// limit, after which the CTA gives up (the others then run out too) and the
-// caller reports SGPU_CUDA_ERROR.
+// The launch is cooperative: it starts once all its CTAs can run at the same
+// time (with 20 SMs held by another kernel for 4.5 s, a solve began after
+// those and took as long as ever), so a poll waits for the grid's own CTAs
+// only.  It still has a limit, after which the CTA gives up (the others then
+// run out too) and the caller reports SGPU_CUDA_ERROR.
 constexpr int kPollLimit = 1 << 22;  // about 3 s of polls
 constexpr int kMaxGrid = 256;        // CTAs the slots hold
 
