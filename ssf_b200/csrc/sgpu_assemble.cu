@@ -146,17 +146,18 @@ __global__ void k_codes(int64_t m, int ndofn, const int64_t *__restrict__ cn, co
 // one warp per node i: the sorted distinct nodes that share an element with
 // i (i among them), at nadj[nne * iptr[i]] -- the candidates' own number, so
 // one pass needs no count before it.  cnt[i]: how many; len[i]: entries of
-// i's rows (components times free components of the list).  Up to 64
-// candidates are sorted in registers, two per lane; more (quadratic elements)
-// bitonically in shared memory.  A node with more than kAdjCap candidates
-// sets err bit 16 (the caller falls back), one with equations but no element
-// bit 2.
+// i's rows (components times free components of the list); longest (zero
+// before): those of the longest row.  Up to 64 candidates
+// are sorted in registers, two per lane; more (quadratic elements) bitonically
+// in shared memory.  A node with more than kAdjCap candidates sets err bit 16
+// (the caller falls back), one with equations but no element bit 2.
 // On the 1.01M-equation cantilever (344,000 nodes of 64 candidates) the list
 // of the lower neighbours took two passes of 0.37 ms in shared memory.
 __global__ void __launch_bounds__(TPB) k_node_adj(int64_t nn, int nne, int ndofn, const int64_t *__restrict__ elems,
                                                   const int *__restrict__ iptr, const int *__restrict__ inc,
                                                   const int *__restrict__ code, int *__restrict__ cnt,
-                                                  int *__restrict__ len, int *__restrict__ nadj, unsigned *err) {
+                                                  int *__restrict__ len, int *__restrict__ nadj, unsigned *err,
+                                                  int *longest) {
   __shared__ int buf[WPB][kAdjCap];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   int *sb = buf[wib];
@@ -248,6 +249,7 @@ __global__ void __launch_bounds__(TPB) k_node_adj(int64_t nn, int nne, int ndofn
       for (int c = 0; c < ndofn; c++) own += code[i * ndofn + c] >= 0;
       cnt[i] = total;
       len[i] = own * nfree;
+      if (own && nfree > *(volatile int *)longest) atomicMax(longest, nfree);
       if (own && !total) atomicOr(err, 2u);  // an equation no element touches
     }
   }
@@ -2141,11 +2143,13 @@ int pattern_adjacency(sgpu_matrix m, const int64_t *elems_d, const int *code_d, 
   SGPU_TRY(nadj.alloc((size_t)ne * nne * nne));
   SGPU_CUDA(cudaMemsetAsync(len.p + nn, 0, sizeof(int), s));
   const int gadj = (int)std::min<int64_t>((nn + WPB - 1) / WPB, (int64_t)kNumSMs * 32);
-  k_node_adj<<<gadj, TPB, 0, s>>>(nn, nne, ndofn, elems_d, iptr_d, inc_d, code_d, cnt.p, len.p, nadj.p, err_d);
+  AsyncBuf<int64_t> total(s);  // the row lengths may add up past int32; and the longest row
+  SGPU_TRY(total.alloc(2));
+  SGPU_CUDA(cudaMemsetAsync(total.p, 0, 2 * sizeof(int64_t), s));
+  k_node_adj<<<gadj, TPB, 0, s>>>(nn, nne, ndofn, elems_d, iptr_d, inc_d, code_d, cnt.p, len.p, nadj.p, err_d,
+                                  reinterpret_cast<int *>(total.p + 1));
   count_launches(1);
-  AsyncBuf<int64_t> total(s);  // the row lengths may add up past int32
   {
-    SGPU_TRY(total.alloc(1));
     size_t tmp = 0;
     cub::DeviceReduce::Reduce(nullptr, tmp, len.p, total.p, (int)nn, cuda::std::plus<int64_t>(), (int64_t)0, s);
     AsyncBuf<unsigned char> t(s);
@@ -2154,8 +2158,8 @@ int pattern_adjacency(sgpu_matrix m, const int64_t *elems_d, const int *code_d, 
     count_launches(1);
   }
   SGPU_TRY(scan_into(len.p, row0.p, nn, s));
-  int64_t nnz = 0;
-  SGPU_CUDA(cudaMemcpyAsync(&nnz, total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  int64_t sums[2] = {0, 0};
+  SGPU_CUDA(cudaMemcpyAsync(sums, total.p, sizeof(sums), cudaMemcpyDeviceToHost, s));
   unsigned e = 0;
   SGPU_TRY(read_err(err_d, s, &e));
   if (e & 16u) {
@@ -2163,9 +2167,11 @@ int pattern_adjacency(sgpu_matrix m, const int64_t *elems_d, const int *code_d, 
     return 1;
   }
   if (e & 3u) return fail(SGPU_BAD_INPUT, "code numbers: element node out of range or unused equation");
+  const int64_t nnz = sums[0];
   if (nnz >= (1LL << 31) - 1) return fail(SGPU_BAD_INPUT, "matrix too large for int32 device indices");
   Csr &c = m->csr;
   SGPU_TRY(matrix_alloc_csr(m, n, nnz));
+  c.longest = (int)sums[1];
   m->src_negm = (nnz + n) / 2;
   k_csr_fill<<<(int)std::min<int64_t>((nn + WPB - 1) / WPB, (int64_t)kNumSMs * 64), TPB, 0, s>>>(
       nn, nne, ndofn, iptr_d, code_d, cnt.p, len.p, row0.p, nadj.p, c.rowptr.p, c.col.p, (int)n);
@@ -2686,6 +2692,7 @@ SGPU_API int sgpu_assemble_copy(sgpu_matrix src, int32_t kind, const double *ema
   Csr &c = m->csr;
   c.n = src->csr.n;
   c.nnz = src->csr.nnz;
+  c.longest = src->csr.longest;
   int st = SGPU_OK;
 #define DUP(dst, from)                                                                        \
   if (st == SGPU_OK && (from).p) {                                                            \

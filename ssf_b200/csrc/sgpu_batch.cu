@@ -30,7 +30,6 @@ using namespace sgpu;
 
 namespace sgpu {
 int pcg_prepare(sgpu_matrix m, bool mixed);
-int longest_row(sgpu_matrix m, int *longest);
 }
 
 namespace {
@@ -1089,8 +1088,7 @@ extern "C" SGPU_API int sgpu_matrix_pcg_batch(sgpu_matrix m, int32_t nsys, const
     const double mean = (double)m->csr.nnz / (double)m->n;
     best.L = mean > 40 ? 16 : (mean > 12 ? 8 : 4);
     best.S = 0;
-    int longest = 0;
-    SGPU_TRY(longest_row(m, &longest));
+    const int longest = m->csr.longest;
     const int64_t most = *std::max_element(rows.begin(), rows.end());
     int rc = kOther;
     if (cluster_fits(longest, most) && cluster_runs(resident_grid()))

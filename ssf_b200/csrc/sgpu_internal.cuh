@@ -148,7 +148,7 @@ struct Csr {
   DevBuf<double> dscale;     // 1 / sqrt(a_ii)
   bool have32 = false;
   bool diag_positive = false;
-  int longest = 0;           // entries of the longest row; 0 not yet known
+  int longest = 0;           // entries of the longest row
 };
 
 // 3x3 block rows (BSR3): node-blocked form of a CSR whose equations come in
@@ -163,7 +163,6 @@ struct Bsr3 {
   bool known = false;  // node-blocked by construction: no check of the rows needed
   bool valid = false;
   bool have32 = false;
-  int longest = 0;  // blocks of the longest block row; 0 not yet known
   // most blocks in one tile of 32 block rows (the FP32 level-0 products that
   // stream tiles through shared memory); 0 not yet known
   int tile_cap = 0;

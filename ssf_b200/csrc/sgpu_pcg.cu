@@ -519,16 +519,6 @@ __global__ void k_pair_h(int n, const double *__restrict__ h, double2 *__restric
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dh[i].y = h[i];
 }
 
-// the longest row (units of ptr)
-__global__ void k_longest(int units, const int *__restrict__ ptr, int *out) {
-  int most = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < units; i += gridDim.x * blockDim.x)
-    most = max(most, ptr[i + 1] - ptr[i]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, most);
-}
-
 __global__ void k_fill(int n, double *__restrict__ a, double v) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a[i] = v;
 }
@@ -1055,39 +1045,35 @@ constexpr long long kPersistChunk = 4096;
 // How an FP64 solve iterates.
 enum class Form { kResident, kTiles, kGraph };
 
-int longest_unit(sgpu_matrix m, int units, const int *ptr, int *cached) {
-  if (*cached > 0) return SGPU_OK;
-  int *out = reinterpret_cast<int *>(m->w.counters.p + 8);
-  SGPU_CUDA(cudaMemsetAsync(out, 0, sizeof(int), m->stream));
-  k_longest<<<std::min((units + TPB - 1) / TPB, 4 * kNumSMs), TPB, 0, m->stream>>>(units, ptr, out);
-  count_launches(1);
-  SGPU_CUDA(cudaMemcpyAsync(cached, out, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
-  SGPU_CUDA(cudaStreamSynchronize(m->stream));
-  return SGPU_OK;
-}
+// Resident where every row has a thread, the entries (12 bytes each) fit the
+// SMs' shared memory with 15 % to spare for uneven rows, and no lane has more
+// than kResidentChain entries: 27,000 equations in 1.96M entries took 8.6 us an
+// iteration resident against 10.1 streamed, 101,404 in 1.8M 8.1 against 10.7;
+// 105,840 in 8M (a quarter fits) 28.5 against 19.  The lanes of one long row
+// hold up the others: 120,000 rows of 9 entries and one of 150 (a lane's) take
+// 20.5 us, 27.6 in the general form, with one of 300 32.5 and 29.7; 20,000
+// rows and one of 600 (four lanes') 21.5 and 23.9, of 1200 32.5 and 26.9.
+// Streamed otherwise, in 3x3 blocks where the matrix has them, if its rows are
+// even and long enough for that (tile_lanes).
+constexpr int kResidentChain = 160;
 
-// Resident where every row has a thread and the entries (12 bytes each) fit
-// the SMs' shared memory with 15 % to spare for uneven rows: 27,000 equations
-// in 1.96M entries took 8.6 us an iteration resident against 10.1 streamed,
-// 101,404 in 1.8M 8.1 against 10.7; 105,840 in 8M (a quarter fits) 28.5
-// against 19.  Streamed otherwise, in 3x3 blocks where the matrix has them.
 int choose_form(sgpu_matrix m, int sms, Form *form, TileMat *tm, int *longest, int *lanes) {
   *form = Form::kGraph;
   if (m->plan64.pinned || getenv("SGPU_SPMV64")) return SGPU_OK;
   const Csr &c = m->csr;
-  if (resident_rows_fit(m->n, sms) && 12.0 * (double)c.nnz <= 0.85 * (double)sms * kResidentSmem) {
+  if (resident_rows_fit(m->n, sms) && 12.0 * (double)c.nnz <= 0.85 * (double)sms * kResidentSmem &&
+      c.longest <= kResidentChain * resident_lanes((int)m->n, sms)) {
     *form = Form::kResident;
     m->used64.format = 0;
     m->used64.variant = 0;
     return SGPU_OK;
   }
   SGPU_TRY(ensure_bsr3(m));
-  Bsr3 &b = m->bsr;
+  const Bsr3 &b = m->bsr;
   *tm = b.valid ? TileMat{b.nb, b.browptr.p, b.bcol.p, b.bval.p, 0, 0, 0}
                 : TileMat{c.n, c.rowptr.p, c.col.p, c.val.p, 0, 0, 0};
-  SGPU_TRY(longest_unit(m, tm->units, tm->ptr, b.valid ? &b.longest : &m->csr.longest));
-  *longest = b.valid ? b.longest : c.longest;
-  *lanes = b.valid ? tile_lanes<3>(*tm, *longest, sms) : tile_lanes<1>(*tm, *longest, sms);
+  *longest = b.valid ? c.longest / 3 : c.longest;
+  *lanes = b.valid ? tile_lanes<3>(*tm, *longest, b.nblk, sms) : tile_lanes<1>(*tm, *longest, c.nnz, sms);
   if (*lanes > 0) {
     *form = Form::kTiles;
     m->used64.format = b.valid ? 3 : 0;
@@ -1399,14 +1385,6 @@ void general_iterations(const GeneralPcg &a, int count, cudaStream_t s) {
     k_pcg64_dir<<<a.blocks, TPB, 0, s>>>(a.n, a.d, a.h, a.st);
   }
   count_launches(3 * count);
-}
-
-// entries of the longest CSR row
-int longest_row(sgpu_matrix m, int *longest) {
-  SGPU_TRY(ensure_work(m, false));
-  SGPU_TRY(longest_unit(m, m->csr.n, m->csr.rowptr.p, &m->csr.longest));
-  *longest = m->csr.longest;
-  return SGPU_OK;
 }
 
 int pcg_prepare(sgpu_matrix m, bool mixed) { return ensure_work(m, mixed); }

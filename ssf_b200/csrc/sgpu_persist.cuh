@@ -448,6 +448,14 @@ inline cudaError_t launch_resident_t(const ResidentArgs &a, int grid, cudaStream
 // Whether n rows have a thread each in the resident grid.
 inline bool resident_rows_fit(int64_t n, int grid) { return grid > 0 && n <= (int64_t)grid * kResidentTPB; }
 
+// Lanes that share a row of the resident grid.
+inline int resident_lanes(int n, int grid) {
+  const int rows = (n + grid - 1) / grid;  // of a CTA
+  int t = 1;
+  while (t < 32 && 2 * t * rows <= kResidentTPB) t *= 2;
+  return t;
+}
+
 // nnz: entries of the matrix where the host knows them (twice a CTA's share
 // is asked for, the rest of the SM's memory stays L1), else 0
 inline cudaError_t launch_resident(ResidentArgs a, int64_t nnz, int grid, cudaStream_t s) {
@@ -455,16 +463,17 @@ inline cudaError_t launch_resident(ResidentArgs a, int64_t nnz, int grid, cudaSt
   if (nnz > 0) cap = std::min<int64_t>(cap, 2 * (nnz / grid) + 2048);
   a.cap = (int)cap & ~31;
   a.rows_per_cta = (a.n + grid - 1) / grid;
+  const int lanes = resident_lanes(a.n, grid);
   grid = (a.n + a.rows_per_cta - 1) / a.rows_per_cta;  // no CTA without rows
-  const int r = a.rows_per_cta;
-  if (r > 512) return launch_resident_t<1>(a, grid, s);
-  if (r > 256) return launch_resident_t<2>(a, grid, s);
-  if (r > 128) return launch_resident_t<4>(a, grid, s);
-  if (r > 64) return launch_resident_t<8>(a, grid, s);
-  if (r > 32) return launch_resident_t<16>(a, grid, s);
-  return launch_resident_t<32>(a, grid, s);
+  switch (lanes) {
+    case 1: return launch_resident_t<1>(a, grid, s);
+    case 2: return launch_resident_t<2>(a, grid, s);
+    case 4: return launch_resident_t<4>(a, grid, s);
+    case 8: return launch_resident_t<8>(a, grid, s);
+    case 16: return launch_resident_t<16>(a, grid, s);
+    default: return launch_resident_t<32>(a, grid, s);
+  }
 }
-
 
 // ---------------------------------------------------------------------------
 // the streaming iteration: matrices that do not fit the SMs
@@ -796,8 +805,8 @@ __global__ void __launch_bounds__(TPBX, 1) k_pcg_tiles(const TileArgs a, const T
 // The rule of the launch: the fewest lanes per unit whose stages (one per
 // warp at least) fit.  Fewer lanes mean wider tiles, fewer shuffles and more
 // gathers in flight per lane; the longest unit decides whether they fit
-// (8 lanes up to 43 blocks a row, 32 up to 166 of BSR3; 2 lanes up to 66
-// entries a row, 8 up to 265, 32 up to 700 of CSR).  16 warps of up to 128
+// (8 lanes up to 41 blocks a row, 16 up to 82, 32 up to 164 of BSR3; 2 lanes up
+// to 66 entries a row, 8 up to 265, 32 up to 704 of CSR).  16 warps of up to 128
 // registers; the rows that 32 lanes share, in which every warp has only its
 // own row's gathers in flight, run 24 (60,000 rows of 401 entries 89.3 us an
 // iteration with 16 warps, 79.4 with 24).  With 24 warps throughout, whose
@@ -835,18 +844,47 @@ inline cudaError_t launch_tiles_as(const TileArgs &a, TileMat m, int longest, in
   return cudaLaunchCooperativeKernel((const void *)k, dim3(grid), dim3(TPBX), p, smem, s);
 }
 
-// lanes per unit (0: the rows are too long or too many for the tiles)
+// A unit costs its lanes' group a gather's latency however short it is, where
+// the general form's kernels have many more warps to hide it.  So the tiles
+// are for units of kTileMean entries and more on average, which a long row
+// among short ones does not make; kTileSlack allows for the launches that the
+// general form pays, i.e. shorter units where there are few of them:
+// kTileMean * units - entries <= kTileSlack.  Time of an iteration in tiles
+// against the general form, us:
+//   CSR, 2 lanes   200,000 rows of 3 13.8 / 22.6; 1M of 3 41.2 / 35.2, of 7 42.0
+//                  / 46.3; 2.5M of 7 107 / 95, of 9 110 / 110, of 13 116 / 135
+//   CSR, 8 lanes   150,000 rows of 25 (one of 200) 29.4 / 33.4, 600,000 95.0 /
+//                  65.0; 300,000 of 101 78.3 / 84.6
+//   CSR, 32 lanes  150,000 rows of 89 (one of 600) 68.6 / 59.1; 60,000 of 271
+//                  47.9 / 53.3, of 601 81.7 / 85.1
+//   BSR3, 8        350,000 rows of 3 57.7 / 49.7, of 13 68.8 / 92.5; 150,000 of
+//                  7 30.7 / 36.6
+//   BSR3, 16       150,000 of 13 (one of 60) 55.1 / 51.4, of 21 59.2 / 62.0;
+//                  50,000 of 45 34.8 / 49.0
+//   BSR3, 32       60,000 of 21 (one of 150) 42.6 / 41.6, 150,000 93.3 / 65.5;
+//                  50,000 of 101 73.6 / 82.6
+template <int ROWS, int LPR>
+constexpr int kTileMean = ROWS == 3 ? (LPR == 8 ? 10 : LPR == 16 ? 18 : 45) : (LPR == 2 ? 9 : LPR == 8 ? 55 : 200);
+template <int ROWS, int LPR>
+constexpr double kTileSlack = ROWS == 3 ? (LPR == 8 ? 1.0e6 : LPR == 16 ? 0.7e6 : 0.8e6)
+                                        : (LPR == 2 ? 3.5e6 : LPR == 8 ? 5e6 : 6e6);
+template <int ROWS, int LPR>
+inline int tiles_pay(const TileMat &m, int64_t entries) {
+  return (double)kTileMean<ROWS, LPR> * m.units - (double)entries <= kTileSlack<ROWS, LPR> ? LPR : 0;
+}
+
+// lanes per unit (0: the units are too long, too many or too uneven for tiles)
 template <int ROWS>
-inline int tile_lanes(const TileMat &m, int longest, int sms) {
+inline int tile_lanes(const TileMat &m, int longest, int64_t entries, int sms) {
   if (sms <= 0) return 0;
   if constexpr (ROWS == 3) {
-    if (tiles_fit<3, 8>(m, longest, sms)) return 8;
-    if (tiles_fit<3, 16>(m, longest, sms)) return 16;
-    if (tiles_fit<3, 32>(m, longest, sms)) return 32;
+    if (tiles_fit<3, 8>(m, longest, sms)) return tiles_pay<3, 8>(m, entries);
+    if (tiles_fit<3, 16>(m, longest, sms)) return tiles_pay<3, 16>(m, entries);
+    if (tiles_fit<3, 32>(m, longest, sms)) return tiles_pay<3, 32>(m, entries);
   } else {
-    if (tiles_fit<1, 2>(m, longest, sms)) return 2;
-    if (tiles_fit<1, 8>(m, longest, sms)) return 8;
-    if (tiles_fit<1, 32>(m, longest, sms)) return 32;
+    if (tiles_fit<1, 2>(m, longest, sms)) return tiles_pay<1, 2>(m, entries);
+    if (tiles_fit<1, 8>(m, longest, sms)) return tiles_pay<1, 8>(m, entries);
+    if (tiles_fit<1, 32>(m, longest, sms)) return tiles_pay<1, 32>(m, entries);
   }
   return 0;
 }

@@ -216,6 +216,7 @@ SGPU_API int sgpu_matrix_combine(sgpu_matrix K, sgpu_matrix C, double a, double 
   const int64_t n = K->n, nnz = K->csr.nnz;
   int st = matrix_alloc_csr(m, n, nnz);
   if (st != SGPU_OK) return bail(st);
+  m->csr.longest = K->csr.longest;
   m->bsr.known = K->bsr.known;
   cudaMemcpyAsync(m->csr.rowptr.p, K->csr.rowptr.p, (n + 1) * sizeof(int), cudaMemcpyDeviceToDevice, s);
   cudaMemcpyAsync(m->csr.col.p, K->csr.col.p, nnz * sizeof(int), cudaMemcpyDeviceToDevice, s);
