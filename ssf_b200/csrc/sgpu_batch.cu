@@ -21,6 +21,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <vector>
 
 #include "sgpu_internal.cuh"
@@ -802,6 +803,32 @@ bool cluster_fits(int longest, int64_t most_rows) {
          28 * per + 256 + 2 * kCluWarps * (int64_t)CluTile::stage_bytes((int)ent) <= kCluSmem;
 }
 
+// Whether clusters finish the batch earlier than CTAs with a system each, two
+// to an SM: the times of an iteration are summed over the waves of either form
+// as if all systems took as many iterations.  A CTA of a cluster has an SM of
+// its own, which small systems do not fill.  Measured for 100 iterations (ms,
+// clusters / CTAs): 5000 systems of 60 rows of 9 entries 8.09 / 3.54, 2000 of
+// 200 4.22 / 2.42, 500 of 1000 2.30 / 1.82; 256 of 2048 rows of 17 3.58 / 4.21,
+// 148 of 2000 2.37 / 3.33, 64 of 8000 4.27 / 15.5, 10 of 30,000 2.34 / 57.7.
+// mean: entries of a row.
+bool cluster_pays(const std::vector<int64_t> &rows, double mean, int sms) {
+  // us of an iteration by these measurements
+  auto on_cta = [&](int64_t r) { return 2.0 + 1.1e-3 * mean * (double)r; };
+  auto on_cluster = [&](int64_t r) {
+    return r <= kCluAlone ? 2.7 + 4.5e-4 * mean * (double)r : 3.0 + 5.6e-5 * mean * (double)r;
+  };
+  std::vector<int64_t> sorted(rows);
+  std::sort(sorted.begin(), sorted.end(), std::greater<int64_t>());
+  double ctas = 0.0;
+  for (int64_t r : sorted) ctas += on_cta(r);
+  ctas = std::max(ctas / (2.0 * sms), on_cta(sorted[0]));
+  // clusters in launch order, each to the slot that is free first
+  std::vector<double> slot((size_t)std::max(1, sms / kClu), 0.0);
+  for (size_t k = 0; k < sorted.size(); k += sorted[k] > kCluAlone ? 1 : kClu)
+    *std::min_element(slot.begin(), slot.end()) += on_cluster(sorted[k]);
+  return *std::max_element(slot.begin(), slot.end()) <= ctas;
+}
+
 constexpr int kOther = 1000;  // run_cluster: not for this batch or device
 
 // Whether the device schedules a cluster with a CTA's shared memory each.
@@ -1091,7 +1118,7 @@ extern "C" SGPU_API int sgpu_matrix_pcg_batch(sgpu_matrix m, int32_t nsys, const
     const int longest = m->csr.longest;
     const int64_t most = *std::max_element(rows.begin(), rows.end());
     int rc = kOther;
-    if (cluster_fits(longest, most) && cluster_runs(resident_grid()))
+    if (cluster_fits(longest, most) && cluster_pays(rows, mean, kNumSMs) && cluster_runs(resident_grid()))
       rc = run_cluster(m, rows, longest, w.x.p, w.f.p, ni, res, zero, hs, &its, &ms);
     if (rc == kOther)
       rc = run_persistent(m, rows, best.L, w.x.p, w.f.p, w.r.p, w.h.p, w.d.p, w.p.p, ni, res, zero, hs, &its, &ms);
