@@ -377,9 +377,12 @@ __global__ void __launch_bounds__(TPB, sizeof(T) == 4 && CPL <= 2 ? 4 : 1)
   op_finish<Op, CPL>(op, acc, partials, ticket, cols, R, ms);
 }
 
-// scalar CSR (warp per row)
+// scalar CSR (warp per row).  With one column a lane the latency of the gathers
+// takes all of an SM's warps to hide, so the registers of the sums at the end
+// are bounded by those of the product: 531,441 rows of 27 entries, 32 columns,
+// FP64 with p.q 326 us an application, 685 without the bound (48 registers).
 template <typename VT, typename T, int CPL, class Op>
-__global__ void __launch_bounds__(TPB) k_mspmm_csr(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
+__global__ void __launch_bounds__(TPB, CPL == 1 ? 8 : 1) k_mspmm_csr(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
                                                    const VT *__restrict__ val, const T *__restrict__ X, Op op,
                                                    MCol *cols, int R, MState *ms, double *partials,
                                                    unsigned *ticket) {
