@@ -625,31 +625,39 @@ __global__ void __launch_bounds__(TPB) k_lv_bsr3_tma(int nb, int cap_blocks, con
   op_reduce<Op>(op, acc, st, partials, ticket);
 }
 
-// level 0 in scalar CSR: L lanes per row.  FP64 has the gathers of U entries a
-// lane in flight and 4 lanes on short rows (2.69M rows of 18 entries 137 ->
-// 100 us, of which the bytes take 85); FP32, whose 4 lanes read half a sector
-// a step, keeps the other half in L1 (118 -> 104 us, bytes 57; 5 entries in
-// flight took 128).  Both read a row's bounds one row ahead.  A warp's entries
-// as one run through shared memory took 156 (FP32) and 244 us (FP64).
-template <typename T, int L, class Op>
+// level 0 in scalar CSR: L lanes per row (a lane's sum runs over its entries in
+// order in every form).  U: entries of a lane whose gathers are in flight
+// together; 1: one, the matrix streamed past L2; 0: one, the matrix cached.
+// All but 1 read a row's bounds one row ahead.  launch_lv_csr has the rule.  A
+// warp's entries as one run through shared memory took 156 (FP32, 2.69M rows of
+// 18 entries, 104 as it is) and 244 us (FP64, 100).
+template <typename T, int L, class Op, int U>
 __global__ void __launch_bounds__(TPB) k_lv_csr(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
                                                 const T *__restrict__ val, const T *__restrict__ v, Op op,
                                                 PcgState *st, double *partials, unsigned *ticket) {
   if (st->done) return;
-  constexpr int GPW = 32 / L, U = L == 4 ? 5 : 4;
+  constexpr int GPW = 32 / L;
   const int lane = threadIdx.x & 31, g = lane / L, sub = lane % L;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   double acc[Op::NV > 0 ? Op::NV : 1] = {};
   int b_next = 0, e_next = 0;  // a row's bounds are on their way while the row before is multiplied
-  if (warp * GPW + g < n) b_next = __ldg(rowptr + warp * GPW + g), e_next = __ldg(rowptr + warp * GPW + g + 1);
+  if (U != 1 && warp * GPW + g < n)
+    b_next = __ldg(rowptr + warp * GPW + g), e_next = __ldg(rowptr + warp * GPW + g + 1);
   for (int base = warp * GPW; base < n; base += nwarps * GPW) {
-    const int i = base + g, b = b_next, e = e_next;
+    const int i = base + g;
+    int b = b_next, e = e_next;
     b_next = e_next = 0;
-    if (i + nwarps * GPW < n) b_next = __ldg(rowptr + i + nwarps * GPW), e_next = __ldg(rowptr + i + nwarps * GPW + 1);
+    if (U == 1) {
+      if (i < n) b = __ldg(rowptr + i), e = __ldg(rowptr + i + 1);
+    } else if (i + nwarps * GPW < n) {
+      b_next = __ldg(rowptr + i + nwarps * GPW), e_next = __ldg(rowptr + i + nwarps * GPW + 1);
+    }
     T s = 0;
-    if constexpr (sizeof(T) == 4) {
+    if constexpr (U == 0) {
       for (int k = b + sub; k < e; k += L) s += __ldg(val + k) * __ldg(v + __ldg(col + k));
+    } else if constexpr (U == 1) {
+      for (int k = b + sub; k < e; k += L) s += __ldcs(val + k) * __ldg(v + __ldcs(col + k));
     } else {
       for (int k = b + sub; k < e; k += L * U) {
         int c[U];
@@ -3746,6 +3754,44 @@ void launch_bsrb(const AmgLevel &L, const T *val, const T *v, const Op &op, cuda
   k<<<resident_grid(k, L.nb), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk);
 }
 
+// A product with level 0 in scalar CSR.  Us for the two products of a cycle,
+// form taken / other:
+//   FP64: gathers in flight where a lane has three entries and more of a row.
+//     531,441 rows of 27: 4 lanes 75 / 84 (one at a time), 8 lanes 81 / 100, 16
+//     lanes 119 / 131 (four), 32 lanes 168 / 214; 2M rows of 18: 4 lanes 211 /
+//     236, 8 lanes 259 / 294; 501,000 of 14: 8 lanes 64 / 75.
+//   FP32: the other half of the sector that 4 lanes read stays in L1 where the
+//     matrix is cached; at about the size of L2 the cached matrix drives out
+//     the vectors, which shows on long rows.  4 lanes, rows of 27: 57 MB 28.7 /
+//     34.2, 111 MB 60.0 / 64.4 (cached), 191 MB 102 / 104, 456 MB 210 / 241; of
+//     18: 122 MB 73.6 / 77.2.
+template <typename T, class Op>
+void launch_lv_csr(int lanes, int n, int64_t nnz, const int *rowptr, const int *col, const T *val, const T *v,
+                   const Op &op, cudaStream_t s, PcgState *st, double *part, unsigned *tk) {
+  auto launch = [&](auto k, int rows) {
+    k<<<resident_grid(k, (n + rows - 1) / rows), TPB, 0, s>>>(n, rowptr, col, val, v, op, st, part, tk);
+  };
+  const bool long_rows = nnz >= (int64_t)24 * n;
+  if constexpr (sizeof(T) == 8) {
+    if (lanes == 32) launch(k_lv_csr<T, 32, Op, 1>, 1);
+    else if (lanes == 16) launch(k_lv_csr<T, 16, Op, 1>, 2);
+    else if (lanes == 4) launch(k_lv_csr<T, 4, Op, 5>, 8);
+    else if (long_rows) launch(k_lv_csr<T, 8, Op, 4>, 4);
+    else launch(k_lv_csr<T, 8, Op, 1>, 4);
+  } else {
+    const double bytes = 8.0 * (double)nnz;
+    if (long_rows && bytes > 85e6 && bytes < 150e6) {
+      if (lanes == 32) launch(k_lv_csr<T, 32, Op, 1>, 1);
+      else if (lanes == 16) launch(k_lv_csr<T, 16, Op, 1>, 2);
+      else if (lanes == 4) launch(k_lv_csr<T, 4, Op, 1>, 8);
+      else launch(k_lv_csr<T, 8, Op, 1>, 4);
+    } else if (lanes == 32) launch(k_lv_csr<T, 32, Op, 0>, 1);
+    else if (lanes == 16) launch(k_lv_csr<T, 16, Op, 0>, 2);
+    else if (lanes == 4) launch(k_lv_csr<T, 4, Op, 0>, 8);
+    else launch(k_lv_csr<T, 8, Op, 0>, 4);
+  }
+}
+
 template <typename T, class Op>
 int launch_level(sgpu_matrix m, const AmgLevel &L, const T *v, const Op &op, cudaStream_t s, int slot) {
   PcgState *st = pcg_state(m);
@@ -3774,20 +3820,7 @@ int launch_level(sgpu_matrix m, const AmgLevel &L, const T *v, const Op &op, cud
       k<<<resident_grid(k, (L.nb + 3) / 4), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk);
     }
   } else if (L.layout == 2) {
-    const int lanes = level0_lanes(m, sizeof(T) == 4);
-    if (lanes == 32) {
-      auto k = k_lv_csr<T, 32, Op>;
-      k<<<resident_grid(k, L.nb), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk);
-    } else if (lanes == 16) {
-      auto k = k_lv_csr<T, 16, Op>;
-      k<<<resident_grid(k, (L.nb + 1) / 2), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk);
-    } else if (lanes == 4) {
-      auto k = k_lv_csr<T, 4, Op>;
-      k<<<resident_grid(k, (L.nb + 7) / 8), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk);
-    } else {
-      auto k = k_lv_csr<T, 8, Op>;
-      k<<<resident_grid(k, (L.nb + 3) / 4), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk);
-    }
+    launch_lv_csr<T>(level0_lanes(m, sizeof(T) == 4), L.nb, m->csr.nnz, L.browptr, L.bcol, val, v, op, s, st, part, tk);
   } else {
     if (record_level(m, L, v, op)) return SGPU_OK;
     switch (L.b) {
@@ -4823,13 +4856,8 @@ int batch_spmv64(sgpu_matrix m, const double *p, double *q, double *prod, cudaSt
                                                   st, m->w.partials.p, m->w.counters.p);
   } else {
     // 4 lanes on rows of up to 5 entries a lane, which all are in flight then
-    auto launch = [&](auto k, int rows) {
-      k<<<resident_grid(k, (m->n + rows - 1) / rows), TPB, 0, s>>>((int)m->n, m->csr.rowptr.p, m->csr.col.p,
-                                                                   m->csr.val.p, p, op, st, m->w.partials.p,
-                                                                   m->w.counters.p);
-    };
-    if (m->csr.nnz <= (int64_t)20 * m->n) launch(k_lv_csr<double, 4, OpStorePQ>, 8);
-    else launch(k_lv_csr<double, 8, OpStorePQ>, 4);
+    launch_lv_csr<double>(m->csr.nnz <= (int64_t)20 * m->n ? 4 : 8, (int)m->n, m->csr.nnz, m->csr.rowptr.p, m->csr.col.p,
+                          m->csr.val.p, p, op, s, st, m->w.partials.p, m->w.counters.p);
   }
   count_launches(1);
   SGPU_CUDA(cudaGetLastError());
