@@ -830,7 +830,7 @@ __global__ void __launch_bounds__(TPB) k_dense_mv(int nc, const T *__restrict__ 
 // Below level 0 a W-cycle is a chain of small dependent steps (smoothing,
 // residual, restriction, dense solve, prolongation): 31 on the 1.01M-equation
 // cantilever, 156 on a batch of plates with five levels, most of them a
-// microsecond of work.  Where level 1 is small (kProgLevelBytes) they run as a
+// microsecond of work.  Where level 1 is small (program_rows) they run as a
 // program -- the list of steps that the cycle would have launched, with
 // their arrays -- inside one cooperative launch of a CTA per SM, a grid
 // barrier (1.25 us) between two steps.  Every row is computed with the loop
@@ -3727,24 +3727,34 @@ int level0_lanes(const sgpu_matrix m, bool fp32) {
   return v;
 }
 
-// The largest level-1 matrix that a program takes.  A graph's kernels follow
-// one another about as fast as a grid barrier opens, so a program gains only
-// where the steps are short; a large level's steps run longer in one CTA per
-// SM than in the separate kernels' grids.  Measured whole solves: 129,480
-// equations (level 1 of 16 MB, FP64) 9.3 -> 8.9 ms; the 1.01M-equation
-// cantilever (57 MB) and 256 plates (41 MB) unchanged where only their deeper
-// levels ran as programs, slower (0.80 against 0.60 ms a cycle) with level 1.
-constexpr double kProgLevelBytes = 20e6;
+// The most block rows of b that level 1 has where it starts a program.  A
+// graph's kernels follow one another about as fast as a grid barrier opens, so
+// a program gains only where the steps are short; a program has 16 warps an SM
+// (FP64; 32 in FP32), the kernels 64, and each row of a step waits for its own
+// gathers.  An iteration with kernels / with the program, us, by level 1's rows:
+//   FP64, 1 x 1  1561 79.1 / 73.3, 3009 86.6 / 88.1, 22,271 251 / 284
+//   FP64, 3 x 3  1337 85.6 / 72.2, 8170 156 / 152, 11,803 220 / 221, 25,056 297 / 331
+//   FP64, 6 x 6  1994 192 / 176, 3049 240 / 222, 5139 354 / 353
+//   FP32, 1 x 1  1561 71.9 / 67.1, 3009 77.0 / 75.9, 5055 83.4 / 91.1
+//   FP32, 3 x 3  483 65.7 / 61.8, 5278 127 / 125, 11,803 154 / 160
+//   FP32, 6 x 6  250 66.1 / 66.2, 1994 149 / 151, 2039 (tetrahedra) 126 / 131
+template <typename T>
+int program_rows(int b) {
+  if (b == 1) return 2500;
+  if (b == 3) return sizeof(T) == 8 ? 8000 : 6500;
+  return b == 6 && sizeof(T) == 8 ? 4500 : 0;
+}
 
 // A coarse level's product: a warp per block row, or 8 lanes where a row has
 // few blocks (plane problems: 9, which leave 23 lanes of a warp idle) and the
-// level is too large to be a step of a program, whose rows a warp sums.  256
-// plates (level 1 of 41 MB) 59.4 ms with a warp, 55.5 with 8 lanes.
+// level is large (far beyond a program's, whose rows a warp sums).  256 plates
+// (level 1 of 41 MB) 59.4 ms with a warp, 55.5 with 8 lanes.
+constexpr double kWideLevelBytes = 20e6;
 template <typename T, int B, class Op>
 void launch_bsrb(const AmgLevel &L, const T *val, const T *v, const Op &op, cudaStream_t s, PcgState *st, double *part,
                  unsigned *tk) {
   if constexpr (B <= 3) {
-    if (L.nblk <= (int64_t)12 * L.nb && (double)L.nblk * B * B * sizeof(T) > kProgLevelBytes) {
+    if (L.nblk <= (int64_t)12 * L.nb && (double)L.nblk * B * B * sizeof(T) > kWideLevelBytes) {
       auto k = k_lv_bsrb<T, B, Op, 8>;
       k<<<resident_grid(k, (L.nb + 3) / 4), TPB, 0, s>>>(L.nb, L.browptr, L.bcol, val, v, op, st, part, tk);
       return;
@@ -4424,7 +4434,9 @@ cudaError_t launch_program_b(sgpu_matrix m, const CoarseProgram &p, cudaStream_t
 }
 template <typename T>
 cudaError_t launch_program(sgpu_matrix m, const CoarseProgram &p, cudaStream_t s) {
-  if (p.block == 6) return launch_program_b<T, 6>(m, p, s);
+  if constexpr (sizeof(T) == 8) {
+    if (p.block == 6) return launch_program_b<T, 6>(m, p, s);
+  }
   if (p.block == 3) return launch_program_b<T, 3>(m, p, s);
   return launch_program_b<T, 1>(m, p, s);
 }
@@ -4460,8 +4472,7 @@ int coarse_program(sgpu_matrix m, int l, int visits, const std::vector<Cheb> &ch
     const AmgLevel &C = *A.lv[l];
     p.current = true;
     p.nsteps = 0;
-    if ((double)C.nblk * C.b * C.b * sizeof(T) > kProgLevelBytes) return SGPU_OK;
-    bool uniform = C.b == 1 || C.b == 3 || C.b == 6;
+    bool uniform = C.nb <= program_rows<T>(C.b);
     for (size_t q = l; q < A.lv.size(); q++)
       uniform = uniform && A.lv[q]->layout == 0 && A.lv[q]->b == C.b && (A.lv[q]->k == C.b || A.lv[q]->k == 0);
     p.grid = ::sgpu::resident_grid();
