@@ -2486,6 +2486,10 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
       return bail(st);                    \
     }                                     \
   } while (0)
+  auto to_device = [&](auto *dst, const void *src, int64_t count) -> int {
+    const cudaError_t e = copy_in(dst, src, (size_t)count * sizeof(*dst), s);
+    return e == cudaSuccess ? SGPU_OK : fail(SGPU_CUDA_ERROR, std::string("copy of the mesh: ") + cudaGetErrorString(e));
+  };
   BAIL_ON(ad.coords.alloc(nn * 3));
   BAIL_ON(ad.elems.alloc(ne * nne));
   ad.general = mesh->dmat != nullptr;
@@ -2494,17 +2498,17 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   DevBuf<int64_t> cn_d;
   BAIL_ON(cn_d.alloc(nn * ndofn));
   BAIL_ON(ad.cne.alloc(ne * ndofe));
-  copy_in(ad.coords.p, mesh->coords, nn * 3 * sizeof(double), s);
-  copy_in(ad.elems.p, mesh->elems, ne * nne * sizeof(int64_t), s);
-  copy_in(ad.emat.p, ad.general ? mesh->dmat : mesh->emat, ne * nmatp * sizeof(double), s);
-  copy_in(cn_d.p, mesh->cn, nn * ndofn * sizeof(int64_t), s);
+  BAIL_ON(to_device(ad.coords.p, mesh->coords, nn * 3));
+  BAIL_ON(to_device(ad.elems.p, mesh->elems, ne * nne));
+  BAIL_ON(to_device(ad.emat.p, ad.general ? mesh->dmat : mesh->emat, ne * nmatp));
+  BAIL_ON(to_device(cn_d.p, mesh->cn, nn * ndofn));
   if (mesh->thick) {
     BAIL_ON(ad.thick.alloc(ne));
-    copy_in(ad.thick.p, mesh->thick, ne * sizeof(double), s);
+    BAIL_ON(to_device(ad.thick.p, mesh->thick, ne));
   }
   if (mesh->rho) {
     BAIL_ON(ad.rho.alloc(ne));
-    copy_in(ad.rho.p, mesh->rho, ne * sizeof(double), s);
+    BAIL_ON(to_device(ad.rho.p, mesh->rho, ne));
   }
   DevBuf<unsigned> err;
   BAIL_ON(err.alloc(1));
@@ -2599,7 +2603,8 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   // the per-colour element lists
   if (const char *why = colouring.finish(nn, ne, nne, mesh->elems, ad)) return bail(fail(SGPU_BAD_INPUT, why));
   if (ad.elist.alloc(ne) != SGPU_OK) return bail(SGPU_CUDA_ERROR);
-  copy_in(ad.elist.p, ad.order.data(), ne * sizeof(int), s);
+  st = to_device(ad.elist.p, ad.order.data(), ne);
+  if (st != SGPU_OK) return bail(st);
   float asm_ms = 0.f;
   st = assemble_values(m, ad, kind, &asm_ms);
   if (st != SGPU_OK) return bail(st);

@@ -102,8 +102,8 @@ struct DevIdle {
 // Copies between a caller's host array and the device, ordered on s
 // (sgpu_transfer.cu).  As with cudaMemcpyAsync, a pageable array may be reused
 // (copy_in) or holds the result (copy_out) on return.
-cudaError_t copy_in(void *dst, const void *src, size_t bytes, cudaStream_t s);
-cudaError_t copy_out(void *dst, const void *src, size_t bytes, cudaStream_t s);
+[[nodiscard]] cudaError_t copy_in(void *dst, const void *src, size_t bytes, cudaStream_t s);
+[[nodiscard]] cudaError_t copy_out(void *dst, const void *src, size_t bytes, cudaStream_t s);
 
 template <class T>
 struct DevBuf {

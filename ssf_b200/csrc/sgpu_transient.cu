@@ -119,14 +119,14 @@ int transient(sgpu_matrix K, sgpu_matrix C, const double *rhs, double *d, double
   cudaStream_t c_stream_saved = C->stream, k_stream_saved = K->stream;
   C->stream = s;  // C's (d-form) or K's (v-form) products run on A's stream for ordering
   K->stream = s;
-  copy_in(d_d.p, d, n * sizeof(double), s);
-  copy_in(v_d.p, v, n * sizeof(double), s);
-  copy_in(rhs_d.p, rhs, n * sizeof(double), s);
+  if (copy_in(d_d.p, d, n * sizeof(double), s) != cudaSuccess || copy_in(v_d.p, v, n * sizeof(double), s) != cudaSuccess ||
+      copy_in(rhs_d.p, rhs, n * sizeof(double), s) != cudaSuccess)
+    st = fail(SGPU_CUDA_ERROR, "copy of the start vectors failed");
   const int vb = blocks_for(n);
   int64_t total_its = 0;
   double total_ms = 0.0, last_true = 0.0, setup_ms = 0.0;
   int32_t levels = 0, coarse_n = 0;
-  for (int64_t step = 0; step < nsteps; step++) {
+  for (int64_t step = 0; st == SGPU_OK && step < nsteps; step++) {
     k_predict<<<vb, TPB, 0, s>>>((int)n, d_d.p, v_d.p, (1.0 - alpha) * dt, dd_d.p);
     count_launches(1);
     if (vform) {
@@ -169,9 +169,9 @@ int transient(sgpu_matrix K, sgpu_matrix C, const double *rhs, double *d, double
   C->stream = c_stream_saved;
   K->stream = k_stream_saved;
   if (st != SGPU_OK) return cleanup(st);
-  copy_out(d, d_d.p, n * sizeof(double), s);
-  copy_out(v, v_d.p, n * sizeof(double), s);
-  if (cudaStreamSynchronize(s) != cudaSuccess) return cleanup(fail(SGPU_CUDA_ERROR, "transient copy-back failed"));
+  if (copy_out(d, d_d.p, n * sizeof(double), s) != cudaSuccess || copy_out(v, v_d.p, n * sizeof(double), s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess)
+    return cleanup(fail(SGPU_CUDA_ERROR, "transient copy-back failed"));
   if (info) {
     info->iterations = total_its;
     info->solve_ms = total_ms;

@@ -2,6 +2,7 @@
 which stream, and what a call that fails leads to.  No device is needed."""
 import ctypes as C
 import os
+import re
 import subprocess
 
 import numpy as np
@@ -59,3 +60,37 @@ def test_every_piece_lands_on_the_callers_stream(host, copies, stream, n):
         assert fn(dst.ctypes.data, src.ctypes.data, 8 * n, stream) == 0
         assert np.array_equal(dst, src)
     assert stream != PER_THREAD or host.fake_foreign_copies(C.c_void_p(stream)) == 0
+
+
+@pytest.mark.parametrize("call", ["cudaMemcpyAsync", "cudaEventRecord", "cudaEventSynchronize", "cudaSetDevice"])
+@pytest.mark.parametrize("k", [1, 3, 7])
+def test_one_failing_call_of_a_copy(host, copies, call, k):
+    """A piece that fails sends the whole array once more, the plain way."""
+    for fn in copies:
+        host.fake_reset()
+        src, dst = np.random.default_rng(k).standard_normal(LARGE), np.zeros(LARGE)
+        host.fake_fail(call.encode(), k)
+        assert fn(dst.ctypes.data, src.ctypes.data, 8 * LARGE, 0x1000) == 0
+        assert np.array_equal(dst, src)
+
+
+@pytest.mark.parametrize("n", [1, LARGE])
+def test_a_copy_that_keeps_failing_says_so(host, copies, n):
+    for fn in copies:
+        host.fake_reset()
+        src, dst = np.ones(n), np.zeros(n)
+        host.fake_fail(b"cudaMemcpyAsync", 0)
+        assert fn(dst.ctypes.data, src.ctypes.data, 8 * n, 0x1000) != 0
+
+
+def test_no_copy_goes_unchecked():
+    """The result of a copy of the caller's arrays is used wherever one is made."""
+    found = 0
+    for name in sorted(os.listdir(os.path.join(ROOT, "ssf_b200", "csrc"))):
+        with open(os.path.join(ROOT, "ssf_b200", "csrc", name)) as f:
+            text = "".join(line.split("//")[0] for line in f)
+        for at in re.finditer(r"\bcopy_(in|out)\(", text):
+            before = text[:at.start()].rstrip()
+            found += 1
+            assert before[-1] not in ";{})", (name, text[at.start():at.start() + 60])
+    assert found > 20
