@@ -104,7 +104,14 @@ int upload(sgpu_matrix m, const int64_t *adr, const int64_t *ci, const double *a
   SGPU_CUDA(copy_in(m->src_ci.p, ci, negm * sizeof(int64_t), s));
   ValueCopy side;
   const size_t bytes = (size_t)negm * sizeof(double);
-  bool aside = bytes >= kAside && cudaStreamCreateWithFlags(&side.s2, cudaStreamNonBlocking) == cudaSuccess;
+  bool aside = false;
+  if (bytes >= kAside) {
+    aside = cudaStreamCreateWithFlags(&side.s2, cudaStreamNonBlocking) == cudaSuccess;
+    if (!aside) {
+      cudaGetLastError();
+      side.s2 = nullptr;
+    }
+  }
   if (aside) {
     int dev = 0;
     SGPU_CUDA(cudaGetDevice(&dev));

@@ -94,3 +94,23 @@ def test_no_copy_goes_unchecked():
             found += 1
             assert before[-1] not in ";{})", (name, text[at.start():at.start() + 60])
     assert found > 20
+
+
+def test_a_side_stream_that_is_not_to_be_had(host):
+    """The values then take the handle's own stream, and no error stays behind for the next check of a launch."""
+    n = 400000  # 3.2 MB of values: from 2 MB on they take a stream of their own
+    adr, ci, a = np.arange(n + 1, dtype=np.int64), np.arange(n, dtype=np.int64), np.ones(n)
+    create = host.sgpu_matrix_create
+    create.argtypes = [C.c_int64] + [C.c_void_p] * 3 + [C.c_int32, C.c_void_p]
+    for k in (0, 1, 2, 3):
+        host.fake_reset()
+        if k:
+            host.fake_fail(b"cudaStreamCreateWithFlags", k)
+        h = C.c_void_p()
+        st = create(n, adr.ctypes.data, ci.ctypes.data, a.ctypes.data, 0, C.byref(h))
+        if k == 1:  # the handle's own stream
+            assert st == 4 and not h.value
+            continue
+        assert st == 0 and h.value
+        assert host.fake_last_error() == 0
+    host.fake_reset()
