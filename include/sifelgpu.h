@@ -69,8 +69,12 @@ typedef struct {
   double setup_ms;          /* upload + format conversion, device timed */
   double solve_ms;          /* iteration, device timed */
   double spmv_bytes;        /* algorithmic bytes of one SpMV of the iteration's format */
-  int32_t spmv_format;      /* 0 = CSR, 3 = 3x3 block rows (BSR3) */
-  int32_t spmv_variant;     /* autotuned kernel variant id */
+  int32_t spmv_format;      /* matrix format of the iteration: 0 = CSR, 2 = sliced ELL, 3 = 3x3 block rows (BSR3) */
+  int32_t spmv_variant;     /* how the iteration multiplied with it.  FP64 Jacobi and unpreconditioned solves in one
+                               launch: the lanes that share a row (CSR: 2, 8 or 32) or block row (8, 16 or 32) of a
+                               matrix streamed through shared memory, 0 where it stays there.  Uneven batches: the
+                               lanes of a row.  Otherwise the tuned kernel's id, as sgpu_matrix_set_spmv takes it
+                               (which makes such solves use that kernel, in launches of their own) */
   int32_t fallback;         /* MIXED: 1 if the FP32 iteration stagnated and the
                                solve was finished in FP64 from its iterate */
   int32_t tile_rows;        /* batched solves: rows per work segment picked by the tuner */

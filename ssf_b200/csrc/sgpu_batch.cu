@@ -1120,6 +1120,7 @@ extern "C" SGPU_API int sgpu_matrix_pcg_batch(sgpu_matrix m, int32_t nsys, const
     int rc = kOther;
     if (cluster_fits(longest, most) && cluster_pays(rows, mean, kNumSMs) && cluster_runs(resident_grid()))
       rc = run_cluster(m, rows, longest, w.x.p, w.f.p, ni, res, zero, hs, &its, &ms);
+    if (rc == SGPU_OK) best.L = CluTile::kLpr;
     if (rc == kOther)
       rc = run_persistent(m, rows, best.L, w.x.p, w.f.p, w.r.p, w.h.p, w.d.p, w.p.p, ni, res, zero, hs, &its, &ms);
     if (rc != SGPU_OK) return rc;

@@ -3,6 +3,8 @@
 
 Systems have condition below 4 (`banded`): a residual of 1e-10 bounds the error by 4e-10; 1e-9 is asserted.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -61,3 +63,16 @@ def test_iteration_limit(gpu_lib, rows):
             assert st[k] == L.OK and its[k] == ani[k] + 1 <= 2
         else:
             assert st[k] == L.NOT_CONVERGED and its[k] == 2 and ani[k] == -1
+
+
+@pytest.mark.parametrize("name", ["many_small", "few_of_2048", "beyond_a_cluster"])
+def test_report_names_the_lanes_that_ran(gpu_lib, name):
+    rows, offsets, clusters = BATCHES[name]
+    rp, col, val = batch(rows, offsets)
+    f, info = np.ones(sum(rows)), L.SolveInfo()
+    mean = val.size / f.size
+    with DeviceMatrix(rp, col, val, 0) as K:
+        rc = gpu_lib.sgpu_matrix_pcg_batch(K.h, len(rows), np.array(rows, dtype=np.int64), np.empty_like(f), f, 2, 1e-20,
+                                           1e-30, 0, None, None, None, None, C.byref(info))
+    assert rc == L.NOT_CONVERGED and info.spmv_format == 0
+    assert info.spmv_variant == (2 if clusters else 8 if mean > 12 else 4)
