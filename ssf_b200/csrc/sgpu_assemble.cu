@@ -2516,17 +2516,27 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   k_elem_codes<<<blocks_for(ne * ndofe), TPB, 0, s>>>(ne, nne, ndofn, ad.elems.p, cn_d.p, ad.cne.p, err.p, nn);
   count_launches(1);
   // are the code numbers gencodnum's (consecutive in node, component order)?
-  // Then their count is the number of equations.
+  // Then their count is the number of equations; else it is the largest one,
+  // fewer than the positive ones where nodes share equations.  The device
+  // counts up to 2^31 of them.
   const int64_t ncode = nn * ndofn;
-  if (ncode > (1LL << 31) - 2) return bail(fail(SGPU_BAD_INPUT, "too many nodes"));
+  const bool counted = ncode <= (1LL << 31) - 2;
   DevBuf<int> code;
-  BAIL_ON(code.alloc(ncode));
-  int nfree = 0;
-  unsigned flags = 0;
-  BAIL_ON(examine_codes(cn_d.p, ncode, ndofn, code.p, err.p, &nfree, &flags, s));
+  int64_t nfree = 0;
+  unsigned flags = 32u;
+  if (counted) {
+    int free32 = 0;
+    BAIL_ON(code.alloc(ncode));
+    BAIL_ON(examine_codes(cn_d.p, ncode, ndofn, code.p, err.p, &free32, &flags, s));
+    nfree = free32;
+  } else {
+    BAIL_ON(read_err(err.p, s, &flags));
+    flags |= 32u;
+    for (int64_t q = 0; q < ncode; q++) nfree += mesh->cn[q] > 0;
+  }
   const bool monotone = !(flags & 32u);
   int64_t n = nfree;
-  if (!monotone) {  // the largest code number: fewer than the positive ones where nodes share equations
+  if (!monotone) {
     n = 0;
     for (int64_t q = 0; q < ncode; q++) n = std::max<int64_t>(n, mesh->cn[q]);
   }
