@@ -222,12 +222,12 @@ SGPU_API int sgpu_matrix_pcg_multi_agg(sgpu_matrix m, int32_t nrhs, double *X, c
 
 /* Many independent systems of uneven size (the diagonal blocks of m, in
  * order; sys_rows[k] equations each, summing to n) solved together: every
- * system its own Jacobi-PCG with the criterion of symcomprow::cg_prec, all
- * advanced by the same kernels (one block-diagonal SpMV and two vector
- * kernels per iteration, captured in a CUDA graph and relaunched until every
- * system has stopped); converged systems drop out of the work.  tune != 0
- * first times a few iterations with each segment size / lanes-per-row pair
- * and keeps the fastest.  x: n (host, out; the iteration starts from 0);
+ * system its own Jacobi-PCG with the criterion of symcomprow::cg_prec, in one
+ * launch in which a cluster of eight SMs or one CTA runs a system to its end.
+ * (SGPU_BATCH_FORM=graph: one block-diagonal SpMV and two vector kernels per
+ * iteration, relaunched until every system has stopped; tune != 0 then first
+ * times a few iterations with each segment size / lanes-per-row pair and keeps
+ * the fastest.)  x: n (host, out; the iteration starts from 0);
  * f: n; per system ani/ares (reference conventions), status and iterations
  * (arrays of nsys, may be NULL). */
 SGPU_API int sgpu_matrix_pcg_batch(sgpu_matrix m, int32_t nsys, const int64_t *sys_rows, double *x,
@@ -240,7 +240,7 @@ SGPU_API int sgpu_matrix_pcg_batch(sgpu_matrix m, int32_t nsys, const int64_t *s
  * ani/ares per system) while the hierarchy of the whole block-diagonal
  * matrix -- whose aggregates never cross systems -- is shared, so every
  * cycle kernel runs once for all systems; per-system sums are formed from
- * per-row products in row order.  mode: SGPU_MIXED (FP32 cycle) or
+ * per-row products in a fixed order.  mode: SGPU_MIXED (FP32 cycle) or
  * SGPU_FP64.  The near-null space comes from sgpu_matrix_set_nullspace on m
  * (e.g. every plate's rigid-body modes).  x starts from 0. */
 SGPU_API int sgpu_matrix_pcg_batch_agg(sgpu_matrix m, int32_t nsys, const int64_t *sys_rows, double *x,

@@ -2202,9 +2202,9 @@ struct AssemblyData {
   bool tied = false;  // several (node, component) pairs have one equation
 };
 
-// The colouring (3 ms for 320,000 elements, one after the other by its
-// definition) in a thread of its own beside the copies and the pattern's
-// construction; joined before its lists are read and on every way out.
+// The colouring (3 ms for 320,000 elements, one after the other on the host) in
+// a thread of its own beside the copies and the pattern's construction; joined
+// before its lists are read and on every way out.
 struct Colouring {
   std::thread t;
   const char *error = nullptr;

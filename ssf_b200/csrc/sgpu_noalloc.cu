@@ -61,8 +61,10 @@ namespace {
 constexpr int kTPB = 256;
 constexpr int kMaxN = SGPU_NOALLOC_MAX_N;
 constexpr int kBlocks = 148 * 4;  // grid of the input check and of the general form
-// iterations of one launch, between two reads of the state: under 50 ms at
-// the largest size, and few enough waits that they cost nothing
+// iterations of one launch, between two reads of the state: 17 ms on a plate of
+// 101,404 equations, 58 ms where three quarters of 8M entries are read from
+// global memory each time, longer with more; few enough waits that they cost
+// nothing
 constexpr long long kChunk = 2048;
 constexpr int kGeneralChunk = 16;  // the same of the general form
 
