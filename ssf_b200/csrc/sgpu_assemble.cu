@@ -2132,7 +2132,8 @@ int examine_codes(const int64_t *cn_d, int64_t ncode, int ndofn, int *code_d, un
 // neighbours (the caller uses the element-pair sort instead).  The rows are
 // symmetric and complete, so the SCR form (and the maps from it, built when
 // values arrive in its order) follow from them; node_blocked says that every
-// node is free or fixed as a whole.
+// node is free or fixed as a whole.  err_d: the error bits and, zero before,
+// the longest row.
 int pattern_adjacency(sgpu_matrix m, const int64_t *elems_d, const int *code_d, int64_t nn, int64_t ne, int nne,
                       int ndofn, int64_t n, const int *iptr_d, const int *inc_d, unsigned *err_d, bool node_blocked,
                       cudaStream_t s) {
@@ -2143,13 +2144,12 @@ int pattern_adjacency(sgpu_matrix m, const int64_t *elems_d, const int *code_d, 
   SGPU_TRY(nadj.alloc((size_t)ne * nne * nne));
   SGPU_CUDA(cudaMemsetAsync(len.p + nn, 0, sizeof(int), s));
   const int gadj = (int)std::min<int64_t>((nn + WPB - 1) / WPB, (int64_t)kNumSMs * 32);
-  AsyncBuf<int64_t> total(s);  // the row lengths may add up past int32; and the longest row
-  SGPU_TRY(total.alloc(2));
-  SGPU_CUDA(cudaMemsetAsync(total.p, 0, 2 * sizeof(int64_t), s));
   k_node_adj<<<gadj, TPB, 0, s>>>(nn, nne, ndofn, elems_d, iptr_d, inc_d, code_d, cnt.p, len.p, nadj.p, err_d,
-                                  reinterpret_cast<int *>(total.p + 1));
+                                  reinterpret_cast<int *>(err_d + 1));
   count_launches(1);
+  AsyncBuf<int64_t> total(s);  // the row lengths may add up past int32
   {
+    SGPU_TRY(total.alloc(1));
     size_t tmp = 0;
     cub::DeviceReduce::Reduce(nullptr, tmp, len.p, total.p, (int)nn, cuda::std::plus<int64_t>(), (int64_t)0, s);
     AsyncBuf<unsigned char> t(s);
@@ -2158,20 +2158,20 @@ int pattern_adjacency(sgpu_matrix m, const int64_t *elems_d, const int *code_d, 
     count_launches(1);
   }
   SGPU_TRY(scan_into(len.p, row0.p, nn, s));
-  int64_t sums[2] = {0, 0};
-  SGPU_CUDA(cudaMemcpyAsync(sums, total.p, sizeof(sums), cudaMemcpyDeviceToHost, s));
-  unsigned e = 0;
-  SGPU_TRY(read_err(err_d, s, &e));
-  if (e & 16u) {
+  int64_t nnz = 0;
+  unsigned e[2] = {0, 0};  // error bits, longest row
+  SGPU_CUDA(cudaMemcpyAsync(&nnz, total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  SGPU_CUDA(cudaMemcpyAsync(e, err_d, sizeof(e), cudaMemcpyDeviceToHost, s));
+  SGPU_CUDA(cudaStreamSynchronize(s));
+  if (e[0] & 16u) {
     SGPU_CUDA(cudaMemsetAsync(err_d, 0, sizeof(unsigned), s));
     return 1;
   }
-  if (e & 3u) return fail(SGPU_BAD_INPUT, "code numbers: element node out of range or unused equation");
-  const int64_t nnz = sums[0];
+  if (e[0] & 3u) return fail(SGPU_BAD_INPUT, "code numbers: element node out of range or unused equation");
   if (nnz >= (1LL << 31) - 1) return fail(SGPU_BAD_INPUT, "matrix too large for int32 device indices");
   Csr &c = m->csr;
   SGPU_TRY(matrix_alloc_csr(m, n, nnz));
-  c.longest = (int)sums[1];
+  c.longest = (int)e[1];
   m->src_negm = (nnz + n) / 2;
   k_csr_fill<<<(int)std::min<int64_t>((nn + WPB - 1) / WPB, (int64_t)kNumSMs * 64), TPB, 0, s>>>(
       nn, nne, ndofn, iptr_d, code_d, cnt.p, len.p, row0.p, nadj.p, c.rowptr.p, c.col.p, (int)n);
@@ -2510,8 +2510,8 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
     BAIL_ON(ad.rho.alloc(ne));
     BAIL_ON(to_device(ad.rho.p, mesh->rho, ne));
   }
-  DevBuf<unsigned> err;
-  BAIL_ON(err.alloc(1));
+  DevBuf<unsigned> err;  // error bits; the longest row (pattern_adjacency)
+  BAIL_ON(err.alloc(2));
   cudaMemsetAsync(err.p, 0, sizeof(unsigned), s);
   k_elem_codes<<<blocks_for(ne * ndofe), TPB, 0, s>>>(ne, nne, ndofn, ad.elems.p, cn_d.p, ad.cne.p, err.p, nn);
   count_launches(1);
@@ -2545,7 +2545,7 @@ SGPU_API int sgpu_assemble(const sgpu_mesh *mesh, sgpu_matrix *out, sgpu_assembl
   if (n >= (1LL << 31) - 1) return bail(fail(SGPU_BAD_INPUT, "n out of range for int32 device indices"));
   m->n = n;
   ad.tied = n < nfree;
-  cudaMemsetAsync(err.p, 0, sizeof(unsigned), s);
+  cudaMemsetAsync(err.p, 0, 2 * sizeof(unsigned), s);
 
   // pattern: from the node adjacency when the code numbers are gencodnum's,
   // else (or for a node of very high valence) lower-triangle element pairs ->

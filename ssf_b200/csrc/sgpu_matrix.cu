@@ -70,10 +70,12 @@ __global__ void k_row_of(int64_t n, const int64_t *__restrict__ adr, int *__rest
   }
 }
 
-// len[i]: entries of full row i; len[n] (zero before): the most of any row
+// len[i]: entries of full row i (len[n] 0); longest (zero before): the most of
+// any row
 __global__ void k_full_len(int64_t n, const int64_t *__restrict__ adr, const int *__restrict__ upcnt,
-                           int *__restrict__ len, int sym) {
+                           int *__restrict__ len, int sym, int *longest) {
   int most = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) len[n] = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int l = (int)(adr[i + 1] - adr[i]) + (sym ? upcnt[i] : 0);
@@ -82,7 +84,7 @@ __global__ void k_full_len(int64_t n, const int64_t *__restrict__ adr, const int
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-  if ((threadIdx.x & 31) == 0 && most > *(volatile int *)(len + n)) atomicMax(len + n, most);
+  if ((threadIdx.x & 31) == 0 && most > *(volatile int *)longest) atomicMax(longest, most);
 }
 
 // lower part (and the diagonal) of every SCR row lands at the start of the
@@ -313,37 +315,32 @@ int matrix_build_from_device_src(sgpu_matrix m) {
   SGPU_CUDA(cudaMemcpy(&negm_chk, m->src_adr.p + n, sizeof(int64_t), cudaMemcpyDeviceToHost));
   if (negm_chk != negm) return fail(SGPU_BAD_INPUT, "adr[n] != number of entries");
 
+  // every row holds its diagonal
+  const int64_t nnz = sym ? 2 * negm - n : negm;
+  if (nnz >= (1LL << 31) - 1) return fail(SGPU_BAD_INPUT, "matrix too large for int32 device indices");
+
   DevBuf<int> row_of, upcnt, len;
   SGPU_TRY(row_of.alloc(negm));
-  SGPU_TRY(upcnt.alloc(n));
+  SGPU_TRY(upcnt.alloc(n + 1));  // and the longest row
   SGPU_TRY(len.alloc(n + 1));
-  SGPU_CUDA(cudaMemsetAsync(upcnt.p, 0, n * sizeof(int), s));
-  SGPU_CUDA(cudaMemsetAsync(len.p + n, 0, sizeof(int), s));
+  SGPU_CUDA(cudaMemsetAsync(upcnt.p, 0, (n + 1) * sizeof(int), s));
   k_row_of<<<blocks_for(n * 32), TPB, 0, s>>>(n, m->src_adr.p, row_of.p);
   if (sym) k_count_upper<<<blocks_for(negm), TPB, 0, s>>>(negm, m->src_ci.p, row_of.p, upcnt.p);
-  k_full_len<<<blocks_for(n), TPB, 0, s>>>(n, m->src_adr.p, upcnt.p, len.p, sym);
+  k_full_len<<<blocks_for(n), TPB, 0, s>>>(n, m->src_adr.p, upcnt.p, len.p, sym, upcnt.p + n);
   count_launches(sym ? 3 : 2);
 
   Csr &c = m->csr;
   SGPU_TRY(c.rowptr.alloc(n + 1));
-  // rowptr = exclusive scan of len (n+1 entries: scan over len with a trailing 0)
   {
     size_t tmp = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tmp, len.p, c.rowptr.p, (int)n, s);
+    cub::DeviceScan::ExclusiveSum(nullptr, tmp, len.p, c.rowptr.p, (int)n + 1, s);
     DevBuf<unsigned char> t;
     SGPU_TRY(t.alloc(tmp));
-    cub::DeviceScan::ExclusiveSum(t.p, tmp, len.p, c.rowptr.p, (int)n, s);
+    cub::DeviceScan::ExclusiveSum(t.p, tmp, len.p, c.rowptr.p, (int)n + 1, s);
     count_launches(2);
   }
-  int last_ptr = 0, last_len[2] = {0, 0};  // and the longest
-  SGPU_CUDA(cudaMemcpyAsync(&last_ptr, c.rowptr.p + n - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-  SGPU_CUDA(cudaMemcpyAsync(last_len, len.p + n - 1, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  SGPU_CUDA(cudaMemcpyAsync(&c.longest, upcnt.p + n, sizeof(int), cudaMemcpyDeviceToHost, s));
   SGPU_CUDA(cudaStreamSynchronize(s));
-  int64_t nnz = (int64_t)last_ptr + last_len[0];
-  c.longest = last_len[1];
-  if (nnz >= (1LL << 31) - 1) return fail(SGPU_BAD_INPUT, "matrix too large for int32 device indices");
-  const int nnz32 = (int)nnz;
-  SGPU_CUDA(cudaMemcpy(c.rowptr.p + n, &nnz32, sizeof(int), cudaMemcpyHostToDevice));
   SGPU_TRY(matrix_alloc_csr(m, n, nnz));
   SGPU_TRY(m->map_lo.alloc(negm));
   SGPU_TRY(m->map_up.alloc(negm));
