@@ -825,6 +825,15 @@ inline bool tiles_fit(const TileMat &m, int longest, int sms) {
   return longest > 0 && longest < 4096 && stage <= kTileRing && stage + 4ll * (per + 1) <= kTileSmem;
 }
 
+// Stages of a warp, as many as fit beside the unit pointers (and are of use).
+template <int ROWS, int LPR>
+inline int tile_stages(const TileMat &m, int longest, int sms) {
+  using K = TileKind<ROWS, LPR>;
+  const int W = kTileTPB<ROWS, LPR> / 32, ent = (longest * K::kUnits + 3) & ~3, per = (m.units + sms - 1) / sms;
+  const int ntiles = (per + K::kUnits - 1) / K::kUnits, room = std::min(kTileRing, kTileSmem - 4 * (per + 1));
+  return std::min(room / (W * (K::stage_bytes(ent) + 8)), (ntiles + W - 1) / W + 1);
+}
+
 template <int ROWS, int LPR>
 inline cudaError_t launch_tiles_as(const TileArgs &a, TileMat m, int longest, int sms, cudaStream_t s) {
   using K = TileKind<ROWS, LPR>;
@@ -832,9 +841,8 @@ inline cudaError_t launch_tiles_as(const TileArgs &a, TileMat m, int longest, in
   m.ent = (longest * K::kUnits + 3) & ~3;
   m.per = (m.units + sms - 1) / sms;
   const int grid = (m.units + m.per - 1) / m.per;  // no CTA without units
-  const int sb = K::stage_bytes(m.ent) + 8, ntiles = (m.per + K::kUnits - 1) / K::kUnits;
-  const int room = std::min(kTileRing, kTileSmem - 4 * (m.per + 1));
-  m.depth = std::min(room / (W * sb), (ntiles + W - 1) / W + 1);
+  const int sb = K::stage_bytes(m.ent) + 8;
+  m.depth = tile_stages<ROWS, LPR>(m, longest, sms);
   const size_t smem = (size_t)W * m.depth * sb + 4ull * (m.per + 1);
   auto k = k_pcg_tiles<ROWS, LPR, TPBX>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem);
@@ -868,9 +876,17 @@ constexpr int kTileMean = ROWS == 3 ? (LPR == 8 ? 10 : LPR == 16 ? 18 : 45) : (L
 template <int ROWS, int LPR>
 constexpr double kTileSlack = ROWS == 3 ? (LPR == 8 ? 1.0e6 : LPR == 16 ? 0.7e6 : 0.8e6)
                                         : (LPR == 2 ? 3.5e6 : LPR == 8 ? 5e6 : 6e6);
+// CSR with 2 lanes of which only one stage fits (many rows, whose pointers take
+// the shared memory, or a long one): 2M rows of 9 (one of 60) 107 / 95, of 13
+// 111 / 127; 4M of 13 (one of 30) 240 / 205, of 17 252 / 240; 3.4M of 27 255 / 285.
 template <int ROWS, int LPR>
-inline int tiles_pay(const TileMat &m, int64_t entries) {
-  return (double)kTileMean<ROWS, LPR> * m.units - (double)entries <= kTileSlack<ROWS, LPR> ? LPR : 0;
+inline int tiles_pay(const TileMat &m, int longest, int64_t entries, int sms) {
+  double mean = kTileMean<ROWS, LPR>, slack = kTileSlack<ROWS, LPR>;
+  if (ROWS == 1 && LPR == 2 && tile_stages<ROWS, LPR>(m, longest, sms) < 2) {
+    mean = 24;
+    slack = 25e6;
+  }
+  return mean * m.units - (double)entries <= slack ? LPR : 0;
 }
 
 // lanes per unit (0: the units are too long, too many or too uneven for tiles)
@@ -878,13 +894,13 @@ template <int ROWS>
 inline int tile_lanes(const TileMat &m, int longest, int64_t entries, int sms) {
   if (sms <= 0) return 0;
   if constexpr (ROWS == 3) {
-    if (tiles_fit<3, 8>(m, longest, sms)) return tiles_pay<3, 8>(m, entries);
-    if (tiles_fit<3, 16>(m, longest, sms)) return tiles_pay<3, 16>(m, entries);
-    if (tiles_fit<3, 32>(m, longest, sms)) return tiles_pay<3, 32>(m, entries);
+    if (tiles_fit<3, 8>(m, longest, sms)) return tiles_pay<3, 8>(m, longest, entries, sms);
+    if (tiles_fit<3, 16>(m, longest, sms)) return tiles_pay<3, 16>(m, longest, entries, sms);
+    if (tiles_fit<3, 32>(m, longest, sms)) return tiles_pay<3, 32>(m, longest, entries, sms);
   } else {
-    if (tiles_fit<1, 2>(m, longest, sms)) return tiles_pay<1, 2>(m, entries);
-    if (tiles_fit<1, 8>(m, longest, sms)) return tiles_pay<1, 8>(m, entries);
-    if (tiles_fit<1, 32>(m, longest, sms)) return tiles_pay<1, 32>(m, entries);
+    if (tiles_fit<1, 2>(m, longest, sms)) return tiles_pay<1, 2>(m, longest, entries, sms);
+    if (tiles_fit<1, 8>(m, longest, sms)) return tiles_pay<1, 8>(m, longest, entries, sms);
+    if (tiles_fit<1, 32>(m, longest, sms)) return tiles_pay<1, 32>(m, longest, entries, sms);
   }
   return 0;
 }

@@ -33,6 +33,8 @@ SYSTEMS = {
     "short_few": (lambda: banded(500003, [1], 1), True),  # 9 n - nnz = 3.0M of 3.5M
     "short_many": (lambda: banded(700001, [1], 1), False),  # 4.2M
     "short_many_of_seven": (lambda: banded(1000003, [1, 2, 50], 1), True),  # 2.0M
+    "one_stage_many": (lambda: one_long(2000003, [1, 2, 3, 5], 50, 8), False),  # 24 n - nnz = 30M of 25M
+    "one_stage_fewer": (lambda: one_long(1000003, [1, 2, 3, 5], 50, 8), True),  # 15M
     "resident_lane_of_160": (lambda: one_long(140001, [1, 2], 160 - 3, 2), True),
     "resident_lane_of_161": (lambda: one_long(140001, [1, 2], 161 - 3, 2), False),  # 8 lanes: 7.0M of 5M
     "resident_32_lanes_of_160": (lambda: one_long(9001, [1], 32 * 64 - 2, 3), True),  # 16 lanes, 2048 entries
