@@ -18,7 +18,8 @@ PER_THREAD = 2                  # cudaStreamPerThread
 
 @pytest.fixture(scope="module")
 def host(tmp_path_factory):
-    """The host sources and the stand-in as one library; what they call in files of kernels returns 0 at once."""
+    """The host sources and the stand-in as one library, bound to each other whatever runtime the process has loaded; what
+    they call in files of kernels returns 0 at once."""
     d = tmp_path_factory.mktemp("host")
     objs = []
     for src in [os.path.join(ROOT, "ssf_b200", "csrc", s) for s in SOURCES] + [os.path.join(HERE, "fake_cudart.cpp")]:
@@ -33,7 +34,7 @@ def host(tmp_path_factory):
     stubs.write_text(".text\n" + "".join(f".globl {n}\n{n}:\n" for n in missing) + "xorl %eax, %eax\nret\n"
                      ".section .note.GNU-stack,\"\",@progbits\n")
     out = str(d / "libhost.so")
-    subprocess.run(["g++", "-shared", "-o", out, *objs, str(stubs), "-lpthread"], check=True)
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", out, *objs, str(stubs), "-lpthread"], check=True)
     lib = C.CDLL(out)
     yield lib
 
