@@ -382,10 +382,9 @@ __global__ void __launch_bounds__(TPB, sizeof(T) == 4 && CPL <= 2 ? 4 : 1)
 // are bounded by those of the product: 531,441 rows of 27 entries, 32 columns,
 // FP64 with p.q 326 us an application, 685 without the bound (48 registers).
 template <typename VT, typename T, int CPL, class Op>
-__global__ void __launch_bounds__(TPB, CPL == 1 ? 8 : 1) k_mspmm_csr(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
-                                                   const VT *__restrict__ val, const T *__restrict__ X, Op op,
-                                                   MCol *cols, int R, MState *ms, double *partials,
-                                                   unsigned *ticket) {
+__global__ void __launch_bounds__(TPB, CPL == 1 ? 8 : 1)
+    k_mspmm_csr(int n, const int *__restrict__ rowptr, const int *__restrict__ col, const VT *__restrict__ val,
+                const T *__restrict__ X, Op op, MCol *cols, int R, MState *ms, double *partials, unsigned *ticket) {
   if (ms->all_done) return;
   constexpr int RP = 32 * CPL;
   constexpr int NVX = Op::NV > 0 ? Op::NV : 1;

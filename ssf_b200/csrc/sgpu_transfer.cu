@@ -109,7 +109,8 @@ cudaError_t copy(void *dst, const void *src, size_t bytes, cudaStream_t s, bool 
   const cudaMemcpyKind kind = in ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
   int dev = 0;
   // the per-thread default stream is another stream in each of the copying threads
-  if (bytes < kLeast || s == cudaStreamPerThread || cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices || !pageable(in ? src : dst))
+  if (bytes < kLeast || s == cudaStreamPerThread || cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices ||
+      !pageable(in ? src : dst))
     return cudaMemcpyAsync(dst, src, bytes, kind, s);
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
