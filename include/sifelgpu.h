@@ -277,7 +277,8 @@ typedef struct {
   const double *coords;  /* nn x 3 (z ignored for the plane kinds) */
   int64_t ne;            /* elements */
   const int64_t *elems;  /* ne x nne, 0-based node ids */
-  const int64_t *cn;     /* nn x ndofn code numbers (1-based, <= 0: no equation) */
+  const int64_t *cn;     /* nn x ndofn code numbers (1-based, <= 0: no equation); n is the largest.  Nodes may share
+                            one: the order of a shared entry's sum is then not fixed */
   const double *emat;    /* ne x 2: (E, nu) for elasticity, (k, c) for hex8t */
   const double *thick;   /* ne thicknesses (plane kinds), else NULL */
   const double *rho;     /* ne densities (capacity), NULL = 1 */
